@@ -74,93 +74,153 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// X[m][p] = sum_k P[aos[m]][aos[k]] phi[k][p]: CTA tile 64 rows x 128 points, K step 16,
-// 8 warps as 2 x 4 warp tiles of 32 x 32 (4 x 4 DMMA tiles). The next K step's operands
-// are fetched into registers while the current one is multiplied. Planes are [nbp][128]
-// arrays of the block's workspace: source plane src0 + z, destination plane dst0 + z for
-// blockIdx.z = z (the build: one plane, phi -> X after the phi planes; the gradient:
-// phi and its three derivatives -> X and Y_x, Y_y, Y_z).
-constexpr int GX_BM = 64, GX_BK = 16, GX_AS = GX_BK + 2, GX_BS = BLOCK_PTS + 4;
+// Asynchronous copies global -> shared; with ok = false the destination is zero-filled and nothing is read.
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(ok ? 8 : 0));
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(ok ? 16 : 0));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// The FP64 contractions cover a block's nb AOs with T = ceil(nb / 64) tiles per dimension, tile i
+// taking an equal share of the 16-row pairs of DMMA rows, cut at the last row of eight: nb rounded up
+// to 8, not to 64, is what the tensor pipe works for. (nb averages 231 on the 100-atom chain, 256 with
+// 64-row padding: sum of nb^2 29 % less together with the last rows' trim.) r8, n8: first row of
+// eight and their number (at most 8).
+__device__ __forceinline__ void fp64_tile(int nb, int T, int i, int& r8, int& n8) {
+    const int pairs = (nb + 15) / 16;
+    r8 = 2 * (i * pairs / T);
+    n8 = min((nb + 7) / 8, 2 * ((i + 1) * pairs / T)) - r8;
+}
+
+// X[m][p] = sum_k P[aos[m]][aos[k]] phi[k][p]: CTA tile up to 64 rows x 128 points, K step 16 in a
+// ring of three shared-memory stages filled by asynchronous copies (one barrier per step), 8 warps
+// of all the tile's rows x 16 points (up to 8 x 2 DMMA tiles), so that a trimmed tile shortens every
+// warp alike. Bound by the FP64 tensor pipe. Planes are [nbp][128] arrays of the block's workspace:
+// source plane src0 + z, destination plane dst0 + z for blockIdx.z = z (the build: one plane, phi ->
+// X after the phi planes; the gradient: phi and its three derivatives -> X and Y_x, Y_y, Y_z).
+// Rows of phi at nb and beyond are not read. Row strides of 20 and 132 doubles keep the fragment
+// loads free of bank conflicts (4 g + t and g + 4 t distinct modulo 16).
+constexpr int GX_BM = 64, GX_BK = 16, GX_S = 3, GX_AS = GX_BK + 4, GX_BS = BLOCK_PTS + 4;
+constexpr int GX_STAGE = GX_BM * GX_AS + GX_BK * GX_BS;  // doubles
+constexpr int GX_SMEM = GX_S * GX_STAGE * 8;
+
+// one K step (kn of its 16 columns, in fours) of a warp's MC x 2 DMMA tiles
+template <int MC>
+__device__ __forceinline__ void gx_step(const double* As, const double* Bs, int kn, double (&acc)[8][2][2]) {
+    auto four = [&](int kk) {
+        double a[MC], b[2];
+#pragma unroll
+        for (int i = 0; i < MC; ++i) a[i] = As[i * 8 * GX_AS + kk];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) b[j] = Bs[kk * GX_BS + j * 8];
+#pragma unroll
+        for (int i = 0; i < MC; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+    };
+    if (kn >= GX_BK) {
+#pragma unroll
+        for (int kk = 0; kk < GX_BK; kk += 4) four(kk);
+    } else {
+#pragma unroll 1
+        for (int kk = 0; kk < kn; kk += 4) four(kk);
+    }
+}
+
 __global__ void __launch_bounds__(256, 2) k_gemm_x(GridView g, const double* __restrict__ P, int nao,
                                                 int blk0, char* ws, int src0, int dst0, int64_t t0) {
-    int blk, m0;
+    extern __shared__ __align__(16) double gx_sm[];
+    int blk, ti;
     if (g.xtiles) {  // one CTA per tile of the list
         const int2 it = g.xtiles[t0 + blockIdx.x];
-        blk = it.x, m0 = it.y * GX_BM;
+        blk = it.x, ti = it.y;
     } else {
-        blk = blk0 + blockIdx.y, m0 = blockIdx.x * GX_BM;
+        blk = blk0 + blockIdx.y, ti = blockIdx.x;
     }
     const BlockMeta m = g.meta[blk];
-    if (m0 >= m.nbp) return;
+    const int T = (m.nb + 63) / 64;
+    if (ti >= T) return;
+    int r8, mc;
+    fp64_tile(m.nb, T, ti, r8, mc);
+    const int m0 = r8 * 8;
     const size_t plane = (size_t)m.nbp * BLOCK_PTS;
     const double* phi = reinterpret_cast<const double*>(ws + m.ws) + (size_t)(src0 + blockIdx.z) * plane;
     double* X = reinterpret_cast<double*>(ws + m.ws) + (size_t)(dst0 + blockIdx.z) * plane;
     const int* aos = g.blk_aos + m.ao0;
 
-    __shared__ double As[GX_BM * GX_AS];   // [m][k]
-    __shared__ double Bs[GX_BK * GX_BS];   // [k][n]
-    __shared__ int s_row[GX_BM];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int wm = warp >> 2, wn = warp & 3, gq = lane >> 2, tq = lane & 3;
-    for (int r = t; r < GX_BM; r += 256) s_row[r] = (m0 + r < m.nb) ? aos[m0 + r] : -1;
-    __syncthreads();
-
-    double acc[4][4][2];
+    const int gq = lane >> 2, tq = lane & 3;
+    // this thread's share of a stage: A column t % 16 of rows t / 16 + 16 q (gathered from P), B
+    // the 16-byte piece t % 64 of phi rows t / 64 + 4 q
+    const double* prow[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-    double ra[4], rb[8];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {  // A: 64 x 16 gathered from P (L2-resident)
-            const int e = t + q * 256, r = e >> 4, c = e & 15, gc = k0 + c;
-            const int row = s_row[r];
-            ra[q] = (row >= 0 && gc < m.nb) ? __ldg(P + (size_t)row * nao + aos[gc]) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {  // B: 16 x 128 of phi, coalesced
-            const int e = t + q * 256, r = e >> 7, c = e & 127;
-            rb[q] = phi[(size_t)(k0 + r) * BLOCK_PTS + c];
-        }
-    };
-    fetch(0);
-    for (int k0 = 0; k0 < m.nbp; k0 += GX_BK) {
+    for (int q = 0; q < 4; ++q) {
+        const int r = (t >> 4) + 16 * q;
+        prow[q] = r < 8 * mc && m0 + r < m.nb ? P + (size_t)aos[m0 + r] * nao : nullptr;
+    }
+    const int nk = (m.nb + GX_BK - 1) / GX_BK;
+    auto issue = [&](int kt) {
+        double* st = gx_sm + (kt % GX_S) * GX_STAGE;
+        const int k = kt * GX_BK + (t & 15);
+        const int col = k < m.nb ? aos[k] : -1;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int e = t + q * 256;
-            As[(e >> 4) * GX_AS + (e & 15)] = ra[q];
+            const bool ok = col >= 0 && prow[q];
+            cp_async8(st + ((t >> 4) + 16 * q) * GX_AS + (t & 15), ok ? prow[q] + col : P, ok);
         }
+        double* bs = st + GX_BM * GX_AS;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int e = t + q * 256;
-            Bs[(e >> 7) * GX_BS + (e & 127)] = rb[q];
+        for (int q = 0; q < 4; ++q) {
+            const int r = (t >> 6) + 4 * q, kr = kt * GX_BK + r;
+            const bool ok = kr < m.nb;
+            cp_async16(bs + r * GX_BS + 2 * (t & 63), phi + (ok ? (size_t)kr * BLOCK_PTS + 2 * (t & 63) : 0), ok);
         }
-        __syncthreads();
-        if (k0 + GX_BK < m.nbp) fetch(k0 + GX_BK);
+    };
+    double acc[8][2][2];
 #pragma unroll
-        for (int kk = 0; kk < GX_BK; kk += 4) {
-            double a[4], b[4];
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[(wm * 32 + i * 8 + gq) * GX_AS + kk + tq];
+        for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[(kk + tq) * GX_BS + wn * 32 + j * 8 + gq];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+    for (int k = 0; k < GX_S - 1; ++k) {
+        if (k < nk) issue(k);
+        cp_async_commit();
+    }
+    for (int kt = 0; kt < nk; ++kt) {
+        cp_async_wait<GX_S - 2>();
+        __syncthreads();  // stage kt has landed for every thread, and stage kt - 1 is consumed
+        if (kt + GX_S - 1 < nk) issue(kt + GX_S - 1);
+        cp_async_commit();
+        const double* st = gx_sm + (kt % GX_S) * GX_STAGE;
+        const double* As = st + gq * GX_AS + tq;
+        const double* Bs = st + GX_BM * GX_AS + tq * GX_BS + warp * 16 + gq;
+        const int kn = m.nb - kt * GX_BK;
+        switch (mc) {  // uniform over the CTA
+            case 8: gx_step<8>(As, Bs, kn, acc); break;
+            case 7: gx_step<7>(As, Bs, kn, acc); break;
+            case 6: gx_step<6>(As, Bs, kn, acc); break;
+            case 5: gx_step<5>(As, Bs, kn, acc); break;
+            case 4: gx_step<4>(As, Bs, kn, acc); break;
+            case 3: gx_step<3>(As, Bs, kn, acc); break;
+            case 2: gx_step<2>(As, Bs, kn, acc); break;
+            default: gx_step<1>(As, Bs, kn, acc);
         }
-        __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
+        if (i < mc)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            double2* dst = reinterpret_cast<double2*>(X + (size_t)(m0 + wm * 32 + i * 8 + gq) * BLOCK_PTS + wn * 32 +
-                                                      j * 8 + 2 * tq);
-            *dst = make_double2(acc[i][j][0], acc[i][j][1]);
-        }
+            for (int j = 0; j < 2; ++j)
+                *reinterpret_cast<double2*>(X + (size_t)(m0 + i * 8 + gq) * BLOCK_PTS + warp * 16 + j * 8 + 2 * tq) =
+                    make_double2(acc[i][j][0], acc[i][j][1]);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -452,12 +512,45 @@ __global__ void __launch_bounds__(BLOCK_PTS, 6) k_z_rad(BasisView bas, GridView 
     for (int r = m.nb; r < m.nbp; ++r) Z[(size_t)r * BLOCK_PTS + p] = 0.0;
 }
 
-// Vacc[aos[m]][aos[n]] += sum_p phi[m][p] Z[n][p]: CTA tile 64 x 64 AOs, K = 128 points in
-// steps of 16, 4 warps as 2 x 2 warp tiles of 32 x 32 (4 x 4 DMMA tiles). Z was formed by
-// k_rho_functional in the place of X; both tiles are staged as [row][k] with 128-byte rows.
-constexpr int GV_B = 64, GV_BK = 16, GV_AS = GV_BK + 2;
+// Vacc[aos[m]][aos[n]] += sum_p phi[m][p] Z[n][p]: CTA tile up to 64 x 64 AOs (fp64_tile in both
+// dimensions), K = 128 points in steps of 16 through a ring of three shared-memory stages, 4 warps as
+// 2 x 2 of up to 4 x 4 DMMA tiles. Bound by the FP64 tensor pipe. A tile of an odd number of rows of
+// eight gives its first warps more work, and a warp stays on its quarter of the SM, so the warps'
+// places in the tile rotate with the CTA. Z was formed in the place of X; rows at nb and beyond are
+// not read.
+constexpr int GV_B = 64, GV_BK = 16, GV_S = 3, GV_AS = GV_BK + 4;
+constexpr int GV_STAGE = 2 * GV_B * GV_AS;  // doubles: A [m][k], B [n][k]
+constexpr int GV_SMEM = GV_S * GV_STAGE * 8;
+
+template <int MI, int NJ>
+__device__ __forceinline__ void gv_step(const double* As, const double* Bs, double (&acc)[4][4][2]) {
+#pragma unroll
+    for (int kk = 0; kk < GV_BK; kk += 4) {
+        double a[MI], b[NJ];
+#pragma unroll
+        for (int i = 0; i < MI; ++i) a[i] = As[i * 8 * GV_AS + kk];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) b[j] = Bs[j * 8 * GV_AS + kk];
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+    }
+}
+template <int MI>
+__device__ __forceinline__ void gv_step_n(int nj, const double* As, const double* Bs, double (&acc)[4][4][2]) {
+    switch (nj) {
+        case 4: gv_step<MI, 4>(As, Bs, acc); break;
+        case 3: gv_step<MI, 3>(As, Bs, acc); break;
+        case 2: gv_step<MI, 2>(As, Bs, acc); break;
+        case 1: gv_step<MI, 1>(As, Bs, acc); break;
+        default: break;
+    }
+}
+
 __global__ void __launch_bounds__(128, 3) k_gemm_v(GridView g, int blk0, char* ws, int zplane, double* Vacc, int nao,
                                                 int tiles, int64_t t0) {
+    extern __shared__ __align__(16) double gv_sm[];
     int blk, tm, tn;
     if (g.vtiles) {  // one CTA per tile of the list
         const int2 it = g.vtiles[t0 + blockIdx.x];
@@ -466,61 +559,67 @@ __global__ void __launch_bounds__(128, 3) k_gemm_v(GridView g, int blk0, char* w
         blk = blk0 + blockIdx.y, tm = blockIdx.x / tiles, tn = blockIdx.x % tiles;
     }
     const BlockMeta m = g.meta[blk];
-    const int m0 = tm * GV_B, n0 = tn * GV_B;
-    if (m0 >= m.nbp || n0 >= m.nbp) return;
+    const int T = (m.nb + 63) / 64;
+    if (tm >= T || tn >= T) return;
+    int mr8, mc, nr8, nc;
+    fp64_tile(m.nb, T, tm, mr8, mc);
+    fp64_tile(m.nb, T, tn, nr8, nc);
+    const int m0 = mr8 * 8, n0 = nr8 * 8;
     const double* phi = reinterpret_cast<const double*>(ws + m.ws);
     const double* Z = phi + (size_t)zplane * m.nbp * BLOCK_PTS;
     const int* aos = g.blk_aos + m.ao0;
-    __shared__ double As[GV_B * GV_AS];  // [m][k]
-    __shared__ double Bs[GV_B * GV_AS];  // [n][k]
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int wm = warp >> 1, wn = warp & 1, gq = lane >> 2, tq = lane & 3;
+    const int t = threadIdx.x, lane = t & 31, warp = ((t >> 5) + blockIdx.x) & 3;
+    const int gq = lane >> 2, tq = lane & 3;
+    const int wm8 = (warp >> 1) * ((mc + 1) >> 1), wn8 = (warp & 1) * ((nc + 1) >> 1);  // the warp's first rows of eight
+    const int mi = warp >> 1 ? mc >> 1 : (mc + 1) >> 1, nj = warp & 1 ? nc >> 1 : (nc + 1) >> 1;
     double acc[4][4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    double ra[8], rb[8];
-    auto fetch = [&](int k0) {
+    auto issue = [&](int kt) {  // thread: the 16-byte piece t % 8 of rows t / 8 + 16 q of both operands
+        double* st = gv_sm + (kt % GV_S) * GV_STAGE;
+        const int c = 2 * (t & 7);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int e = t + q * 128, r = e >> 4, c = e & 15;  // row within tile, point within K step
-            ra[q] = phi[(size_t)(m0 + r) * BLOCK_PTS + k0 + c];
-            rb[q] = Z[(size_t)(n0 + r) * BLOCK_PTS + k0 + c];
+        for (int q = 0; q < 4; ++q) {
+            const int r = (t >> 3) + 16 * q;
+            const bool oka = r < 8 * mc && m0 + r < m.nb, okb = r < 8 * nc && n0 + r < m.nb;
+            cp_async16(st + r * GV_AS + c, phi + (oka ? (size_t)(m0 + r) * BLOCK_PTS + kt * GV_BK + c : 0), oka);
+            cp_async16(st + (GV_B + r) * GV_AS + c, Z + (okb ? (size_t)(n0 + r) * BLOCK_PTS + kt * GV_BK + c : 0), okb);
         }
     };
-    fetch(0);
-    for (int k0 = 0; k0 < BLOCK_PTS; k0 += GV_BK) {
+    constexpr int nk = BLOCK_PTS / GV_BK;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int e = t + q * 128, r = e >> 4, c = e & 15;
-            As[r * GV_AS + c] = ra[q];
-            Bs[r * GV_AS + c] = rb[q];
+    for (int k = 0; k < GV_S - 1; ++k) {
+        issue(k);
+        cp_async_commit();
+    }
+#pragma unroll 1
+    for (int kt = 0; kt < nk; ++kt) {
+        cp_async_wait<GV_S - 2>();
+        __syncthreads();  // stage kt has landed for every thread, and stage kt - 1 is consumed
+        if (kt + GV_S - 1 < nk) issue(kt + GV_S - 1);
+        cp_async_commit();
+        const double* st = gv_sm + (kt % GV_S) * GV_STAGE;
+        const double* As = st + (wm8 * 8 + gq) * GV_AS + tq;
+        const double* Bs = st + (GV_B + wn8 * 8 + gq) * GV_AS + tq;
+        switch (mi) {  // uniform over the warp
+            case 4: gv_step_n<4>(nj, As, Bs, acc); break;
+            case 3: gv_step_n<3>(nj, As, Bs, acc); break;
+            case 2: gv_step_n<2>(nj, As, Bs, acc); break;
+            case 1: gv_step_n<1>(nj, As, Bs, acc); break;
+            default: break;
         }
-        __syncthreads();
-        if (k0 + GV_BK < BLOCK_PTS) fetch(k0 + GV_BK);
-#pragma unroll
-        for (int kk = 0; kk < GV_BK; kk += 4) {
-            double a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[(wm * 32 + i * 8 + gq) * GV_AS + kk + tq];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[(wn * 32 + j * 8 + gq) * GV_AS + kk + tq];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-        }
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int r = m0 + wm * 32 + i * 8 + gq;
-        if (r >= m.nb) continue;
+        const int r = m0 + (wm8 + i) * 8 + gq;
+        if (i >= mi || r >= m.nb) continue;
         const size_t rowoff = (size_t)aos[r] * nao;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int c = n0 + wn * 32 + j * 8 + 2 * tq;
+            const int c = n0 + (wn8 + j) * 8 + 2 * tq;
+            if (j >= nj) continue;
             if (c < m.nb) atomicAdd(&Vacc[rowoff + aos[c]], acc[i][j][0]);
             if (c + 1 < m.nb) atomicAdd(&Vacc[rowoff + aos[c + 1]], acc[i][j][1]);
         }
@@ -665,13 +764,14 @@ void launch_gemm_x(const GridView& g, const double* P, int nao, int blk0, int nb
 
 void launch_gemm_x_planes(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src0,
                           int dst0, int nz, char* ws, cudaStream_t s) {
+    cudaFuncSetAttribute(k_gemm_x, cudaFuncAttributeMaxDynamicSharedMemorySize, GX_SMEM);
     if (g.xtiles && g.h_xtile0) {
         const int64_t t0 = g.h_xtile0[blk0], n = g.h_xtile0[blk0 + nblk] - t0;
-        if (n > 0) k_gemm_x<<<dim3((unsigned)n, 1, nz), 256, 0, s>>>(g, P, nao, blk0, ws, src0, dst0, t0);
+        if (n > 0) k_gemm_x<<<dim3((unsigned)n, 1, nz), 256, GX_SMEM, s>>>(g, P, nao, blk0, ws, src0, dst0, t0);
         return;
     }
     dim3 grid((max_nbp + GX_BM - 1) / GX_BM, nblk, nz);
-    k_gemm_x<<<grid, 256, 0, s>>>(g, P, nao, blk0, ws, src0, dst0, 0);
+    k_gemm_x<<<grid, 256, GX_SMEM, s>>>(g, P, nao, blk0, ws, src0, dst0, 0);
 }
 
 void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, char* ws, cudaStream_t s) {
@@ -710,13 +810,14 @@ void launch_gemm_v(const GridView& g, int blk0, int nblk, int max_nbp, bool gga,
 void launch_gemm_v_plane(const GridView& g, int blk0, int nblk, int max_nbp, int zplane, char* ws, double* Vacc,
                          int nao, cudaStream_t s) {
     const int tiles = (max_nbp + GV_B - 1) / GV_B;
+    cudaFuncSetAttribute(k_gemm_v, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM);
     if (g.vtiles && g.h_vtile0) {
         const int64_t t0 = g.h_vtile0[blk0], n = g.h_vtile0[blk0 + nblk] - t0;
-        if (n > 0) k_gemm_v<<<(unsigned)n, 128, 0, s>>>(g, blk0, ws, zplane, Vacc, nao, tiles, t0);
+        if (n > 0) k_gemm_v<<<(unsigned)n, 128, GV_SMEM, s>>>(g, blk0, ws, zplane, Vacc, nao, tiles, t0);
         return;
     }
     dim3 grid(tiles * tiles, nblk);
-    k_gemm_v<<<grid, 128, 0, s>>>(g, blk0, ws, zplane, Vacc, nao, tiles, 0);
+    k_gemm_v<<<grid, 128, GV_SMEM, s>>>(g, blk0, ws, zplane, Vacc, nao, tiles, 0);
 }
 
 void launch_rho_functional_uks(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,

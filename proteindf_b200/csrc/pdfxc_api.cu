@@ -752,7 +752,7 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
                 m.sh0 = sh0, m.ao0 = ao0;
                 m.nsh = (int)P.shells.size() - sh0;
                 m.nb = row;
-                m.nbp = mixed ? std::max(128, (row + 127) / 128 * 128) : std::max(64, (row + 63) / 64 * 64);
+                m.nbp = mixed ? std::max(128, (row + 127) / 128 * 128) : std::max(8, (row + 7) / 8 * 8);
                 blk_flops[bb] = 4.0 * double(m.nb) * m.nb * m.npts;
             }
         }
@@ -856,11 +856,11 @@ void build_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* ato
         upload(&ctx->d_blk_row_geom, geom, s);
     }
     upload(&ctx->d_seg_blk, ctx->seg_blk, s);
-    {  // the FP64 contractions' tile lists (64-AO tiles of each block's nbp rows)
+    {  // the FP64 contractions' tile lists (up to 64 of a block's nb AOs each)
         std::vector<int2> xt, vt;
         ctx->h_xtile0.assign(1, 0), ctx->h_vtile0.assign(1, 0);
         for (int b = 0; b < nblk; ++b) {
-            const int nt = (ctx->h_meta[b].nbp + 63) / 64;
+            const int nt = (ctx->h_meta[b].nb + 63) / 64;
             for (int i = 0; i < nt; ++i) xt.push_back(make_int2(b, i));
             for (int i = 0; i < nt; ++i)
                 for (int j = 0; j < nt; ++j) vt.push_back(make_int2(b, (i << 16) | j));

@@ -22,7 +22,7 @@ struct BlockMeta {
     int nsh;       // screened shells
     int ao0;       // first entry in blk_aos
     int nb;        // screened AOs
-    int nbp;       // nb rounded up to the contraction tile
+    int nbp;       // rows of a workspace plane: nb rounded up to 8 (FP64) or to the 128-row tile (mixed)
     int npts;      // real points in the block (<= BLOCK_PTS)
     int lead;      // first block of this block's group (the block itself when ungrouped)
     int gn;        // blocks in the group; a group's blocks are consecutive and share one screened basis
