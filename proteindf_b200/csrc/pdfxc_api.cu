@@ -105,23 +105,21 @@ pdfxc_status guarded(pdfxc_ctx* ctx, F&& f) {
     }
 }
 
-// Distance beyond which a shell's value and gradient bounds both stay below
-// `cutoff`: bound(r) = sum_k |c_k| e^{-a_k r^2} max(r^L, L r^(L-1) + 2 a_k r^(L+1)).
-double shell_cutoff_radius(int L, const double* e, const double* c, int np, double cutoff) {
-    double R = 0.0;
+// Distances beyond which a shell's value and gradient bounds both stay below `cutoff` (first) and
+// below share * cutoff (second), share <= 1:
+// bound(r) = sum_k |c_k| e^{-a_k r^2} max(r^L, L r^(L-1) + 2 a_k r^(L+1)).
+std::pair<double, double> shell_cutoff_radius(int L, const double* e, const double* c, int np, double cutoff,
+                                              double share) {
+    double outer = 0.0;
     for (double r = 60.0; r > 0.0; r -= 0.01) {
+        const double rl = std::pow(r, L), dl = L > 0 ? L * std::pow(r, L - 1) : 0.0;
         double b = 0.0;
-        for (int k = 0; k < np; ++k) {
-            const double rl = std::pow(r, L);
-            const double g = std::max(rl, (L > 0 ? L * std::pow(r, L - 1) : 0.0) + 2.0 * e[k] * rl * r);
-            b += std::fabs(c[k]) * std::exp(-e[k] * r * r) * g;
-        }
-        if (b >= cutoff) {
-            R = r + 0.01;
-            break;
-        }
+        for (int k = 0; k < np; ++k)
+            b += std::fabs(c[k]) * std::exp(-e[k] * r * r) * std::max(rl, dl + 2.0 * e[k] * rl * r);
+        if (outer == 0.0 && b >= share * cutoff) outer = r + 0.01;
+        if (b >= cutoff) return {r + 0.01, outer};
     }
-    return R;
+    return {0.0, outer};
 }
 
 uint64_t spread3(uint64_t v) {
@@ -489,7 +487,7 @@ void resolve_shapes(pdfxc_ctx* ctx, int64_t npts, size_t nseg) {
 // are put in Morton order over the segment's bounding box and cut into groups of up to
 // group_blocks x block_points consecutive points, each group into blocks of block_points;
 // every group keeps the shells of its segment whose value/gradient envelope reaches
-// ao_cutoff at the group's nearest point.
+// ao_cutoff at the nearest point of its bounding sphere and 0.3 of it at its own nearest point.
 // The host side of a blocked grid (plan_grid), before it is uploaded.
 struct HostGrid {
     std::vector<double> px, py, pz, pw;
@@ -622,8 +620,15 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
     });
     // 2. per-shell screening radius, then the per-block shell lists
     // (once per distinct shell: the shells of one element's basis repeat on every such atom)
-    std::vector<double> Rs(ctx->nshell);
-    std::map<std::vector<double>, double> radius_of;
+    // Rs: where the envelope falls below ao_cutoff, tested against the group's bounding sphere; Rn: where
+    // it falls below kNearShare of it, tested against the group's nearest point. (The sphere test alone
+    // keeps shells that no point reaches. Without the share the results at a loose cut-off would lie
+    // further from the unscreened ones than with the sphere test alone; 90-atom B3LYP chain, cut-off
+    // 1e-10, relative error of Vxc: sphere 3.4e-12; nearest point at 1.0, 0.5, 0.3 of the cut-off
+    // 9.3e-12, 4.5e-12, 2.6e-12.)
+    constexpr double kNearShare = 0.3;
+    std::vector<double> Rs(ctx->nshell), Rn(ctx->nshell);
+    std::map<std::vector<double>, std::pair<double, double>> radius_of;
     for (int sh = 0; sh < ctx->nshell; ++sh) {
         const int p0 = ctx->h_sh_p0[sh], np = ctx->h_sh_nprim[sh];
         std::vector<double> k = {(double)ctx->h_sh_l[sh]};
@@ -632,8 +637,8 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
         auto it = radius_of.find(k);
         if (it == radius_of.end())
             it = radius_of.emplace(k, shell_cutoff_radius(ctx->h_sh_l[sh], &ctx->h_p_exp[p0], &ctx->h_p_coef[p0], np,
-                                                          ctx->opt.ao_cutoff)).first;
-        Rs[sh] = it->second;
+                                                          ctx->opt.ao_cutoff, kNearShare)).first;
+        Rs[sh] = it->second.first, Rn[sh] = it->second.second;
     }
     std::vector<int>&shells = G.shells, &rows = G.rows, &aos = G.aos, &row_info = G.row_info;
     shells.clear(), rows.clear(), aos.clear(), row_info.clear();
@@ -732,12 +737,45 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
             const int sh0 = (int)P.shells.size(), ao0 = (int)P.aos.size();
             int row = 0;
             candidates(si, (int)gi, cand_sh, ats);
+            // A shell must pass both tests (Rs, Rn above). The sphere settles the shells that every point
+            // reaches and the bounding box most of those that none reaches; for the rest the points are
+            // looked through, as far as the first one inside, once per atom.
+            double blo[3] = {1e300, 1e300, 1e300}, bhi[3] = {-1e300, -1e300, -1e300};
+            const size_t slot0 = (size_t)grp_blk[gi] * BLOCK_PTS;  // the group's slots; only its last block may be padded
+            const size_t slot1 = (size_t)(grp_blk[gi + 1] - 1) * BLOCK_PTS + ctx->h_meta[grp_blk[gi + 1] - 1].npts;
+            const bool padded = bp < BLOCK_PTS;  // smaller blocks: every block is padded
+            for (size_t i = slot0; i < slot1; ++i) {
+                const double r[3] = {px[i], py[i], pz[i]};  // (a padding slot holds its block's centroid)
+                for (int k = 0; k < 3; ++k) blo[k] = std::min(blo[k], r[k]), bhi[k] = std::max(bhi[k], r[k]);
+            }
+            int near_atom = -1;
+            size_t next = slot0;  // the first slot not yet looked at for near_atom
+            double near2 = 0.0;
+            auto beyond = [&](int a, double R) {  // no point of the group lies within R of atom a
+                const double* A = &ctx->h_atom_xyz[3 * a];
+                double d2 = 0.0;
+                for (int k = 0; k < 3; ++k) {
+                    const double d = std::max({blo[k] - A[k], A[k] - bhi[k], 0.0});
+                    d2 += d * d;
+                }
+                if (d2 > R * R) return true;
+                if (a != near_atom) near_atom = a, near2 = 1e300, next = slot0;
+                const double ax = A[0], ay = A[1], az = A[2];
+                for (; next < slot1 && near2 > R * R; ++next) {
+                    if (padded && ctx->h_src[next] < 0) continue;
+                    const double x = px[next] - ax, y = py[next] - ay, z = pz[next] - az;
+                    near2 = std::min(near2, x * x + y * y + z * z);
+                }
+                return near2 > R * R;
+            };
             for (int sh : cand_sh) {
-                const double* A = &ctx->h_atom_xyz[3 * ctx->h_sh_atom[sh]];
+                const int at = ctx->h_sh_atom[sh];
+                const double* A = &ctx->h_atom_xyz[3 * at];
                 const double d = std::sqrt((A[0] - cen[3 * gi]) * (A[0] - cen[3 * gi]) +
                                            (A[1] - cen[3 * gi + 1]) * (A[1] - cen[3 * gi + 1]) +
                                            (A[2] - cen[3 * gi + 2]) * (A[2] - cen[3 * gi + 2]));
                 if (d - rad[gi] > Rs[sh]) continue;
+                if (d + rad[gi] > Rn[sh] && beyond(at, Rn[sh])) continue;
                 P.shells.push_back(sh);
                 P.rows.push_back(row);
                 const int L = ctx->h_sh_l[sh], nc = 2 * L + 1;
