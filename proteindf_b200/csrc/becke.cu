@@ -71,73 +71,282 @@ __global__ void __launch_bounds__(128) k_becke(const double* __restrict__ atom_x
     }
 }
 
-// Pair constants: inv[m*n_atom + n] = 1/|R_m - R_n|, adj[m*n_atom + n] = a_mn (0 without size adjustment).
+// Pair constants of atoms m and n: inv = 1/|R_m - R_n|, adj = a_mn (0 without size adjustment).
 // A dummy partner n (ghost[n] != 0) gets inv = 0 and adj = -1: then nu = -1 and its factor
 // s = (1 - f3(-1)) / 2 is exactly 1 (f(-1) = -1 in IEEE arithmetic), the same as leaving it out.
-__global__ void k_becke_pairs(const double* __restrict__ atom_xyz, const double* __restrict__ brad,
-                              const int* __restrict__ ghost, int natom, int size_adjust, double* inv, double* adj) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < natom * natom; e += gridDim.x * blockDim.x) {
-        const int m = e / natom, n = e % natom;
-        if (m == n) {
-            inv[e] = adj[e] = 0.0;
-            continue;
-        }
-        if (ghost && ghost[n]) {
-            inv[e] = 0.0, adj[e] = -1.0;
-            continue;
-        }
-        const double dx = atom_xyz[3 * m] - atom_xyz[3 * n], dy = atom_xyz[3 * m + 1] - atom_xyz[3 * n + 1],
-                     dz = atom_xyz[3 * m + 2] - atom_xyz[3 * n + 2];
-        inv[e] = 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
-        double a = 0.0;
-        if (size_adjust) {
-            const double au = (brad[m] - brad[n]) / (brad[m] + brad[n]);
-            a = au / (au * au - 1.0);
-            a = a < -0.5 ? -0.5 : (a > 0.5 ? 0.5 : a);
-        }
-        adj[e] = a;
+__device__ __forceinline__ void becke_pair(const double* __restrict__ atom_xyz, const double* __restrict__ brad,
+                                           const int* __restrict__ ghost, int size_adjust, int m, int n, double& inv,
+                                           double& adj) {
+    inv = adj = 0.0;
+    if (m == n) return;
+    if (ghost && ghost[n]) {
+        adj = -1.0;
+        return;
+    }
+    const double dx = atom_xyz[3 * m] - atom_xyz[3 * n], dy = atom_xyz[3 * m + 1] - atom_xyz[3 * n + 1],
+                 dz = atom_xyz[3 * m + 2] - atom_xyz[3 * n + 2];
+    inv = 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
+    if (size_adjust) {
+        const double au = (brad[m] - brad[n]) / (brad[m] + brad[n]);
+        const double a = au / (au * au - 1.0);
+        adj = a < -0.5 ? -0.5 : (a > 0.5 ? 0.5 : a);
     }
 }
 
-// Same weights as k_becke, one point per thread, with each thread's point-atom distances kept in
-// shared memory ([atom][thread]) and the pair constants read from the table: one multiply per
-// pair instead of two square roots and a division. Its shared memory per CTA grows with the atom
-// count, so it is the form for small molecules (becke_small_atoms), k_becke_warp the one above.
-constexpr int BECKE_T = 64;
-__global__ void __launch_bounds__(BECKE_T) k_becke_tab(const double* __restrict__ atom_xyz, int natom,
-                                                       const double* __restrict__ inv, const double* __restrict__ adj,
-                                                       int64_t npts, const double* __restrict__ xyz,
-                                                       const int* __restrict__ owner,
-                                                       const double* __restrict__ w_single, double* __restrict__ w_out) {
-    extern __shared__ double rr[];  // [natom][BECKE_T]
-    const int t = threadIdx.x;
-    for (int64_t i0 = blockIdx.x * (int64_t)BECKE_T; i0 < npts; i0 += (int64_t)gridDim.x * BECKE_T) {
-        const int64_t i = i0 + t;
+// The pair table: inv[m*n_atom + n], adj[m*n_atom + n].
+__global__ void k_becke_pairs(const double* __restrict__ atom_xyz, const double* __restrict__ brad,
+                              const int* __restrict__ ghost, int natom, int size_adjust, double* inv, double* adj) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < natom * natom; e += gridDim.x * blockDim.x)
+        becke_pair(atom_xyz, brad, ghost, size_adjust, e / natom, e % natom, inv[e], adj[e]);
+}
+
+// The tables of k_becke_near, one CTA per atom m: (inv, adj) of its row in FP64 and in FP32, and
+// its kNearList nearest atoms by distance, itself first (ties by index).
+constexpr int kNearList = 16;
+__global__ void __launch_bounds__(128) k_becke_near_tables(const double* __restrict__ atom_xyz,
+                                                           const double* __restrict__ brad,
+                                                           const int* __restrict__ ghost, int natom, int size_adjust,
+                                                           double2* __restrict__ pair, float2* __restrict__ pairf,
+                                                           int* __restrict__ near) {
+    extern __shared__ double nd[];  // [natom] squared distance to m
+    __shared__ double bd[128];
+    __shared__ int bi[128];
+    const int m = blockIdx.x, t = threadIdx.x;
+    for (int n = t; n < natom; n += blockDim.x) {
+        double inv, adj;
+        becke_pair(atom_xyz, brad, ghost, size_adjust, m, n, inv, adj);
+        pair[(size_t)m * natom + n] = make_double2(inv, adj);
+        pairf[(size_t)m * natom + n] = make_float2((float)inv, (float)adj);
+        const double dx = atom_xyz[3 * m] - atom_xyz[3 * n], dy = atom_xyz[3 * m + 1] - atom_xyz[3 * n + 1],
+                     dz = atom_xyz[3 * m + 2] - atom_xyz[3 * n + 2];
+        nd[n] = n == m ? -1.0 : dx * dx + dy * dy + dz * dz;
+    }
+    for (int k = 0; k < kNearList && k < natom; ++k) {
+        __syncthreads();
+        double d = 1e300;
+        int b = natom;
+        for (int n = t; n < natom; n += blockDim.x)
+            if (nd[n] < d) d = nd[n], b = n;
+        bd[t] = d, bi[t] = b;
+        __syncthreads();
+        for (int s = 64; s > 0; s >>= 1) {
+            if (t < s && (bd[t + s] < bd[t] || (bd[t + s] == bd[t] && bi[t + s] < bi[t]))) bd[t] = bd[t + s], bi[t] = bi[t + s];
+            __syncthreads();
+        }
+        if (t == 0) {
+            const int w = bi[0] < natom ? bi[0] : m;  // only NaN coordinates leave none
+            near[m * kNearList + k] = w;
+            nd[w] = 1e301;
+        }
+    }
+}
+
+// The weights of k_becke at a fraction of its work, bit for bit the same. Far from most atoms m the
+// product P_m is so small against sum_m P_m that its exact value cannot change any rounding of the
+// sum. A CTA takes 32 points:
+//   1. the distances |r - R_n| (FP64, and an FP32 copy), each point's nearest atom c and an FP32
+//      estimate of P_c;
+//   2. the filter, a warp per m with a lane per point: an FP32 upper bound of P_m from the factors of
+//      c's nearest atoms alone (every factor is at most 1 and carries a margin for the FP32 rounding);
+//      m is dropped when the bound falls below 2^-80 of P_c;
+//   3. P_m of the kept (m, point) pairs (about 10 of 100 atoms), packed over the CTA's threads in the
+//      order of m, with the operations and the order of k_becke;
+//   4. per point the sum over m in ascending order, twice: with every dropped P_m at its lower and at
+//      its upper bound. FP64 addition is monotone, so when both sums agree to the bit they are the sum
+//      of all P_m; when they do not (a rounding boundary within 2^-73 of the sum) the point is summed
+//      over all atoms.
+// Bound by the issue of the FP32 filter and the FP64 pipe in step 3. Seeded chains on USER 75 x 302
+// grids, ncu (this form / one point per thread up to 48 atoms, a warp per point above): 30 atoms 0.57 /
+// 0.94 ms, 43 atoms 1.28 / 3.58, 77 atoms 5.9 / 17.4, 100 atoms 12.6 / 39.
+constexpr int kNearPts = 32, kNearThreads = 128, kNearCap = 1024;
+
+// P_m at the point whose distances are r[n * kNearPts]: the factors in ascending partner order, up
+// to a product of zero. Four factors are formed ahead of the products.
+__device__ __forceinline__ double becke_product(const double* r, const double2* __restrict__ pm, int m, int natom) {
+    const double rm = r[m * kNearPts];
+    auto factor = [&](int n) {
+        const double2 c = __ldg(pm + n);
+        double u = (rm - r[n * kNearPts]) * c.x;
+        u = u + c.y * (1.0 - u * u);
+        return becke_s(u);
+    };
+    double p = 1.0;
+    int n = 0;
+    for (; n + 4 <= natom && p != 0.0; n += 4) {
+        double s[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[k] = n + k == m ? 1.0 : factor(n + k);
+        const double q = (((p * s[0]) * s[1]) * s[2]) * s[3];
+        if (fabs(q) > 0.0) {
+            p = q;
+        } else {  // a zero (or a NaN that may follow one): factor by factor, up to the zero
+            for (int k = 0; k < 4 && p != 0.0; ++k) p *= s[k];
+        }
+    }
+    for (; n < natom && p != 0.0; ++n)
+        if (n != m) p *= factor(n);
+    return p;
+}
+
+// FP32 factor s(nu_mn) and a bound of its rounding error: |d mu| <= 1.8e-7 (r_m + r_n) / R_mn, at most
+// 3.4 times that in s, and 1e-6 for the polynomial.
+__device__ __forceinline__ float becke_s32(float rm, float rn, float2 c, float& margin) {
+    const float u = (rm - rn) * c.x;
+    float nu = fmaf(c.y, fmaf(-u, u, 1.0f), u);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) nu *= fmaf(-0.5f, nu * nu, 1.5f);
+    margin = fmaf((rm + rn) * c.x, 8e-7f, 1e-6f);
+    return fmaf(-0.5f, nu, 0.5f);
+}
+
+__global__ void __launch_bounds__(kNearThreads) k_becke_near(const double* __restrict__ atom_xyz, int natom,
+                                                             const double2* __restrict__ pair,
+                                                             const float2* __restrict__ pairf,
+                                                             const int* __restrict__ near, int64_t npts,
+                                                             const double* __restrict__ xyz,
+                                                             const int* __restrict__ owner,
+                                                             const double* __restrict__ w_single,
+                                                             double* __restrict__ w_out) {
+    extern __shared__ double sm[];
+    double* rr = sm;                                               // [natom][32]: |r - R_n|
+    double* pe = rr + (size_t)natom * kNearPts;                    // [kNearCap]: P_m of the kept pairs
+    float* rf = reinterpret_cast<float*>(pe + kNearCap);           // [natom][32]: FP32 copy of rr
+    uint32_t* mask = reinterpret_cast<uint32_t*>(rf + (size_t)natom * kNearPts);  // [natom]: points that keep m
+    int* off = reinterpret_cast<int*>(mask + natom);               // [natom + 1]: pairs before m
+    __shared__ float s_min[4][kNearPts], s_prod[4][kNearPts];
+    __shared__ int s_arg[4][kNearPts], s_c[kNearPts], s_end;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int nlist = min(kNearList, natom);
+    for (int64_t i0 = blockIdx.x * (int64_t)kNearPts; i0 < npts; i0 += (int64_t)gridDim.x * kNearPts) {
+        const int64_t i = i0 + lane;
         const bool live = i < npts;
+        const int own = live ? owner[i] : -1;
+        // 1. distances (lane = point), the nearest atom
         const double rx = live ? xyz[3 * i] : 0.0, ry = live ? xyz[3 * i + 1] : 0.0, rz = live ? xyz[3 * i + 2] : 0.0;
-        for (int m = 0; m < natom; ++m) {
+        float best = 3e38f;
+        int arg = 0;
+        for (int m = warp; m < natom; m += 4) {
             const double ax = atom_xyz[3 * m] - rx, ay = atom_xyz[3 * m + 1] - ry, az = atom_xyz[3 * m + 2] - rz;
-            rr[m * BECKE_T + t] = sqrt(ax * ax + ay * ay + az * az);
+            const double d = sqrt(ax * ax + ay * ay + az * az);
+            rr[m * kNearPts + lane] = d;
+            rf[m * kNearPts + lane] = (float)d;
+            if ((float)d < best) best = (float)d, arg = m;
         }
-        if (live) {
-            const int own = owner[i];
-            double tot = 0.0, pown = 0.0;
-            for (int m = 0; m < natom; ++m) {
-                const double rm = rr[m * BECKE_T + t];
-                const double* im = inv + (size_t)m * natom;
-                const double* am = adj + (size_t)m * natom;
-                double p = 1.0;
-                for (int n = 0; n < natom && p != 0.0; ++n) {
-                    if (n == m) continue;
-                    double u = (rm - rr[n * BECKE_T + t]) * __ldg(im + n);
-                    u = u + __ldg(am + n) * (1.0 - u * u);
-                    p *= becke_s(u);
-                }
-                tot += p;
-                if (m == own) pown = p;
+        s_min[warp][lane] = best, s_arg[warp][lane] = arg;
+        __syncthreads();
+        if (warp == 0) {
+            for (int w = 1; w < 4; ++w)
+                if (s_min[w][lane] < best) best = s_min[w][lane], arg = s_arg[w][lane];
+            s_c[lane] = arg;
+        }
+        __syncthreads();
+        const int c = s_c[lane];
+        {  // P_c in FP32, a quarter of its factors per warp
+            const float rc = rf[c * kNearPts + lane];
+            float p = 1.0f;
+            for (int n = warp; n < natom; n += 4) {
+                float e;
+                const float s = becke_s32(rc, rf[n * kNearPts + lane], __ldg(pairf + (size_t)c * natom + n), e);
+                p *= n == c ? 1.0f : s;
             }
-            w_out[i] = w_single[i] * (pown / tot);
+            s_prod[warp][lane] = p;
         }
+        __syncthreads();
+        // the drop threshold: 2^-80 P_c, and nothing dropped where P_c is near the end of the FP32 range
+        const float pc = s_prod[0][lane] * s_prod[1][lane] * s_prod[2][lane] * s_prod[3][lane];
+        const float thr = pc > 1e-10f ? pc * 8.271806e-25f : 0.0f;
+        // 2. the filter
+        for (int m = warp; m < natom; m += 4) {
+            const float rm = rf[m * kNearPts + lane];
+            float p = 1.0f;
+            bool drop = !live;
+            for (int k = 0; k < nlist; ++k) {
+                const int n = __ldg(near + c * kNearList + k);
+                float e;
+                const float s = becke_s32(rm, rf[n * kNearPts + lane], __ldg(pairf + (size_t)m * natom + n), e);
+                if (n != m) p *= s + e;
+                drop = drop || p < thr;
+                if (__all_sync(kAll, drop)) break;
+            }
+            const unsigned keep = __ballot_sync(kAll, live && (!drop || m == own));
+            if (lane == 0) mask[m] = keep;
+        }
+        __syncthreads();
+        if (warp == 0) {  // pairs before each m
+            int run = 0;
+            for (int m0 = 0; m0 < natom; m0 += 32) {
+                const int v = m0 + lane < natom ? __popc(mask[m0 + lane]) : 0;
+                int x = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kAll, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (m0 + lane < natom) off[m0 + lane] = run + x - v;
+                run += __shfl_sync(kAll, x, 31);
+            }
+            if (lane == 0) off[natom] = run;
+        }
+        __syncthreads();
+        // 3. and 4., in runs of whole atoms of at most kNearCap kept pairs
+        const double bound = 2.0 * (double)thr;
+        double lo = 0.0, hi = 0.0, pown = 0.0;
+        for (int ms = 0; ms < natom;) {
+            if (t == 0) {
+                int me = natom;
+                if (off[natom] - off[ms] > kNearCap) {  // the last atom end within the capacity
+                    int a = ms + 1, b = natom;
+                    while (b - a > 1) {
+                        const int mid = (a + b) / 2;
+                        if (off[mid] - off[ms] <= kNearCap) a = mid;
+                        else b = mid;
+                    }
+                    me = a;
+                }
+                s_end = me;
+            }
+            __syncthreads();
+            const int me = s_end, e0 = off[ms], ne = off[me] - e0;
+            for (int e = t; e < ne; e += kNearThreads) {
+                int a = ms, b = me;  // the atom of pair e0 + e: the last m with off[m] <= e0 + e
+                while (b - a > 1) {
+                    const int mid = (a + b) / 2;
+                    if (off[mid] <= e0 + e) a = mid;
+                    else b = mid;
+                }
+                unsigned bits = mask[a];
+                for (int k = e0 + e - off[a]; k > 0; --k) bits &= bits - 1;
+                pe[e] = becke_product(rr + __ffs(bits) - 1, pair + (size_t)a * natom, a, natom);
+            }
+            __syncthreads();
+            if (warp == 0 && live) {
+                for (int m = ms; m < me; ++m) {
+                    const unsigned bits = mask[m];
+                    if (bits >> lane & 1) {
+                        const double p = pe[off[m] - e0 + __popc(bits & ((1u << lane) - 1))];
+                        lo += p, hi += p;
+                        if (m == own) pown = p;
+                    } else {
+                        lo -= bound, hi += bound;
+                    }
+                }
+            }
+            __syncthreads();
+            ms = me;
+        }
+        if (warp == 0 && live) {
+            if (!(lo == hi)) {
+                lo = 0.0;
+                for (int m = 0; m < natom; ++m) {
+                    const double p = becke_product(rr + lane, pair + (size_t)m * natom, m, natom);
+                    lo += p;
+                    if (m == own) pown = p;
+                }
+            }
+            w_out[i] = w_single[i] * (pown / lo);
+        }
+        __syncthreads();  // the shared rows are rewritten for the next points
     }
 }
 
@@ -233,8 +442,7 @@ void launch_becke_pairs(const double* atom_xyz, const double* brad, int natom, i
 // operations and order of k_becke. The pair constants are read from the transposed table
 // (invT[n][m] = inv[m][n], adjT[n][m] = adj[m][n]), so that the lanes' loads for one partner n
 // are consecutive; per warp, the point's distances and the P_m sit in shared memory, 16 bytes
-// per atom. (k_becke_tab keeps one point per thread, with that point's natom distances per thread
-// in shared memory: at 100 atoms a few warps per SM and twice this kernel's time.)
+// per atom.
 constexpr int BECKE_WW = 8;  // warps per CTA
 __global__ void __launch_bounds__(32 * BECKE_WW) k_becke_warp(const double* __restrict__ atom_xyz, int natom,
                                                               const double* __restrict__ invT,
@@ -283,24 +491,31 @@ __global__ void k_transpose_n2(const double* __restrict__ a, double* __restrict_
     }
 }
 
-void launch_becke_tab(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
-                      double* inv, double* adj, int64_t npts, const double* xyz, const int* owner,
-                      const double* w_single, double* w_out, cudaStream_t s) {
-    k_becke_pairs<<<(natom * natom + 255) / 256, 256, 0, s>>>(atom_xyz, brad, ghost, natom, size_adjust, inv, adj);
-    int64_t blocks = (npts + BECKE_T - 1) / BECKE_T;
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    if (blocks < 1) blocks = 1;
-    const size_t smem = sizeof(double) * BECKE_T * natom;
-    cudaFuncSetAttribute(k_becke_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_becke_tab<<<(unsigned)blocks, BECKE_T, smem, s>>>(atom_xyz, natom, inv, adj, npts, xyz, owner, w_single,
-                                                        w_out);
+// Above this many atoms (32 points' distances and lists past 200 KiB of shared memory) the warp form.
+size_t becke_near_max_atoms() { return 480; }
+
+size_t becke_near_table_bytes(int natom) {
+    return (size_t)natom * natom * (sizeof(double2) + sizeof(float2)) + sizeof(int) * kNearList * (size_t)natom;
 }
 
-// Up to this many atoms the one-point-per-thread form; above it the warp form. Measured on seeded
-// chains with USER 75 x 302 grids (ncu durations, table form / warp form): 20 atoms 0.28 / 0.48 ms,
-// 32 atoms 1.07 / 1.15 ms, 48 atoms 4.57 / 4.66 ms, 64 atoms 15.8 / 8.2 ms, 100 atoms 77 / 39 ms.
-constexpr int kBeckeSmallAtoms = 48;
-size_t becke_small_atoms() { return kBeckeSmallAtoms; }
+void launch_becke_near(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
+                       void* tab, int64_t npts, const double* xyz, const int* owner, const double* w_single,
+                       double* w_out, cudaStream_t s) {
+    const size_t n2 = (size_t)natom * natom;
+    double2* pair = static_cast<double2*>(tab);
+    float2* pairf = reinterpret_cast<float2*>(pair + n2);
+    int* near = reinterpret_cast<int*>(pairf + n2);
+    k_becke_near_tables<<<natom, 128, sizeof(double) * natom, s>>>(atom_xyz, brad, ghost, natom, size_adjust, pair,
+                                                                    pairf, near);
+    const size_t smem = (size_t)natom * kNearPts * (sizeof(double) + sizeof(float)) + sizeof(double) * kNearCap +
+                        sizeof(int) * (2 * (size_t)natom + 1);
+    int64_t blocks = (npts + kNearPts - 1) / kNearPts;
+    if (blocks > 148 * 64) blocks = 148 * 64;
+    if (blocks < 1) blocks = 1;
+    cudaFuncSetAttribute(k_becke_near, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_becke_near<<<(unsigned)blocks, kNearThreads, smem, s>>>(atom_xyz, natom, pair, pairf, near, npts, xyz, owner,
+                                                              w_single, w_out);
+}
 
 size_t becke_warp_max_atoms() { return (200u * 1024u) / (2 * sizeof(double) * BECKE_WW); }
 
