@@ -790,7 +790,11 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
                 m.sh0 = sh0, m.ao0 = ao0;
                 m.nsh = (int)P.shells.size() - sh0;
                 m.nb = row;
-                m.nbp = mixed ? std::max(128, (row + 127) / 128 * 128) : std::max(8, (row + 7) / 8 * 8);
+                // FP64: rows of eight; BF16 split: its 128 x 128 tiles; INT8: 64, the width of an output
+                // tile and of a K slab (nb averages 228 on the 100-atom chain: 128-row padding adds a
+                // quarter to the slabs that the contractions copy and multiply)
+                const int q = !mixed ? 8 : (ctx->opt.split_terms == 10 ? 64 : 128);
+                m.nbp = std::max(q, (row + q - 1) / q * q);
                 blk_flops[bb] = 4.0 * double(m.nb) * m.nb * m.npts;
             }
         }
@@ -927,7 +931,7 @@ void build_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* ato
             for (int b = c.b0; b < c.b1; ++b) {  // Vxc: (group, 128-AO row tile, 64-AO column tile); cost ~ K = points
                 const BlockMeta& m = ctx->h_meta[b];
                 if (m.lead != b) continue;
-                for (int mt = 0; mt < m.nbp / 128; ++mt)
+                for (int mt = 0; mt < (m.nbp + 127) / 128; ++mt)
                     for (int nt = 0; nt < m.nbp / 64; ++nt) it.push_back({m.gn, make_int2(b, (mt << 16) | nt)});
             }
             std::stable_sort(it.begin(), it.end(), [](const auto& x, const auto& y) { return x.first > y.first; });

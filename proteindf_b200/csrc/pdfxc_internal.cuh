@@ -22,7 +22,7 @@ struct BlockMeta {
     int nsh;       // screened shells
     int ao0;       // first entry in blk_aos
     int nb;        // screened AOs
-    int nbp;       // rows of a workspace plane: nb rounded up to 8 (FP64) or to the 128-row tile (mixed)
+    int nbp;       // rows of a workspace plane: nb rounded up to 8 (FP64), 64 (INT8) or 128 (BF16 split)
     int npts;      // real points in the block (<= BLOCK_PTS)
     int lead;      // first block of this block's group (the block itself when ungrouped)
     int gn;        // blocks in the group; a group's blocks are consecutive and share one screened basis
@@ -365,7 +365,7 @@ __host__ __device__ inline MixedLayout mixed_layout(int nbp) {
 // over the group's points (e_z_g, written by the group's first block). P_sub is shared by the
 // group and lives only in the first block's region, after `total` (`total_lead` bytes in all).
 constexpr int OZ_SLICES = 4;
-// Largest K (screened AOs of a group, padded to 128) of the INT8 rho contraction: its order-5
+// Largest K (screened AOs of a group, padded to 64) of the INT8 rho contraction: its order-5
 // int32 accumulator sums four digit products of at most 128^2 per K index (exact in int32 while
 // 4 * 128^2 * K < 2^31, K < 32768), and the FP64 combination of the orders,
 // n = ((D2 256 + D3) 256 + D4) 256 + D5 with |D_k| <= (k - 1) 128^2 K, stays below 2^53 while
@@ -374,7 +374,7 @@ constexpr int OZ_MAX_K = 32512;
 struct OzLayout {
     size_t rad;                 // radial sums: S0 [nsh][128], then S1 [nsh][128]
     size_t phi1, phi1_plane;    // phi^T digits: rows = 128 points, K = nbp AOs
-    size_t zpack, zpack_plane;  // Z' digits: rows = nbp AOs (128-row tiles), K = 128 points
+    size_t zpack, zpack_plane;  // Z' digits: rows = nbp AOs in 128-row tiles, K = 128 points
     size_t e_pt, e_z_g, e_p;    // int exponents: per point, per AO row of the group (Z'), P_sub
     size_t total;
     size_t ppack, ppack_plane;  // P_sub digits of the group: rows = nbp, K = nbp (first block only)
@@ -390,15 +390,18 @@ __host__ __device__ inline OzLayout oz_layout(int nbp, int nsh) {
     L.phi1 = o;
     L.phi1_plane = (size_t)BLOCK_PTS * nbp;
     o = a256(o + OZ_SLICES * L.phi1_plane);
+    // nbp is a multiple of 64; the M tiles of Z' have 128 rows, and the last one's rows past nb are
+    // neither written nor used
+    const size_t zrows = ((size_t)nbp + 127) / 128 * 128;
     L.zpack = o;
-    L.zpack_plane = (size_t)nbp * BLOCK_PTS;
+    L.zpack_plane = zrows * BLOCK_PTS;
     o = a256(o + OZ_SLICES * L.zpack_plane);
     L.e_pt = o;
     o = a256(o + sizeof(int) * BLOCK_PTS);
     size_t* e[2] = {&L.e_z_g, &L.e_p};
     for (size_t* f : e) {
         *f = o;
-        o = a256(o + sizeof(int) * nbp);
+        o = a256(o + sizeof(int) * zrows);
     }
     L.total = o;
     L.ppack = o;
