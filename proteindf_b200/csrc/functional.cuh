@@ -12,7 +12,7 @@
 //   composites   SVWN (DfFunctional_SVWN.cpp:25-41), B88LYP (DfFunctional_B88LYP.cpp),
 //                B3LYP 0.80/0.72/0.19/0.81 (DfFunctional_B3LYP.cpp:25-150)
 //   PBE          not in the reference: pbe.cuh (Perdew-Burke-Ernzerhof 1996, PW92 correlation)
-// Transcendentals are CUDA's own pow/exp/log/atan/sqrt.
+// Transcendentals are CUDA's own cbrt/exp/log/atan/sqrt.
 #pragma once
 
 #include "pbe.cuh"
@@ -25,14 +25,17 @@ struct XcOut {
 
 namespace fdetail {
 
-__device__ __forceinline__ void slater(double ra, double rb, double& f, double& va, double& vb) {
-    const double k = 3.0 / (4.0 * M_PI);
-    const double ck = pow(k, 1.0 / 3.0);
+// Cube roots: the fractional powers of the densities (4/3, 8/3, 11/3, 1/6, ...) are products of
+// cbrt(rho) and whole powers, so a spin's cube root is taken once and shared by the parts of a
+// functional. (The functional kernels are bound by the FP64 pipe; pow costs several times cbrt. B3LYP
+// over 3.5 M points: 0.88 -> 0.25 ms.)
+__device__ __forceinline__ void slater(double ra, double rb, double ca, double cb, double& f, double& va, double& vb) {
+    const double ck = 0.62035049089940001667;  // (3 / (4 pi))^(1/3)
     const double coef = -(9.0 / 4.0) * ck * (2.0 / 3.0);
     const double dcoef = -3.0 * ck * (2.0 / 3.0);
-    f = coef * (pow(ra, 4.0 / 3.0) + pow(rb, 4.0 / 3.0));
-    va = dcoef * pow(ra, 1.0 / 3.0);
-    vb = dcoef * pow(rb, 1.0 / 3.0);
+    f = coef * (ra * ca + rb * cb);
+    va = dcoef * ca;
+    vb = dcoef * cb;
 }
 
 struct VwnPar {
@@ -66,18 +69,27 @@ __device__ __forceinline__ void vwn(bool v3, double ra, double rb, double& f, do
     const VwnPar F = v3 ? VwnPar{0.01554535, 20.1231, 101.578, -0.743294}
                         : VwnPar{0.01554535, 7.06042, 18.0578, -0.325};
     const VwnPar A = VwnPar{-1.0 / (6.0 * M_PI * M_PI), 1.13107, 13.0045, -0.0047584};
-    const double ec_coef = 4.0 / (9.0 * (pow(2.0, 1.0 / 3.0) - 1.0));
+    const double ec_coef = 1.70992093416136561766;  // 4 / (9 (2^(1/3) - 1))
     const double rho = ra + rb;
     const double inv = 1.0 / rho;
-    const double x = pow(3.0 / (4.0 * M_PI) * inv, 1.0 / 6.0);
+    const double x = sqrt(cbrt(3.0 / (4.0 * M_PI) * inv));
     const double zeta = (ra - rb) * inv;
-    const double ep = vwn_eps(P, x), ef = vwn_eps(F, x), ea = vwn_eps(A, x);
-    const double g = 9.0 / 8.0 * (pow(1.0 + zeta, 4.0 / 3.0) + pow(1.0 - zeta, 4.0 / 3.0) - 2.0);
+    const double ep = vwn_eps(P, x), epp = vwn_eps_prime(P, x);
+    if (zeta == 0.0) {  // no polarisation: g = g' = 0, only the paramagnetic fit remains
+        f = rho * ep;
+        const double v = ep + rho * (-x / (6.0 * rho) * epp);
+        va = (ra > 1.0e-20) ? v : 0.0;
+        vb = (rb > 1.0e-20) ? v : 0.0;
+        return;
+    }
+    const double ef = vwn_eps(F, x), ea = vwn_eps(A, x);
+    const double zp13 = cbrt(1.0 + zeta), zm13 = cbrt(1.0 - zeta);
+    const double g = 9.0 / 8.0 * ((1.0 + zeta) * zp13 + (1.0 - zeta) * zm13 - 2.0);
     const double z3 = zeta * zeta * zeta, z4 = z3 * zeta;
     const double EC = ep + ea * g * (1.0 + (ec_coef * (ef - ep) / ea - 1.0) * z4);
     f = rho * EC;
-    const double epp = vwn_eps_prime(P, x), efp = vwn_eps_prime(F, x), eap = vwn_eps_prime(A, x);
-    const double gp = 1.5 * (pow(1.0 + zeta, 1.0 / 3.0) - pow(1.0 - zeta, 1.0 / 3.0));
+    const double efp = vwn_eps_prime(F, x), eap = vwn_eps_prime(A, x);
+    const double gp = 1.5 * (zp13 - zm13);
     const double h = ec_coef * ((ef - ep) / ea) - 1.0;
     const double hp = ec_coef / ea * (efp - epp - (ef - ep) / ea * eap);
     const double t1 = -x / (6.0 * rho) * (epp + eap * g * (1.0 + h * z4) + ea * g * hp * z4);
@@ -86,57 +98,44 @@ __device__ __forceinline__ void vwn(bool v3, double ra, double rb, double& f, do
     vb = (rb > 1.0e-20) ? EC + rho * (t1 + t2c * (-inv * (1.0 + zeta))) : 0.0;
 }
 
-__device__ __forceinline__ double b88_g(double x, bool full) {
-    const double beta = 0.0042;
-    const double G = -(3.0 / 2.0) * pow(3.0 / (4.0 * M_PI), 1.0 / 3.0);
-    const double bx = beta * x;
-    const double as = log(x + sqrt(x * x + 1));
-    return (full ? G : 0.0) - (bx * x) / (1.0 + 6.0 * bx * as);
-}
-
-__device__ __forceinline__ double b88_gp(double x) {
-    const double beta = 0.0042;
-    const double bx = beta * x;
-    const double as = log(x + sqrt(x * x + 1));
-    const double M = 1.0 + 6.0 * bx * as;
-    return 6.0 * bx * bx * (as + x / sqrt(x * x + 1.0)) / (M * M) - 2.0 * bx / M;
-}
-
-__device__ __forceinline__ void b88(bool full, double ra, double rb, double gaa, double gbb, double& f,
-                                    double& va, double& vb, double& vgaa, double& vgbb) {
+// One spin of Becke 88 from its density r, cube root c and gamma g: energy, d/dr, d/dgamma (zero
+// potential where the density or gamma is below 1e-16, as the reference).
+__device__ __forceinline__ void b88_spin(bool full, double r, double c, double g, double& t, double& v, double& vg) {
     const double EPS = 1.0e-16;
-    double tA = 0.0, tB = 0.0;
-    if (ra > EPS) tA = pow(ra, 4.0 / 3.0) * b88_g(sqrt(gaa) / pow(ra, 4.0 / 3.0), full);
-    if (rb > EPS) tB = pow(rb, 4.0 / 3.0) * b88_g(sqrt(gbb) / pow(rb, 4.0 / 3.0), full);
+    t = v = vg = 0.0;
+    if (!(r > EPS)) return;
+    const double beta = 0.0042;
+    const double G = full ? -0.93052573634910002500 : 0.0;  // -(3/2) (3 / (4 pi))^(1/3)
+    const double r43 = r * c, sg = sqrt(g), x = sg / r43;
+    const double bx = beta * x, sq = sqrt(x * x + 1.0);
+    const double as = log(x + sq);
+    const double M = 1.0 + 6.0 * bx * as;
+    const double gx = G - (bx * x) / M;
+    t = r43 * gx;
+    if (!(g > EPS)) return;
+    const double gp = 6.0 * bx * bx * (as + x / sq) / (M * M) - 2.0 * bx / M;
+    v = 4.0 / 3.0 * c * (gx - x * gp);
+    vg = 0.5 / sg * gp;
+}
+
+__device__ __forceinline__ void b88(bool full, double ra, double rb, double ca, double cb, double gaa, double gbb,
+                                    double& f, double& va, double& vb, double& vgaa, double& vgbb) {
+    double tA, tB;
+    b88_spin(full, ra, ca, gaa, tA, va, vgaa);
+    if (rb == ra && gbb == gaa) tB = tA, vb = va, vgbb = vgaa;
+    else b88_spin(full, rb, cb, gbb, tB, vb, vgbb);
     f = tA + tB;
-    va = vb = vgaa = vgbb = 0.0;
-    if (ra > EPS && gaa > EPS) {
-        const double x = sqrt(gaa) / pow(ra, 4.0 / 3.0);
-        const double g = b88_g(x, full), gp = b88_gp(x);
-        va = 4.0 / 3.0 * pow(ra, 1.0 / 3.0) * (g - x * gp);
-        vgaa = 0.5 / sqrt(gaa) * gp;
-    }
-    if (rb > EPS && gbb > EPS) {
-        const double x = sqrt(gbb) / pow(rb, 4.0 / 3.0);
-        const double g = b88_g(x, full), gp = b88_gp(x);
-        vb = 4.0 / 3.0 * pow(rb, 1.0 / 3.0) * (g - x * gp);
-        vgbb = 0.5 / sqrt(gbb) * gp;
-    }
 }
 
 constexpr double LA = 0.04918, LB = 0.132, LC = 0.2533, LD = 0.349;
 
-__device__ __forceinline__ double lyp_coef() {
-    return pow(2.0, 11.0 / 3.0) * 0.3 * pow(3.0 * M_PI * M_PI, 2.0 / 3.0);
+constexpr double LCF = 36.462398978764778;  // 2^(11/3) 3/10 (3 pi^2)^(2/3)
+// omega and delta from m13 = rho^(-1/3)
+__device__ __forceinline__ double lyp_omega(double rho, double m13) {
+    const double m113 = m13 * m13 / (rho * rho * rho);  // rho^(-11/3)
+    return exp(-LC * m13) * m113 / (1.0 + LD * m13);
 }
-__device__ __forceinline__ double lyp_omega(double rho) {
-    const double m13 = pow(rho, -1.0 / 3.0);
-    return exp(-LC * m13) * pow(rho, -11.0 / 3.0) / (1.0 + LD * m13);
-}
-__device__ __forceinline__ double lyp_delta(double rho) {
-    const double m13 = pow(rho, -1.0 / 3.0);
-    return LC * m13 + LD * m13 / (1.0 + LD * m13);
-}
+__device__ __forceinline__ double lyp_delta(double m13) { return LC * m13 + LD * m13 / (1.0 + LD * m13); }
 __device__ __forceinline__ void lyp_dgamma(double rho, double ra, double rb, double om, double de,
                                            double& gaa, double& gab, double& gbb) {
     const double rab = ra * rb, abo = LA * LB * om;
@@ -145,34 +144,24 @@ __device__ __forceinline__ void lyp_dgamma(double rho, double ra, double rb, dou
     gab = -abo * (1.0 / 9.0 * rab * (47.0 - 7.0 * de) - 4.0 / 3.0 * rho * rho);
 }
 
-__device__ __forceinline__ double lyp_f(double ra, double rb, double gaa, double gab, double gbb) {
-    const double rho = ra + rb, rab = ra * rb;
-    const double om = lyp_omega(rho), de = lyp_delta(rho);
-    double daa, dab, dbb;
-    lyp_dgamma(rho, ra, rb, om, de, daa, dab, dbb);
-    const double t1 = -4.0 * LA / (1.0 + LD * pow(rho, -1.0 / 3.0)) * rab / rho;
-    const double t2 = -lyp_coef() * LA * LB * om * rab * (pow(ra, 8.0 / 3.0) + pow(rb, 8.0 / 3.0));
-    return t1 + t2 + daa * gaa + dab * gab + dbb * gbb;
-}
-
-__device__ __forceinline__ void lyp_v(double ra, double rb, double gaa, double gab, double gbb,
-                                      double& va, double& vb, double& vgaa, double& vgab,
-                                      double& vgbb) {
+// energy (every density) and potential (both densities above 1e-20)
+__device__ __forceinline__ void lyp(double ra, double rb, double ca, double cb, double gaa, double gab, double gbb,
+                                    double& f, double& va, double& vb, double& vgaa, double& vgab, double& vgbb) {
     const double TOL = 1.0e-20;
     va = vb = vgaa = vgab = vgbb = 0.0;
-    if (!(fabs(ra) > TOL && fabs(rb) > TOL)) return;
     const double rho = ra + rb, rab = ra * rb, ir = 1.0 / rho;
-    const double r13 = pow(rho, 1.0 / 3.0), rm13 = 1.0 / r13, rm43 = pow(rho, -4.0 / 3.0);
-    const double ra83 = pow(ra, 8.0 / 3.0), rb83 = pow(rb, 8.0 / 3.0);
-    const double om = lyp_omega(rho), abo = LA * LB * om;
-    const double omp = -1.0 / 3.0 * (ir * rm13) * om * (11.0 * r13 - LC - LD / (1.0 + LD * rm13));
-    const double de = lyp_delta(rho);
-    const double d1 = 1.0 + LD * pow(rho, -1.0 / 3.0);
-    const double dep = 1.0 / 3.0 * (LD * LD * pow(rho, -5.0 / 3.0) / (d1 * d1) - ir * de);
-    const double opo = -1.0 / 3.0 * pow(rho, -4.0 / 3.0) *
-                       (11.0 * pow(rho, 1.0 / 3.0) - LC - LD / (1.0 + LD * pow(rho, -1.0 / 3.0)));
+    const double r13 = cbrt(rho), rm13 = 1.0 / r13, rm43 = ir * rm13;
+    const double ra83 = ra * ra * ca * ca, rb83 = rb * rb * cb * cb;
+    const double om = lyp_omega(rho, rm13), abo = LA * LB * om;
+    const double de = lyp_delta(rm13);
+    const double d1 = 1.0 + LD * rm13;
     double daa, dab, dbb;
     lyp_dgamma(rho, ra, rb, om, de, daa, dab, dbb);
+    f = -4.0 * LA / d1 * rab / rho - LCF * abo * rab * (ra83 + rb83) + daa * gaa + dab * gab + dbb * gbb;
+    if (!(fabs(ra) > TOL && fabs(rb) > TOL)) return;
+    const double opo = -1.0 / 3.0 * rm43 * (11.0 * r13 - LC - LD / d1);  // omega' / omega
+    const double omp = opo * om;
+    const double dep = 1.0 / 3.0 * (LD * LD * rm43 * rm13 / (d1 * d1) - ir * de);
     const double ra_aa = opo * daa - abo * (1.0 / 9.0 * rb * (1.0 - 3.0 * de - (de - 11.0) * ra * ir) -
                                             1.0 / 9.0 * rab * ((3.0 + ra * ir) * dep + (de - 11.0) * rb * ir * ir));
     const double rb_bb = opo * dbb - abo * (1.0 / 9.0 * ra * (1.0 - 3.0 * de - (de - 11.0) * rb * ir) -
@@ -186,12 +175,11 @@ __device__ __forceinline__ void lyp_v(double ra, double rb, double gaa, double g
     const double rb_aa = opo * daa - abo * (1.0 / 9.0 * ra * (1.0 - 3.0 * de - (de - 11.0) * ra * ir) -
                                             1.0 / 9.0 * rab * ((3.0 + ra * ir) * dep - (de - 11.0) * ra * ir * ir) -
                                             2.0 * rb);
-    const double a1c = -4.0 * LA / (1.0 + LD * rm13) * rab / rho;
-    const double a1A = a1c * (1.0 / 3.0 * LD * rm43 / (1.0 + LD * rm13) + 1.0 / ra - ir);
-    const double a1B = a1c * (1.0 / 3.0 * LD * rm43 / (1.0 + LD * rm13) + 1.0 / rb - ir);
-    const double lc = lyp_coef();
-    const double a2A = -lc * LA * LB * (omp * rab * (ra83 + rb83) + om * rb * (11.0 / 3.0 * ra83 + rb83));
-    const double a2B = -lc * LA * LB * (omp * rab * (rb83 + ra83) + om * ra * (11.0 / 3.0 * rb83 + ra83));
+    const double a1c = -4.0 * LA / d1 * rab / rho;
+    const double a1A = a1c * (1.0 / 3.0 * LD * rm43 / d1 + 1.0 / ra - ir);
+    const double a1B = a1c * (1.0 / 3.0 * LD * rm43 / d1 + 1.0 / rb - ir);
+    const double a2A = -LCF * LA * LB * (omp * rab * (ra83 + rb83) + om * rb * (11.0 / 3.0 * ra83 + rb83));
+    const double a2B = -LCF * LA * LB * (omp * rab * (rb83 + ra83) + om * ra * (11.0 / 3.0 * rb83 + ra83));
     if (ra > TOL) {
         va = a1A + a2A + ra_aa * gaa + ra_ab * gab + ra_bb * gbb;
         vgaa = daa;
@@ -212,22 +200,22 @@ __device__ __forceinline__ XcOut eval_functional(int fn, double ra, double rb, d
     using namespace fdetail;
     XcOut o{0, 0, 0, 0, 0, 0};
     double f1, a1, b1, f2, a2, b2, g1, g2, g3, g4, g5;
+    const double ca = fn == 5 ? 0.0 : cbrt(ra), cb = fn == 5 ? 0.0 : (rb == ra ? ca : cbrt(rb));
     switch (fn) {
         case 0:  // SVWN
-            slater(ra, rb, f1, a1, b1);
+            slater(ra, rb, ca, cb, f1, a1, b1);
             vwn(false, ra, rb, f2, a2, b2);
             o.f = f1 + f2, o.va = a1 + a2, o.vb = b1 + b2;
             break;
         case 1:  // HFS
-            slater(ra, rb, o.f, o.va, o.vb);
+            slater(ra, rb, ca, cb, o.f, o.va, o.vb);
             break;
         case 2:  // HFB
-            b88(true, ra, rb, gaa, gbb, o.f, o.va, o.vb, o.vgaa, o.vgbb);
+            b88(true, ra, rb, ca, cb, gaa, gbb, o.f, o.va, o.vb, o.vgaa, o.vgbb);
             break;
         case 3:  // BLYP
-            b88(true, ra, rb, gaa, gbb, f1, a1, b1, g1, g3);
-            f2 = lyp_f(ra, rb, gaa, gab, gbb);
-            lyp_v(ra, rb, gaa, gab, gbb, a2, b2, g2, g4, g5);
+            b88(true, ra, rb, ca, cb, gaa, gbb, f1, a1, b1, g1, g3);
+            lyp(ra, rb, ca, cb, gaa, gab, gbb, f2, a2, b2, g2, g4, g5);
             o.f = f1 + f2, o.va = a1 + a2, o.vb = b1 + b2;
             o.vgaa = g1 + g2, o.vgab = g4, o.vgbb = g3 + g5;
             break;
@@ -238,11 +226,10 @@ __device__ __forceinline__ XcOut eval_functional(int fn, double ra, double rb, d
         }
         default: {  // B3LYP
             double fs, as, bs, fv, av, bv, fb, ab, bb, gba, gbb2, fl, al, bl, gla, glab, glb;
-            slater(ra, rb, fs, as, bs);
+            slater(ra, rb, ca, cb, fs, as, bs);
             vwn(true, ra, rb, fv, av, bv);
-            b88(false, ra, rb, gaa, gbb, fb, ab, bb, gba, gbb2);
-            fl = lyp_f(ra, rb, gaa, gab, gbb);
-            lyp_v(ra, rb, gaa, gab, gbb, al, bl, gla, glab, glb);
+            b88(false, ra, rb, ca, cb, gaa, gbb, fb, ab, bb, gba, gbb2);
+            lyp(ra, rb, ca, cb, gaa, gab, gbb, fl, al, bl, gla, glab, glb);
             o.f = 0.80 * fs + 0.72 * fb + 0.19 * fv + 0.81 * fl;
             o.va = 0.80 * as + 0.72 * ab + 0.19 * av + 0.81 * al;
             o.vb = 0.80 * bs + 0.72 * bb + 0.19 * bv + 0.81 * bl;

@@ -93,17 +93,24 @@ __host__ __device__ inline Dual5 dsqrt(const Dual5& a) {
     const double s = sqrt(a.v);
     return dchain(a, s, 0.5 / s);
 }
-// a^c for a > 0
-__host__ __device__ inline Dual5 dpow(const Dual5& a, double c) {
-    const double p = pow(a.v, c);
-    return dchain(a, p, c * p / a.v);
+// cube root of a > 0
+__host__ __device__ inline Dual5 dcbrt(const Dual5& a) {
+    const double c = cbrt(a.v);
+    return dchain(a, c, c / (3.0 * a.v));
+}
+// the dual of the spin-mirrored expression: the tangents of (rhoA, rhoB) and (gAA, gBB) exchanged
+__host__ __device__ inline Dual5 dmirror(const Dual5& a) {
+    Dual5 r = a;
+    r.d[0] = a.d[1], r.d[1] = a.d[0], r.d[2] = a.d[4], r.d[4] = a.d[2];
+    return r;
 }
 
 // scalar overloads so that the functional template also runs on plain doubles
 __host__ __device__ inline double dexp(double a) { return exp(a); }
 __host__ __device__ inline double dlog(double a) { return log(a); }
 __host__ __device__ inline double dsqrt(double a) { return sqrt(a); }
-__host__ __device__ inline double dpow(double a, double c) { return pow(a, c); }
+__host__ __device__ inline double dcbrt(double a) { return cbrt(a); }
+__host__ __device__ inline double dmirror(double a) { return a; }
 __host__ __device__ inline double dval(double a) { return a; }
 __host__ __device__ inline double dval(const Dual5& a) { return a.v; }
 __host__ __device__ inline double dconst_like(double, double c) { return c; }
@@ -118,6 +125,9 @@ constexpr double kMu = kBeta * kPi * kPi / 3.0;
 constexpr double kGamma = 0.03109069086965489503494086371273;  // (1 - ln 2) / pi^2
 constexpr double kGam = 0.5198420997897463295344212145565;      // 2^(4/3) - 2
 constexpr double kFzz = 8.0 / (9.0 * kGam);                        // f''(0)
+constexpr double kCbrt3Pi2 = 3.0936677262801359310;             // (3 pi^2)^(1/3)
+constexpr double kEx = -0.73855876638202240588;                 // -3/4 (3/pi)^(1/3)
+constexpr double kRs = 0.62035049089940001667;                  // (3 / (4 pi))^(1/3)
 constexpr double kTiny = 1e-30;
 
 template <class T>
@@ -131,19 +141,17 @@ __host__ __device__ inline T pw92_g(const T& rs, double A, double a1, double b1,
 template <class T>
 __host__ __device__ inline T exchange_spin(const T& rs_, const T& g_) {
     const T n = 2.0 * rs_;
-    const double cx = -0.75 * pow(3.0 / kPi, 1.0 / 3.0);
-    const T n43 = dpow(n, 4.0 / 3.0);
-    const T kf2n2 = dpow(3.0 * kPi * kPi * n, 2.0 / 3.0) * n * n;
-    const T s2 = g_ / kf2n2;
+    const T c = dcbrt(n), n43 = c * n;
+    const T s2 = g_ / (kCbrt3Pi2 * kCbrt3Pi2 * n43 * n43);
     const T fx = 1.0 + kKappa - kKappa / (1.0 + kMu * s2 / kKappa);
-    return 0.5 * cx * n43 * fx;
+    return 0.5 * kEx * n43 * fx;
 }
 
 template <class T>
 __host__ __device__ inline T pbe(const T& ra, const T& rb, const T& gaa, const T& gab, const T& gbb) {
     T f = dconst_like(ra, 0.0);
     if (dval(ra) > kTiny) f = f + exchange_spin(ra, gaa);
-    if (dval(rb) > kTiny) f = f + exchange_spin(rb, gbb);
+    if (dval(rb) > kTiny) f = f + (dval(rb) == dval(ra) && dval(gbb) == dval(gaa) ? dmirror(f) : exchange_spin(rb, gbb));
     const T rho = ra + rb;
     if (dval(rho) <= kTiny) return f;
     T zeta = (ra - rb) / rho;
@@ -151,17 +159,22 @@ __host__ __device__ inline T pbe(const T& ra, const T& rb, const T& gaa, const T
     const double zmax = 1.0 - 1e-12;
     if (dval(zeta) > zmax) zeta = dconst_like(ra, zmax);
     if (dval(zeta) < -zmax) zeta = dconst_like(ra, -zmax);
-    const T rs = dpow(3.0 / (4.0 * kPi) / rho, 1.0 / 3.0);
-    const T e0 = pw92_g(rs, 0.0310907, 0.21370, 7.5957, 3.5876, 1.6382, 0.49294);
-    const T e1 = pw92_g(rs, 0.01554535, 0.20548, 14.1189, 6.1977, 3.3662, 0.62517);
-    const T ac = -pw92_g(rs, 0.0168869, 0.11125, 10.357, 3.6231, 0.88026, 0.49671);
-    const T opz = 1.0 + zeta, omz = 1.0 - zeta;
-    const T fz = (dpow(opz, 4.0 / 3.0) + dpow(omz, 4.0 / 3.0) - 2.0) / kGam;
-    const T z4 = zeta * zeta * zeta * zeta;
-    const T ec = e0 + ac * fz * (1.0 - z4) / kFzz + (e1 - e0) * fz * z4;
-    const T phi = 0.5 * (dpow(opz, 2.0 / 3.0) + dpow(omz, 2.0 / 3.0));
+    const T r13 = dcbrt(rho);
+    const T rs = kRs / r13;
+    T ec = pw92_g(rs, 0.0310907, 0.21370, 7.5957, 3.5876, 1.6382, 0.49294);
+    T phi = dconst_like(ra, 1.0);
+    if (dval(zeta) != 0.0) {  // at zeta = 0, f(zeta) = 0 and phi = 1 with zero first derivatives
+        const T e0 = ec;
+        const T e1 = pw92_g(rs, 0.01554535, 0.20548, 14.1189, 6.1977, 3.3662, 0.62517);
+        const T ac = -pw92_g(rs, 0.0168869, 0.11125, 10.357, 3.6231, 0.88026, 0.49671);
+        const T opz = 1.0 + zeta, omz = 1.0 - zeta, op13 = dcbrt(opz), om13 = dcbrt(omz);
+        const T fz = (opz * op13 + omz * om13 - 2.0) / kGam;
+        const T z4 = zeta * zeta * zeta * zeta;
+        ec = e0 + ac * fz * (1.0 - z4) / kFzz + (e1 - e0) * fz * z4;
+        phi = 0.5 * (op13 * op13 + om13 * om13);
+    }
     const T phi3 = phi * phi * phi;
-    const T kf = dpow(3.0 * kPi * kPi * rho, 1.0 / 3.0);
+    const T kf = kCbrt3Pi2 * r13;
     const T ks2 = 4.0 * kf / kPi;
     const T grad2 = gaa + 2.0 * gab + gbb;
     const T t2 = grad2 / (4.0 * phi * phi * ks2 * rho * rho);
