@@ -276,6 +276,7 @@ void free_grid(pdfxc_ctx* c) {
     free_plan(c->gplan);
     free_plan(c->uplan);
     dev_free(c->d_rho_b), dev_free(c->d_blk_sum_b);
+    dev_free(c->d_rho_acc_b), dev_free(c->d_coef_b), dev_free(c->d_counters_b);
     c->rho_spin = 0;
     c->nblk = 0;
     c->npts = 0;
@@ -424,6 +425,7 @@ pdfxc_status pdfxc_set_system(pdfxc_ctx* ctx, int natom, const double* atom_xyz,
         dev_free(ctx->d_row_cols);  // a batch sets it after this call
         if (ctx->opt.precision == PDFXC_PRECISION_MIXED && ctx->opt.split_terms == 10) dev_alloc(&ctx->d_p_words, n2);
         dev_free(ctx->d_P_b), dev_free(ctx->d_V_b), dev_free(ctx->d_Vacc_b);  // open shell: sized on first use
+        dev_free(ctx->d_p_words_b), dev_free(ctx->d_p_rowexp_b);
         PDFXC_CUDA(cudaStreamSynchronize(s));
         free_grid(ctx);
         return PDFXC_OK;
@@ -2476,6 +2478,7 @@ void pdfxc_destroy(pdfxc_ctx* ctx) {
     dev_free(ctx->d_P), dev_free(ctx->d_V), dev_free(ctx->d_Vacc), dev_free(ctx->d_scalars), dev_free(ctx->d_err);
     dev_free(ctx->d_p_rowexp); dev_free(ctx->d_Vprev); dev_free(ctx->d_p_words); dev_free(ctx->d_row_cols);
     dev_free(ctx->d_P_b), dev_free(ctx->d_V_b), dev_free(ctx->d_Vacc_b), dev_free(ctx->d_scalars_b);
+    dev_free(ctx->d_p_words_b), dev_free(ctx->d_p_rowexp_b);
     for (auto& e : ctx->ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : ctx->stage_ev) cudaEventDestroy(e);
