@@ -377,7 +377,8 @@ void launch_ao_grad(const BasisView& b, const GridView& g, int blk0, int nblk, b
 void launch_grad_x(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, bool gga, char* ws,
                    cudaStream_t s) {
     // X = P_sub phi (LDA); X, Y_x, Y_y, Y_z = P_sub (phi, d_x phi, d_y phi, d_z phi) (GGA)
-    launch_gemm_x_planes(g, P, nao, blk0, nblk, max_nbp, 0, grad_phi_planes(gga), gga ? 4 : 1, ws, s);
+    for (int z = 0; z < (gga ? 4 : 1); ++z)
+        launch_gemm_x_plane(g, P, nao, blk0, nblk, max_nbp, z, grad_phi_planes(gga) + z, ws, s);
 }
 
 void launch_grad_point(const GridView& g, const int* ao_atom, const int* owner, int blk0, int nblk, int fn,

@@ -1,17 +1,18 @@
 // FP64 drop-in kernels of the XC build.
 //
-// Per block of up to 128 grid points with its screened AO list (nb AOs, padded
-// to nbp rows), one build runs
-//   ao_eval      phi[mu][p], grad phi[k][mu][p]                (DfCalcGridX.cpp:667-769)
-//   gemm_x       X = P_sub * phi, P_sub = P_A[aos, aos]
-//   rho_functional  rho_A(p) = sum_mu phi X, grad rho_A = 2 sum_mu grad phi X
-//                (:865-931), the functional, Exc and electron-count partials,
-//                and the per-point Vxc coefficients (:2056-2193, :2455-2500)
-//   gemm_v       Vacc[aos, aos] += phi * Z^T with
-//                Z[nu][p] = 0.5 w vrho phi + c . grad phi, c = w (2 vgAA + vgAB) grad rho_A
+// Per block of up to 128 grid points with its screened AO list (nb AOs), one build runs
+//   ao_eval      phi[mu][p] and, for a GGA, the shells' radial sums (DfCalcGridX.cpp:667-769)
+//   gemm_x       X = P_sub * phi, P_sub = P_A[aos, aos]; an LDA's epilogue sums rho per tile of rows
+//   rho_rad      rho_A(p) = sum_mu phi X, grad rho_A = 2 sum_mu grad phi X (:865-931) (GGA)
+//   functional   the functional, Exc and electron-count partials, and the
+//                per-point Vxc coefficients (:2056-2193, :2455-2500)
+//   z_rad        Z[nu][p] = 0.5 w vrho phi + c . grad phi, c = w (2 vgAA + vgAB) grad rho_A (GGA)
+//   gemm_v       Vacc[aos, aos] += phi * Z^T (an LDA scales phi by 0.5 w vrho instead)
 //   finish       V = Vacc + Vacc^T, FP64 block sums of Exc and the electron count
 // V = phi Z^T + Z phi^T reproduces the reference's element formula
 // V_ij += w vrho phi_i phi_j + phi_i (c . grad phi_j) + phi_j (c . grad phi_i).
+// The open shell runs the same kernels with two densities and two Z planes. The no-allocation build,
+// the density at points and the adjoint store X (rho_functional, gradient.cu).
 #include <cuda_runtime.h>
 
 #include "ao.cuh"
@@ -104,13 +105,22 @@ __device__ __forceinline__ void fp64_tile(int nb, int T, int i, int& r8, int& n8
 // ring of three shared-memory stages filled by asynchronous copies (one barrier per step), 8 warps
 // of all the tile's rows x 16 points (up to 8 x 2 DMMA tiles), so that a trimmed tile shortens every
 // warp alike. Bound by the FP64 tensor pipe. Planes are [nbp][128] arrays of the block's workspace:
-// source plane src0 + z, destination plane dst0 + z for blockIdx.z = z (the build: one plane, phi ->
-// X after the phi planes; the gradient: phi and its three derivatives -> X and Y_x, Y_y, Y_z).
+// source plane src0, destination plane dst0 (the gradient: phi and its derivatives too).
+// MODE (bits): X_STORE writes X. X_PHI (LDA) reduces it: the tile goes to shared memory and each thread
+// sums rho for its point and half of the tile's rows; the tile's sums go to row 4 tile of plane sum0
+// (nb >= 1 AOs give ceil(nb / 64) tiles and at least 8 rows). An LDA build needs the sums only, which
+// saves X's round trip through HBM and the pass over phi and X: (H2O)8 SVWN, with the symmetric Vxc
+// contraction below, 0.83 -> 0.64 ms. The same for a GGA (grad rho from the radial sums in the epilogue)
+// was slower, 21.5 -> 22.7 ms at 100 atoms: with two CTAs per SM the radial sums' latency is not hidden,
+// and k_rho_rad, a pass of its own, streams them.
 // Rows of phi at nb and beyond are not read. Row strides of 20 and 132 doubles keep the fragment
 // loads free of bank conflicts (4 g + t and g + 4 t distinct modulo 16).
 constexpr int GX_BM = 64, GX_BK = 16, GX_S = 3, GX_AS = GX_BK + 4, GX_BS = BLOCK_PTS + 4;
 constexpr int GX_STAGE = GX_BM * GX_AS + GX_BK * GX_BS;  // doubles
 constexpr int GX_SMEM = GX_S * GX_STAGE * 8;
+constexpr int GX_XS = BLOCK_PTS + 8;  // row of the X tile in shared memory: its 16-byte stores conflict-free
+static_assert(GX_BM * GX_XS <= GX_S * GX_STAGE, "the X tile reuses the stages");
+enum { X_STORE = 1, X_PHI = 2 };
 
 // one K step (kn of its 16 columns, in fours) of a warp's MC x 2 DMMA tiles
 template <int MC>
@@ -135,8 +145,9 @@ __device__ __forceinline__ void gx_step(const double* As, const double* Bs, int 
     }
 }
 
+template <int MODE>
 __global__ void __launch_bounds__(256, 2) k_gemm_x(GridView g, const double* __restrict__ P, int nao,
-                                                int blk0, char* ws, int src0, int dst0, int64_t t0) {
+                                                int blk0, char* ws, int src0, int dst0, int sum0, int64_t t0) {
     extern __shared__ __align__(16) double gx_sm[];
     int blk, ti;
     if (g.xtiles) {  // one CTA per tile of the list
@@ -152,8 +163,8 @@ __global__ void __launch_bounds__(256, 2) k_gemm_x(GridView g, const double* __r
     fp64_tile(m.nb, T, ti, r8, mc);
     const int m0 = r8 * 8;
     const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    const double* phi = reinterpret_cast<const double*>(ws + m.ws) + (size_t)(src0 + blockIdx.z) * plane;
-    double* X = reinterpret_cast<double*>(ws + m.ws) + (size_t)(dst0 + blockIdx.z) * plane;
+    const double* phi = reinterpret_cast<const double*>(ws + m.ws) + (size_t)src0 * plane;
+    double* X = reinterpret_cast<double*>(ws + m.ws) + (size_t)dst0 * plane;
     const int* aos = g.blk_aos + m.ao0;
 
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -214,13 +225,38 @@ __global__ void __launch_bounds__(256, 2) k_gemm_x(GridView g, const double* __r
             default: gx_step<1>(As, Bs, kn, acc);
         }
     }
+    if (MODE & X_STORE) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < mc)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    *reinterpret_cast<double2*>(X + (size_t)(m0 + i * 8 + gq) * BLOCK_PTS + warp * 16 + j * 8 + 2 * tq) =
+                        make_double2(acc[i][j][0], acc[i][j][1]);
+    }
+    if (MODE == X_STORE) return;
+    __syncthreads();  // the last stage is consumed (no copies are in flight)
+    double* Xs = gx_sm;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
         if (i < mc)
 #pragma unroll
             for (int j = 0; j < 2; ++j)
-                *reinterpret_cast<double2*>(X + (size_t)(m0 + i * 8 + gq) * BLOCK_PTS + warp * 16 + j * 8 + 2 * tq) =
+                *reinterpret_cast<double2*>(Xs + (i * 8 + gq) * GX_XS + warp * 16 + j * 8 + 2 * tq) =
                     make_double2(acc[i][j][0], acc[i][j][1]);
+    __syncthreads();
+    const int p = t & (BLOCK_PTS - 1), half = t >> 7;
+    const int rows = min(8 * mc, m.nb - m0), mid = (rows + 1) / 2;
+    double sum = 0.0;
+    for (int r = half ? mid : 0; r < (half ? rows : mid); ++r)
+        sum = fma(phi[(size_t)(m0 + r) * BLOCK_PTS + p], Xs[r * GX_XS + p], sum);
+    __syncthreads();  // the X tile is read
+    if (half) gx_sm[p] = sum;
+    __syncthreads();
+    if (!half) {
+        double* sums = reinterpret_cast<double*>(ws + m.ws) + sum0 * plane;
+        sums[(size_t)4 * ti * BLOCK_PTS + p] = sum + gx_sm[p];
+    }
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -295,21 +331,19 @@ __global__ void __launch_bounds__(BLOCK_PTS) k_rho_functional(GridView g, int bl
     }
 }
 
-// GGA closed-shell build without stored AO gradients. Layout of a block (doubles):
-// phi [nbp][128], X then Z [nbp][128], then the radial sums S0 [nsh][128] and S1 [nsh][128]
-// (block_ws_doubles_rad). k_ao_eval_rad writes phi and the radial sums; k_rho_functional_rad
-// forms phi and grad phi of every component from the radial sums (ao_from_radial, the
-// formulas of k_ao_eval) in row order, so rho and grad rho are summed as from stored planes,
-// and reads 2 nsh + nb rows per point instead of 5 nbp (and 2 nsh + nbp instead of 4 nbp for Z).
-// The shells (rows, angular momenta, atoms, primitives) are staged in shared memory, 64 at a time.
-__global__ void __launch_bounds__(256) k_ao_eval_rad(BasisView bas, GridView g, int blk0, char* ws) {
+// GGA builds without stored AO gradients. Layout of a block (doubles): phi [nbp][128], one plane per
+// spin [nbp][128] (X, then Z), then the radial sums S0 [nsh][128] and
+// S1 [nsh][128]. k_ao_eval_rad writes phi and the radial sums; everything that needs grad phi forms
+// it from them (ao.cuh). The shells (rows, angular momenta, atoms, primitives) are staged in shared
+// memory, 64 at a time.
+__global__ void __launch_bounds__(256) k_ao_eval_rad(BasisView bas, GridView g, int blk0, char* ws, int rad0) {
     const int blk = blk0 + blockIdx.x;
     const BlockMeta m = g.meta[blk];
     const int p = threadIdx.x & (BLOCK_PTS - 1);
     const int half = threadIdx.x >> 7;
     double* phi = reinterpret_cast<double*>(ws + m.ws);
     const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    double* S0p = phi + 2 * plane;
+    double* S0p = phi + rad0 * plane;
     double* S1p = S0p + (size_t)m.nsh * BLOCK_PTS;
     const int gp = blk * BLOCK_PTS + p;
     const double rx = g.px[gp], ry = g.py[gp], rz = g.pz[gp];
@@ -334,7 +368,6 @@ __global__ void __launch_bounds__(256) k_ao_eval_rad(BasisView bas, GridView g, 
             }
         }
     }
-    for (int r = m.nb + half; r < m.nbp; r += 2) phi[(size_t)r * BLOCK_PTS + p] = 0.0;
 }
 
 struct ShellStage {
@@ -353,207 +386,166 @@ __device__ __forceinline__ void stage_shells(const BasisView& bas, const GridVie
     }
 }
 
-__global__ void __launch_bounds__(BLOCK_PTS) k_rho_functional_rad(BasisView bas, GridView g, int blk0, int fn,
-                                                                  int incremental, double rho_cut, char* ws,
-                                                                  double* rho_store, double* coef, double* blk_sum) {
+// Prefetch into L1 of the line holding p (no wait, no register).
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+// The passes over the radial sums: 256 threads per block, the point is threadIdx.x % 128, the two
+// halves of the CTA take alternate shells. Bound by HBM; what a thread itself can keep in flight (one
+// shell's loads) is a third of what the bandwidth needs at 24 warps per SM, so the lines of the shell
+// kRadAhead shells on are prefetched into L1.
+constexpr int kRadAhead = 8;
+
+// rho and sum grad phi X per point of one spin (X in plane xplane, sums to acc_a) or both (xplane + 1,
+// acc_b; one pass over the radial sums). 100-atom ULTRA_FINE build: 2.8 ms (128 threads per block, no
+// prefetch: 3.0).
+template <int NS>
+__global__ void __launch_bounds__(256, 3) k_rho_rad(BasisView bas, GridView g, int blk0, const char* ws, int xplane,
+                                                    int rad0, double* acc_a, double* acc_b) {
     __shared__ ShellStage st;
+    __shared__ double s_half[NS][4][BLOCK_PTS];
     const int blk = blk0 + blockIdx.x;
     const BlockMeta m = g.meta[blk];
-    const int p = threadIdx.x;
+    const int p = threadIdx.x & (BLOCK_PTS - 1), half = threadIdx.x >> 7;
     const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    double* X = reinterpret_cast<double*>(ws + m.ws) + plane;
-    const double* S0p = X + plane;
+    const double* X = reinterpret_cast<const double*>(ws + m.ws) + xplane * plane + p;
+    const double* S0p = reinterpret_cast<const double*>(ws + m.ws) + rad0 * plane + p;
     const double* S1p = S0p + (size_t)m.nsh * BLOCK_PTS;
     const size_t gp = (size_t)blk * BLOCK_PTS + p;
     const double px = g.px[gp], py = g.py[gp], pz = g.pz[gp];
-    double rho = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-    double v[5], ax[5], ay[5], az[5];
+    double sum[NS][4];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) sum[s][0] = sum[s][1] = sum[s][2] = sum[s][3] = 0.0;
     for (int i0 = 0; i0 < m.nsh; i0 += 128) {
         __syncthreads();
         stage_shells(bas, g, m, i0, st);
         __syncthreads();
         const int kn = min(128, m.nsh - i0);
-        double S0n = S0p[(size_t)i0 * BLOCK_PTS + p], S1n = S1p[(size_t)i0 * BLOCK_PTS + p];
-        for (int k = 0; k < kn; ++k) {
-            const int i = i0 + k;
-            const double S0 = S0n, S1 = S1n;
-            if (k + 1 < kn) S0n = S0p[(size_t)(i + 1) * BLOCK_PTS + p], S1n = S1p[(size_t)(i + 1) * BLOCK_PTS + p];
-            const int L = st.lq[k], row0 = st.row0[k];
-            shell_components(L, px - st.ax[k], py - st.ay[k], pz - st.az[k], S0, S1, v, ax, ay, az);
+        for (int k = half; k < kn; k += 2) {
+            if (k + kRadAhead < kn) {
+                const int ka = k + kRadAhead, na = 2 * st.lq[ka] + 1;
+                prefetch_l1(S0p + (size_t)(i0 + ka) * BLOCK_PTS);
+                prefetch_l1(S1p + (size_t)(i0 + ka) * BLOCK_PTS);
+                for (int c = 0; c < na; ++c)
 #pragma unroll
-            for (int c = 0; c < 5; ++c) {
-                if (c < 2 * L + 1) {
-                    const double xv = X[(size_t)(row0 + c) * BLOCK_PTS + p];
-                    rho = fma(v[c], xv, rho);
-                    gx = fma(ax[c], xv, gx);
-                    gy = fma(ay[c], xv, gy);
-                    gz = fma(az[c], xv, gz);
-                }
+                    for (int s = 0; s < NS; ++s) prefetch_l1(X + s * plane + (size_t)(st.row0[ka] + c) * BLOCK_PTS);
+            }
+            const int L = st.lq[k], row0 = st.row0[k];
+            const double S0 = S0p[(size_t)(i0 + k) * BLOCK_PTS], S1 = S1p[(size_t)(i0 + k) * BLOCK_PTS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                double xv[5];
+#pragma unroll
+                for (int c = 0; c < 5; ++c) xv[c] = c < 2 * L + 1 ? X[s * plane + (size_t)(row0 + c) * BLOCK_PTS] : 0.0;
+                shell_rho<true>(L, px - st.ax[k], py - st.ay[k], pz - st.az[k], S0, S1, xv, sum[s][0], sum[s][1],
+                                sum[s][2], sum[s][3]);
             }
         }
     }
-    gx *= 2.0, gy *= 2.0, gz *= 2.0;
-    double* rs = rho_store + gp * 4;
-    if (incremental) {
-        rho += rs[0];
-        gx += rs[1], gy += rs[2], gz += rs[3];
-    }
-    rs[0] = rho, rs[1] = gx, rs[2] = gy, rs[3] = gz;
-    const double w = g.pw[gp];
-    double e = 0.0, a = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
-    if (w != 0.0 && rho > rho_cut) {
-        const double gam = gx * gx + gy * gy + gz * gz;
-        const XcOut o = eval_functional(fn, rho, rho, gam, gam, gam);
-        e = w * o.f;
-        a = 0.5 * w * o.va;
-        const double cc = w * (2.0 * o.vgaa + o.vgab);
-        cx = cc * gx, cy = cc * gy, cz = cc * gz;
-    }
-    double* cf = coef + gp * 4;
-    cf[0] = a, cf[1] = cx, cf[2] = cy, cf[3] = cz;
-    // Z[nu][p] = 0.5 w vrho phi + c . grad phi over X (every row of X has been read by this thread)
-    for (int i0 = 0; i0 < m.nsh; i0 += 128) {
-        __syncthreads();
-        stage_shells(bas, g, m, i0, st);
-        __syncthreads();
-        const int kn = min(128, m.nsh - i0);
-        double S0n = S0p[(size_t)i0 * BLOCK_PTS + p], S1n = S1p[(size_t)i0 * BLOCK_PTS + p];
-        for (int k = 0; k < kn; ++k) {
-            const int i = i0 + k;
-            const double S0 = S0n, S1 = S1n;
-            if (k + 1 < kn) S0n = S0p[(size_t)(i + 1) * BLOCK_PTS + p], S1n = S1p[(size_t)(i + 1) * BLOCK_PTS + p];
-            const int L = st.lq[k], row0 = st.row0[k];
-            shell_components(L, px - st.ax[k], py - st.ay[k], pz - st.az[k], S0, S1, v, ax, ay, az);
+    if (half)
 #pragma unroll
-            for (int c = 0; c < 5; ++c)
-                if (c < 2 * L + 1) X[(size_t)(row0 + c) * BLOCK_PTS + p] = a * v[c] + cx * ax[c] + cy * ay[c] + cz * az[c];
-        }
-    }
-    for (int r = m.nb; r < m.nbp; ++r) X[(size_t)r * BLOCK_PTS + p] = 0.0;
-    // block sums in FP64 (deterministic order)
-    __shared__ double red[2][BLOCK_PTS / 32];
-    double se = warp_sum(e), sn = warp_sum(w * rho);
-    if ((p & 31) == 0) red[0][p >> 5] = se, red[1][p >> 5] = sn;
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s_half[s][k][p] = sum[s][k];
     __syncthreads();
-    if (p == 0) {
-        double E = 0.0, N = 0.0;
-        for (int q = 0; q < BLOCK_PTS / 32; ++q) E += red[0][q], N += red[1][q];
-        blk_sum[2 * blk] = E;
-        blk_sum[2 * blk + 1] = N;
-    }
+    if (!half)
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) (s ? acc_b : acc_a)[gp * 4 + k] = sum[s][k] + s_half[s][k][p];
 }
 
-// The same build in three light kernels: rho and sum grad phi X per point (k_rho_rad, into
-// rho_acc), the functional (launch_functional_points), then Z over X (k_z_rad). Each loop over
-// the AO components holds few registers, so that enough warps hide the loads of X and of the
-// radial sums; k_rho_functional_rad keeps all three in one kernel of 138 registers.
-__global__ void __launch_bounds__(BLOCK_PTS, 6) k_rho_rad(BasisView bas, GridView g, int blk0, const char* ws,
-                                                       double* rho_acc) {
+// Z[nu][p] = 0.5 w vrho phi + c . grad phi for one spin (plane zplane, over X) or both (zplane + 1).
+// 100-atom ULTRA_FINE build: 2.35 ms (128 threads per block, no prefetch: 3.55).
+template <int NS>
+__global__ void __launch_bounds__(256, 3) k_z_rad(BasisView bas, GridView g, int blk0, const double* coef_a,
+                                                  const double* coef_b, char* ws, int zplane, int rad0) {
     __shared__ ShellStage st;
     const int blk = blk0 + blockIdx.x;
     const BlockMeta m = g.meta[blk];
-    const int p = threadIdx.x;
+    const int p = threadIdx.x & (BLOCK_PTS - 1), half = threadIdx.x >> 7;
     const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    const double* X = reinterpret_cast<const double*>(ws + m.ws) + plane;
-    const double* S0p = X + plane;
+    double* Z = reinterpret_cast<double*>(ws + m.ws) + zplane * plane + p;
+    const double* S0p = reinterpret_cast<const double*>(ws + m.ws) + rad0 * plane + p;
     const double* S1p = S0p + (size_t)m.nsh * BLOCK_PTS;
     const size_t gp = (size_t)blk * BLOCK_PTS + p;
     const double px = g.px[gp], py = g.py[gp], pz = g.pz[gp];
-    double rho = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+    double cf[NS][4];
+#pragma unroll
+    for (int s = 0; s < NS; ++s)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) cf[s][k] = (s ? coef_b : coef_a)[gp * 4 + k];
     for (int i0 = 0; i0 < m.nsh; i0 += 128) {
         __syncthreads();
         stage_shells(bas, g, m, i0, st);
         __syncthreads();
         const int kn = min(128, m.nsh - i0);
-        for (int k = 0; k < kn; ++k) {
-            const int i = i0 + k;
+        for (int k = half; k < kn; k += 2) {
+            if (k + kRadAhead < kn) {
+                prefetch_l1(S0p + (size_t)(i0 + k + kRadAhead) * BLOCK_PTS);
+                prefetch_l1(S1p + (size_t)(i0 + k + kRadAhead) * BLOCK_PTS);
+            }
             const int L = st.lq[k], row0 = st.row0[k];
-            double xv[5];
+            const double S0 = S0p[(size_t)(i0 + k) * BLOCK_PTS], S1 = S1p[(size_t)(i0 + k) * BLOCK_PTS];
+            const double x = px - st.ax[k], y = py - st.ay[k], z = pz - st.az[k];
 #pragma unroll
-            for (int c = 0; c < 5; ++c) xv[c] = c < 2 * L + 1 ? X[(size_t)(row0 + c) * BLOCK_PTS + p] : 0.0;
-            shell_rho<true>(L, px - st.ax[k], py - st.ay[k], pz - st.az[k], S0p[(size_t)i * BLOCK_PTS + p],
-                            S1p[(size_t)i * BLOCK_PTS + p], xv, rho, gx, gy, gz);
+            for (int s = 0; s < NS; ++s) {
+                double zc[5];
+                shell_z(L, x, y, z, S0, S1, cf[s][0], cf[s][1], cf[s][2], cf[s][3], zc);
+#pragma unroll
+                for (int c = 0; c < 5; ++c)
+                    if (c < 2 * L + 1) Z[s * plane + (size_t)(row0 + c) * BLOCK_PTS] = zc[c];
+            }
         }
     }
-    double* ra = rho_acc + gp * 4;
-    ra[0] = rho, ra[1] = gx, ra[2] = gy, ra[3] = gz;
-}
-
-__global__ void __launch_bounds__(BLOCK_PTS, 6) k_z_rad(BasisView bas, GridView g, int blk0, const double* coef,
-                                                     char* ws) {
-    __shared__ ShellStage st;
-    const int blk = blk0 + blockIdx.x;
-    const BlockMeta m = g.meta[blk];
-    const int p = threadIdx.x;
-    const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    double* Z = reinterpret_cast<double*>(ws + m.ws) + plane;
-    const double* S0p = Z + plane;
-    const double* S1p = S0p + (size_t)m.nsh * BLOCK_PTS;
-    const size_t gp = (size_t)blk * BLOCK_PTS + p;
-    const double px = g.px[gp], py = g.py[gp], pz = g.pz[gp];
-    const double* cf = coef + gp * 4;
-    const double a = cf[0], cx = cf[1], cy = cf[2], cz = cf[3];
-    double zc[5];
-    for (int i0 = 0; i0 < m.nsh; i0 += 128) {
-        __syncthreads();
-        stage_shells(bas, g, m, i0, st);
-        __syncthreads();
-        const int kn = min(128, m.nsh - i0);
-        for (int k = 0; k < kn; ++k) {
-            const int i = i0 + k;
-            const int L = st.lq[k], row0 = st.row0[k];
-            shell_z(L, px - st.ax[k], py - st.ay[k], pz - st.az[k], S0p[(size_t)i * BLOCK_PTS + p],
-                    S1p[(size_t)i * BLOCK_PTS + p], a, cx, cy, cz, zc);
-#pragma unroll
-            for (int c = 0; c < 5; ++c)
-                if (c < 2 * L + 1) Z[(size_t)(row0 + c) * BLOCK_PTS + p] = zc[c];
-        }
-    }
-    for (int r = m.nb; r < m.nbp; ++r) Z[(size_t)r * BLOCK_PTS + p] = 0.0;
 }
 
 // Vacc[aos[m]][aos[n]] += sum_p phi[m][p] Z[n][p]: CTA tile up to 64 x 64 AOs (fp64_tile in both
 // dimensions), K = 128 points in steps of 16 through a ring of three shared-memory stages, 4 warps as
 // 2 x 2 of up to 4 x 4 DMMA tiles. Bound by the FP64 tensor pipe. A tile of an odd number of rows of
 // eight gives its first warps more work, and a warp stays on its quarter of the SM, so the warps'
-// places in the tile rotate with the CTA. Z was formed in the place of X; rows at nb and beyond are
-// not read.
+// places in the tile rotate with the CTA. Rows at nb and beyond are not read.
+// LDA: Z = a phi with a = 0.5 w vrho per point, so there is no Z plane: B is phi again, scaled by a as
+// its fragments are loaded, and phi diag(a) phi^T is symmetric: only the tiles tm <= tn are computed
+// (the list ltiles), those off the diagonal counted twice (the finish adds Vacc^T).
 constexpr int GV_B = 64, GV_BK = 16, GV_S = 3, GV_AS = GV_BK + 4;
 constexpr int GV_STAGE = 2 * GV_B * GV_AS;  // doubles: A [m][k], B [n][k]
 constexpr int GV_SMEM = GV_S * GV_STAGE * 8;
 
-template <int MI, int NJ>
-__device__ __forceinline__ void gv_step(const double* As, const double* Bs, double (&acc)[4][4][2]) {
+template <bool LDA, int MI, int NJ>
+__device__ __forceinline__ void gv_step(const double* As, const double* Bs, const double* av, double (&acc)[4][4][2]) {
 #pragma unroll
     for (int kk = 0; kk < GV_BK; kk += 4) {
         double a[MI], b[NJ];
 #pragma unroll
         for (int i = 0; i < MI; ++i) a[i] = As[i * 8 * GV_AS + kk];
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) b[j] = Bs[j * 8 * GV_AS + kk];
+        for (int j = 0; j < NJ; ++j) b[j] = LDA ? av[kk] * Bs[j * 8 * GV_AS + kk] : Bs[j * 8 * GV_AS + kk];
 #pragma unroll
         for (int i = 0; i < MI; ++i)
 #pragma unroll
             for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
 }
-template <int MI>
-__device__ __forceinline__ void gv_step_n(int nj, const double* As, const double* Bs, double (&acc)[4][4][2]) {
+template <bool LDA, int MI>
+__device__ __forceinline__ void gv_step_n(int nj, const double* As, const double* Bs, const double* av,
+                                          double (&acc)[4][4][2]) {
     switch (nj) {
-        case 4: gv_step<MI, 4>(As, Bs, acc); break;
-        case 3: gv_step<MI, 3>(As, Bs, acc); break;
-        case 2: gv_step<MI, 2>(As, Bs, acc); break;
-        case 1: gv_step<MI, 1>(As, Bs, acc); break;
+        case 4: gv_step<LDA, MI, 4>(As, Bs, av, acc); break;
+        case 3: gv_step<LDA, MI, 3>(As, Bs, av, acc); break;
+        case 2: gv_step<LDA, MI, 2>(As, Bs, av, acc); break;
+        case 1: gv_step<LDA, MI, 1>(As, Bs, av, acc); break;
         default: break;
     }
 }
 
-__global__ void __launch_bounds__(128, 3) k_gemm_v(GridView g, int blk0, char* ws, int zplane, double* Vacc, int nao,
-                                                int tiles, int64_t t0) {
+template <bool LDA>
+__global__ void __launch_bounds__(128, 3) k_gemm_v(GridView g, int blk0, char* ws, int zplane, const double* coef,
+                                                double* Vacc, int nao, int tiles, int64_t t0) {
     extern __shared__ __align__(16) double gv_sm[];
+    __shared__ double s_a[LDA ? BLOCK_PTS : 1];
     int blk, tm, tn;
-    if (g.vtiles) {  // one CTA per tile of the list
-        const int2 it = g.vtiles[t0 + blockIdx.x];
+    if (LDA || g.vtiles) {  // one CTA per tile of the list
+        const int2 it = (LDA ? g.ltiles : g.vtiles)[t0 + blockIdx.x];
         blk = it.x, tm = it.y >> 16, tn = it.y & 0xFFFF;
     } else {
         blk = blk0 + blockIdx.y, tm = blockIdx.x / tiles, tn = blockIdx.x % tiles;
@@ -566,9 +558,11 @@ __global__ void __launch_bounds__(128, 3) k_gemm_v(GridView g, int blk0, char* w
     fp64_tile(m.nb, T, tn, nr8, nc);
     const int m0 = mr8 * 8, n0 = nr8 * 8;
     const double* phi = reinterpret_cast<const double*>(ws + m.ws);
-    const double* Z = phi + (size_t)zplane * m.nbp * BLOCK_PTS;
+    const double* Z = LDA ? phi : phi + (size_t)zplane * m.nbp * BLOCK_PTS;
     const int* aos = g.blk_aos + m.ao0;
     const int t = threadIdx.x, lane = t & 31, warp = ((t >> 5) + blockIdx.x) & 3;
+    // a (read after the first barrier of the loop), doubled for a tile that stands for its mirror too
+    if (LDA) s_a[t] = coef[4 * ((size_t)blk * BLOCK_PTS + t)] * (tm == tn ? 1.0 : 2.0);
     const int gq = lane >> 2, tq = lane & 3;
     const int wm8 = (warp >> 1) * ((mc + 1) >> 1), wn8 = (warp & 1) * ((nc + 1) >> 1);  // the warp's first rows of eight
     const int mi = warp >> 1 ? mc >> 1 : (mc + 1) >> 1, nj = warp & 1 ? nc >> 1 : (nc + 1) >> 1;
@@ -603,11 +597,12 @@ __global__ void __launch_bounds__(128, 3) k_gemm_v(GridView g, int blk0, char* w
         const double* st = gv_sm + (kt % GV_S) * GV_STAGE;
         const double* As = st + (wm8 * 8 + gq) * GV_AS + tq;
         const double* Bs = st + (GV_B + wn8 * 8 + gq) * GV_AS + tq;
+        const double* av = s_a + (LDA ? kt * GV_BK + tq : 0);
         switch (mi) {  // uniform over the warp
-            case 4: gv_step_n<4>(nj, As, Bs, acc); break;
-            case 3: gv_step_n<3>(nj, As, Bs, acc); break;
-            case 2: gv_step_n<2>(nj, As, Bs, acc); break;
-            case 1: gv_step_n<1>(nj, As, Bs, acc); break;
+            case 4: gv_step_n<LDA, 4>(nj, As, Bs, av, acc); break;
+            case 3: gv_step_n<LDA, 3>(nj, As, Bs, av, acc); break;
+            case 2: gv_step_n<LDA, 2>(nj, As, Bs, av, acc); break;
+            case 1: gv_step_n<LDA, 1>(nj, As, Bs, av, acc); break;
             default: break;
         }
     }
@@ -631,84 +626,6 @@ __global__ void k_symmetrize(const double* __restrict__ Vacc, double* V, int nao
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n2; e += (int64_t)gridDim.x * blockDim.x) {
         const int i = (int)(e / nao), j = (int)(e % nao);
         V[e] = Vacc[e] + Vacc[(int64_t)j * nao + i];
-    }
-}
-
-// Open shell (DfCalcGridX::calcRho_{LDA,GGA}_part(P_A, P_B, ...) :1891-1922, :1963-2016, and
-// buildVxc(gridMatrix, functional, F_A, F_B) :2093-2135, :2195-2278). One CTA per block,
-// one thread per point; X_A and X_B follow the phi planes. A point contributes when
-// rho_A or rho_B exceeds the cut-off. Per spin s the Vxc coefficients are the reference's:
-// 0.5 w vrho_s and c_s = w (2 vgamma_ss + vgamma_AB) grad rho_s (build_XC_Matrix,
-// :2455-2500, is called once per spin with that spin's gradient). Z_s replaces X_s.
-template <bool GGA>
-__global__ void __launch_bounds__(BLOCK_PTS) k_rho_functional_uks(GridView g, int blk0, int fn, int incremental,
-                                                                  double rho_cut, char* ws, double* rho_a,
-                                                                  double* rho_b, double* blk_sum, double* blk_sum_b) {
-    const int blk = blk0 + blockIdx.x;
-    const BlockMeta m = g.meta[blk];
-    const int p = threadIdx.x;
-    const int nplanes = GGA ? 4 : 1;
-    const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    const double* phi = reinterpret_cast<const double*>(ws + m.ws);
-    double* XA = const_cast<double*>(phi) + nplanes * plane;
-    double* XB = XA + plane;
-    double ra = 0.0, ax = 0.0, ay = 0.0, az = 0.0, rb = 0.0, bx = 0.0, by = 0.0, bz = 0.0;
-    for (int r = 0; r < m.nb; ++r) {
-        const size_t o = (size_t)r * BLOCK_PTS + p;
-        const double xa = XA[o], xb = XB[o];
-        ra = fma(phi[o], xa, ra);
-        rb = fma(phi[o], xb, rb);
-        if (GGA) {
-            const double dx = phi[plane + o], dy = phi[2 * plane + o], dz = phi[3 * plane + o];
-            ax = fma(dx, xa, ax), ay = fma(dy, xa, ay), az = fma(dz, xa, az);
-            bx = fma(dx, xb, bx), by = fma(dy, xb, by), bz = fma(dz, xb, bz);
-        }
-    }
-    ax *= 2.0, ay *= 2.0, az *= 2.0, bx *= 2.0, by *= 2.0, bz *= 2.0;
-    const size_t gp = (size_t)blk * BLOCK_PTS + p;
-    double* sa = rho_a + gp * 4;
-    double* sb = rho_b + gp * 4;
-    if (incremental) {
-        ra += sa[0], ax += sa[1], ay += sa[2], az += sa[3];
-        rb += sb[0], bx += sb[1], by += sb[2], bz += sb[3];
-    }
-    sa[0] = ra, sa[1] = ax, sa[2] = ay, sa[3] = az;
-    sb[0] = rb, sb[1] = bx, sb[2] = by, sb[3] = bz;
-    const double w = g.pw[gp];
-    double e = 0.0, a_a = 0.0, a_b = 0.0, ca[3] = {0.0, 0.0, 0.0}, cb[3] = {0.0, 0.0, 0.0};
-    if (w != 0.0 && (ra > rho_cut || rb > rho_cut)) {
-        const double gaa = ax * ax + ay * ay + az * az, gbb = bx * bx + by * by + bz * bz;
-        const double gab = ax * bx + ay * by + az * bz;
-        const XcOut o = eval_functional(fn, ra, rb, gaa, gab, gbb);
-        e = w * o.f;
-        a_a = 0.5 * w * o.va, a_b = 0.5 * w * o.vb;
-        if (GGA) {
-            const double cca = w * (2.0 * o.vgaa + o.vgab), ccb = w * (2.0 * o.vgbb + o.vgab);
-            ca[0] = cca * ax, ca[1] = cca * ay, ca[2] = cca * az;
-            cb[0] = ccb * bx, cb[1] = ccb * by, cb[2] = ccb * bz;
-        }
-    }
-    for (int r = 0; r < m.nbp; ++r) {
-        const size_t o = (size_t)r * BLOCK_PTS + p;
-        double za = a_a * phi[o], zb = a_b * phi[o];
-        if (GGA) {
-            const double dx = phi[plane + o], dy = phi[2 * plane + o], dz = phi[3 * plane + o];
-            za += ca[0] * dx + ca[1] * dy + ca[2] * dz;
-            zb += cb[0] * dx + cb[1] * dy + cb[2] * dz;
-        }
-        XA[o] = za, XB[o] = zb;
-    }
-    __shared__ double red[3][BLOCK_PTS / 32];
-    const double se = warp_sum(e), sna = warp_sum(w * ra), snb = warp_sum(w * rb);
-    if ((p & 31) == 0) red[0][p >> 5] = se, red[1][p >> 5] = sna, red[2][p >> 5] = snb;
-    __syncthreads();
-    if (p == 0) {
-        double E = 0.0, NA = 0.0, NB = 0.0;
-        for (int i = 0; i < BLOCK_PTS / 32; ++i) E += red[0][i], NA += red[1][i], NB += red[2][i];
-        blk_sum[2 * blk] = E;
-        blk_sum[2 * blk + 1] = NA;
-        blk_sum_b[2 * blk] = NB;
-        blk_sum_b[2 * blk + 1] = 0.0;
     }
 }
 
@@ -759,38 +676,50 @@ void launch_ao_eval(const BasisView& b, const GridView& g, int blk0, int nblk, b
 void launch_gemm_x(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp,
                           int nplanes, char* ws, cudaStream_t s) {
     // X follows the phi planes (1 for LDA, 4 with gradients)
-    launch_gemm_x_planes(g, P, nao, blk0, nblk, max_nbp, 0, nplanes, 1, ws, s);
+    launch_gemm_x_plane(g, P, nao, blk0, nblk, max_nbp, 0, nplanes, ws, s);
 }
 
-void launch_gemm_x_planes(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src0,
-                          int dst0, int nz, char* ws, cudaStream_t s) {
-    cudaFuncSetAttribute(k_gemm_x, cudaFuncAttributeMaxDynamicSharedMemorySize, GX_SMEM);
+template <int MODE>
+static void run_gemm_x(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src0, int dst0,
+                       int sum0, char* ws, cudaStream_t s) {
+    cudaFuncSetAttribute(k_gemm_x<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GX_SMEM);
     if (g.xtiles && g.h_xtile0) {
         const int64_t t0 = g.h_xtile0[blk0], n = g.h_xtile0[blk0 + nblk] - t0;
-        if (n > 0) k_gemm_x<<<dim3((unsigned)n, 1, nz), 256, GX_SMEM, s>>>(g, P, nao, blk0, ws, src0, dst0, t0);
+        if (n > 0) k_gemm_x<MODE><<<(unsigned)n, 256, GX_SMEM, s>>>(g, P, nao, blk0, ws, src0, dst0, sum0, t0);
         return;
     }
-    dim3 grid((max_nbp + GX_BM - 1) / GX_BM, nblk, nz);
-    k_gemm_x<<<grid, 256, GX_SMEM, s>>>(g, P, nao, blk0, ws, src0, dst0, 0);
+    dim3 grid((max_nbp + GX_BM - 1) / GX_BM, nblk);
+    k_gemm_x<MODE><<<grid, 256, GX_SMEM, s>>>(g, P, nao, blk0, ws, src0, dst0, sum0, 0);
 }
 
-void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, char* ws, cudaStream_t s) {
-    k_ao_eval_rad<<<nblk, 256, 0, s>>>(b, g, blk0, ws);
+void launch_gemm_x_plane(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src, int dst,
+                         char* ws, cudaStream_t s) {
+    run_gemm_x<X_STORE>(g, P, nao, blk0, nblk, max_nbp, src, dst, 0, ws, s);
 }
 
-void launch_rho_functional_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int fn, bool incremental,
-                               double rho_cut, char* ws, double* rho, double* coef, double* blk_sum, cudaStream_t s) {
-    k_rho_functional_rad<<<nblk, BLOCK_PTS, 0, s>>>(b, g, blk0, fn, incremental, rho_cut, ws, rho, coef, blk_sum);
+void launch_gemm_x_lda(const GridView& g, const double* P, int nao, int blk0, int nblk, int sum0, char* ws,
+                       cudaStream_t s) {
+    run_gemm_x<X_PHI>(g, P, nao, blk0, nblk, 0, 0, 0, sum0, ws, s);
 }
 
-void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const char* ws, double* rho_acc,
-                    cudaStream_t s) {
-    k_rho_rad<<<nblk, BLOCK_PTS, 0, s>>>(b, g, blk0, ws, rho_acc);
+void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int xplane, int rad0, const char* ws,
+                    double* acc_a, double* acc_b, cudaStream_t s) {
+    if (acc_b)
+        k_rho_rad<2><<<nblk, 256, 0, s>>>(b, g, blk0, ws, xplane, rad0, acc_a, acc_b);
+    else
+        k_rho_rad<1><<<nblk, 256, 0, s>>>(b, g, blk0, ws, xplane, rad0, acc_a, nullptr);
 }
 
-void launch_z_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const double* coef, char* ws,
-                  cudaStream_t s) {
-    k_z_rad<<<nblk, BLOCK_PTS, 0, s>>>(b, g, blk0, coef, ws);
+void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, char* ws, cudaStream_t s) {
+    k_ao_eval_rad<<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
+}
+
+void launch_z_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const double* coef_a, const double* coef_b,
+                  int zplane, int rad0, char* ws, cudaStream_t s) {
+    if (coef_b)
+        k_z_rad<2><<<nblk, 256, 0, s>>>(b, g, blk0, coef_a, coef_b, ws, zplane, rad0);
+    else
+        k_z_rad<1><<<nblk, 256, 0, s>>>(b, g, blk0, coef_a, nullptr, ws, zplane, rad0);
 }
 
 void launch_rho_functional(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
@@ -810,25 +739,22 @@ void launch_gemm_v(const GridView& g, int blk0, int nblk, int max_nbp, bool gga,
 void launch_gemm_v_plane(const GridView& g, int blk0, int nblk, int max_nbp, int zplane, char* ws, double* Vacc,
                          int nao, cudaStream_t s) {
     const int tiles = (max_nbp + GV_B - 1) / GV_B;
-    cudaFuncSetAttribute(k_gemm_v, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM);
+    cudaFuncSetAttribute(k_gemm_v<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM);
     if (g.vtiles && g.h_vtile0) {
         const int64_t t0 = g.h_vtile0[blk0], n = g.h_vtile0[blk0 + nblk] - t0;
-        if (n > 0) k_gemm_v<<<(unsigned)n, 128, GV_SMEM, s>>>(g, blk0, ws, zplane, Vacc, nao, tiles, t0);
+        if (n > 0)
+            k_gemm_v<false><<<(unsigned)n, 128, GV_SMEM, s>>>(g, blk0, ws, zplane, nullptr, Vacc, nao, tiles, t0);
         return;
     }
     dim3 grid(tiles * tiles, nblk);
-    k_gemm_v<<<grid, 128, GV_SMEM, s>>>(g, blk0, ws, zplane, Vacc, nao, tiles, 0);
+    k_gemm_v<false><<<grid, 128, GV_SMEM, s>>>(g, blk0, ws, zplane, nullptr, Vacc, nao, tiles, 0);
 }
 
-void launch_rho_functional_uks(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
-                               char* ws, double* rho_a, double* rho_b, double* blk_sum, double* blk_sum_b,
-                               cudaStream_t s) {
-    if (functional_is_gga(fn))
-        k_rho_functional_uks<true><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, ws, rho_a, rho_b,
-                                                               blk_sum, blk_sum_b);
-    else
-        k_rho_functional_uks<false><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, ws, rho_a, rho_b,
-                                                                blk_sum, blk_sum_b);
+void launch_gemm_v_lda(const GridView& g, int blk0, int nblk, const double* coef, char* ws, double* Vacc, int nao,
+                       cudaStream_t s) {
+    cudaFuncSetAttribute(k_gemm_v<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM);
+    const int64_t t0 = g.h_ltile0[blk0], n = g.h_ltile0[blk0 + nblk] - t0;
+    if (n > 0) k_gemm_v<true><<<(unsigned)n, 128, GV_SMEM, s>>>(g, blk0, ws, 0, coef, Vacc, nao, 0, t0);
 }
 
 void launch_block_sums(const double* blk_sum, int nblk, double* scalars, cudaStream_t s) {

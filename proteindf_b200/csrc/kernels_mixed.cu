@@ -162,15 +162,32 @@ __device__ __forceinline__ double warp_sum_m(double v) {
     return v;
 }
 
-// rho accumulators -> functional -> Vxc coefficients, per point (128 threads per block).
+// rho and sum_mu grad phi X of a point and spin
+template <bool GGA>
+__device__ __forceinline__ void load_rho(const GridView& g, int blk, int p, const RhoSource& src, int spin,
+                                         double d[4]) {
+    if (GGA || src.acc_a) {
+        const double* a = (spin ? src.acc_b : src.acc_a) + ((size_t)blk * BLOCK_PTS + p) * 4;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) d[k] = a[k];
+        return;
+    }
+    const BlockMeta m = g.meta[blk];
+    const double* z = reinterpret_cast<const double*>(src.ws + m.ws) + (size_t)(src.sum0 + spin) * m.nbp * BLOCK_PTS + p;
+    d[0] = d[1] = d[2] = d[3] = 0.0;
+    for (int t = 0; t < (m.nb + 63) / 64; ++t) d[0] += z[(size_t)4 * t * BLOCK_PTS];
+}
+
+// rho -> functional -> Vxc coefficients, per point (128 threads per block).
 template <bool GGA>
 __global__ void __launch_bounds__(BLOCK_PTS) k_functional_mixed(GridView g, int blk0, int fn, int incremental,
-                                                                double rho_cut, const double* rho_acc,
+                                                                double rho_cut, RhoSource src,
                                                                 double* rho_store, double* coef, double* blk_sum) {
     const int blk = blk0 + blockIdx.x;
     const int p = threadIdx.x;
     const size_t gp = (size_t)blk * BLOCK_PTS + p;
-    const double* ra = rho_acc + gp * 4;
+    double ra[4];
+    load_rho<GGA>(g, blk, p, src, 0, ra);
     double rho = ra[0], gx = 2.0 * ra[1], gy = 2.0 * ra[2], gz = 2.0 * ra[3];
     double* rs = rho_store + gp * 4;
     if (incremental) rho += rs[0], gx += rs[1], gy += rs[2], gz += rs[3];
@@ -207,19 +224,18 @@ __global__ void __launch_bounds__(BLOCK_PTS) k_functional_mixed(GridView g, int 
 // kernel); a point contributes when rho_A or rho_B exceeds the cut-off.
 template <bool GGA>
 __global__ void __launch_bounds__(BLOCK_PTS) k_functional_mixed_uks(GridView g, int blk0, int fn, int incremental,
-                                                                    double rho_cut, const double* rho_acc_a,
-                                                                    const double* rho_acc_b, double* rho_store_a,
+                                                                    double rho_cut, RhoSource src, double* rho_store_a,
                                                                     double* rho_store_b, double* coef_a, double* coef_b,
                                                                     double* blk_sum, double* blk_sum_b) {
     const int blk = blk0 + blockIdx.x;
     const int p = threadIdx.x;
     const size_t gp = (size_t)blk * BLOCK_PTS + p;
     double d[2][4];
-    const double* acc[2] = {rho_acc_a + gp * 4, rho_acc_b + gp * 4};
     double* st[2] = {rho_store_a + gp * 4, rho_store_b + gp * 4};
 #pragma unroll
     for (int sp = 0; sp < 2; ++sp) {
-        d[sp][0] = acc[sp][0], d[sp][1] = 2.0 * acc[sp][1], d[sp][2] = 2.0 * acc[sp][2], d[sp][3] = 2.0 * acc[sp][3];
+        load_rho<GGA>(g, blk, p, src, sp, d[sp]);
+        d[sp][1] *= 2.0, d[sp][2] *= 2.0, d[sp][3] *= 2.0;
         if (incremental)
             for (int k = 0; k < 4; ++k) d[sp][k] += st[sp][k];
         for (int k = 0; k < 4; ++k) st[sp][k] = d[sp][k];
@@ -1370,15 +1386,25 @@ size_t oz_smem_bytes() {
     return (size_t)oz_bar_off<MODE, S>() + (2 * S + 4 + 2 * kOzRing) * 8 + 16;
 }
 
-void launch_functional_points(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
-                              const double* rho_acc, double* rho_store, double* coef, double* blk_sum,
-                              cudaStream_t s) {
+void launch_functional(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
+                       const RhoSource& src, double* rho_store, double* coef, double* blk_sum, cudaStream_t s) {
     if (functional_is_gga(fn))
-        k_functional_mixed<true><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, rho_acc, rho_store,
-                                                            coef, blk_sum);
+        k_functional_mixed<true><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, src, rho_store, coef,
+                                                            blk_sum);
     else
-        k_functional_mixed<false><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, rho_acc, rho_store,
-                                                             coef, blk_sum);
+        k_functional_mixed<false><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, src, rho_store, coef,
+                                                             blk_sum);
+}
+
+void launch_functional_uks(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
+                           const RhoSource& src, double* rho_store_a, double* rho_store_b, double* coef_a,
+                           double* coef_b, double* blk_sum, double* blk_sum_b, cudaStream_t s) {
+    if (functional_is_gga(fn))
+        k_functional_mixed_uks<true><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, src, rho_store_a,
+                                                                rho_store_b, coef_a, coef_b, blk_sum, blk_sum_b);
+    else
+        k_functional_mixed_uks<false><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, src, rho_store_a,
+                                                                 rho_store_b, coef_a, coef_b, blk_sum, blk_sum_b);
 }
 
 // The failure path of the bounded waits, exercised without a fault: one thread waits on an
@@ -1470,12 +1496,8 @@ void oz_rho(const MixedArgs& a, cudaStream_t s) {
 }
 
 void oz_functional(const MixedArgs& a, cudaStream_t s) {
-    if (functional_is_gga(a.fn))
-        k_functional_mixed<true><<<a.nblk, BLOCK_PTS, 0, s>>>(a.g, a.blk0, a.fn, a.incremental, a.rho_cut, a.rho_acc,
-                                                              a.rho_store, a.coef, a.blk_sum);
-    else
-        k_functional_mixed<false><<<a.nblk, BLOCK_PTS, 0, s>>>(a.g, a.blk0, a.fn, a.incremental, a.rho_cut, a.rho_acc,
-                                                               a.rho_store, a.coef, a.blk_sum);
+    launch_functional(a.g, a.blk0, a.nblk, a.fn, a.incremental != 0, a.rho_cut, RhoSource{a.rho_acc}, a.rho_store,
+                      a.coef, a.blk_sum, s);
     oz_pack_z(a, s);
 }
 
@@ -1485,14 +1507,8 @@ void oz_pack_p(const MixedArgs& a, cudaStream_t s) {
 
 void oz_functional_uks(const MixedArgs& a, const double* rho_acc_b, double* rho_store_b, double* coef_b,
                        double* blk_sum_b, cudaStream_t s) {
-    if (functional_is_gga(a.fn))
-        k_functional_mixed_uks<true><<<a.nblk, BLOCK_PTS, 0, s>>>(a.g, a.blk0, a.fn, a.incremental, a.rho_cut,
-                                                                  a.rho_acc, rho_acc_b, a.rho_store, rho_store_b,
-                                                                  a.coef, coef_b, a.blk_sum, blk_sum_b);
-    else
-        k_functional_mixed_uks<false><<<a.nblk, BLOCK_PTS, 0, s>>>(a.g, a.blk0, a.fn, a.incremental, a.rho_cut,
-                                                                   a.rho_acc, rho_acc_b, a.rho_store, rho_store_b,
-                                                                   a.coef, coef_b, a.blk_sum, blk_sum_b);
+    launch_functional_uks(a.g, a.blk0, a.nblk, a.fn, a.incremental != 0, a.rho_cut, RhoSource{a.rho_acc, rho_acc_b},
+                          a.rho_store, rho_store_b, a.coef, coef_b, a.blk_sum, blk_sum_b, s);
 }
 
 void oz_pack_z(const MixedArgs& a, cudaStream_t s) {
@@ -1544,15 +1560,12 @@ void mixed_rho(const MixedArgs& a, cudaStream_t s) {
 }
 
 void mixed_functional(const MixedArgs& a, cudaStream_t s) {
-    if (functional_is_gga(a.fn)) {
-        k_functional_mixed<true><<<a.nblk, BLOCK_PTS, 0, s>>>(a.g, a.blk0, a.fn, a.incremental, a.rho_cut, a.rho_acc,
-                                                              a.rho_store, a.coef, a.blk_sum);
+    launch_functional(a.g, a.blk0, a.nblk, a.fn, a.incremental != 0, a.rho_cut, RhoSource{a.rho_acc}, a.rho_store,
+                      a.coef, a.blk_sum, s);
+    if (functional_is_gga(a.fn))
         k_pack_z<true><<<a.nblk, 256, 0, s>>>(a.g, a.blk0, a.coef, a.ws);
-    } else {
-        k_functional_mixed<false><<<a.nblk, BLOCK_PTS, 0, s>>>(a.g, a.blk0, a.fn, a.incremental, a.rho_cut, a.rho_acc,
-                                                               a.rho_store, a.coef, a.blk_sum);
+    else
         k_pack_z<false><<<a.nblk, 256, 0, s>>>(a.g, a.blk0, a.coef, a.ws);
-    }
 }
 
 void mixed_vxc(const MixedArgs& a, cudaStream_t s) {

@@ -193,8 +193,8 @@ pdfxc::BasisView basis_view(const pdfxc_ctx* c) {
 pdfxc::GridView grid_view(const pdfxc_ctx* c) {
     return {c->d_px,         c->d_py,         c->d_pz,          c->d_pw,         c->d_meta,
             c->d_blk_shells, c->d_blk_shell_row, c->d_blk_aos, c->d_blk_row_info, c->d_blk_row_geom,
-            c->d_xtiles,     c->d_vtiles,        c->h_xtile0.empty() ? nullptr : c->h_xtile0.data(),
-            c->h_vtile0.empty() ? nullptr : c->h_vtile0.data()};
+            c->d_xtiles,     c->d_vtiles,        c->d_ltiles,   c->h_xtile0.empty() ? nullptr : c->h_xtile0.data(),
+            c->h_vtile0.empty() ? nullptr : c->h_vtile0.data(), c->h_ltile0.empty() ? nullptr : c->h_ltile0.data()};
 }
 
 void drop_graph(pdfxc_ctx* c) {
@@ -214,16 +214,17 @@ void free_plan(pdfxc::Plan& p) {
 }
 
 // Per-block workspace offsets and chunks for `planes` FP64 planes of nbp x BLOCK_PTS per
-// block, within the workspace budget; recomputed only when the plane count changes.
-void ensure_plan(pdfxc_ctx* ctx, pdfxc::Plan& p, int planes) {
-    if (p.planes == planes) return;
+// block and `rad` radial sums of its shells, within the workspace budget; recomputed only
+// when the plane count changes.
+void ensure_plan(pdfxc_ctx* ctx, pdfxc::Plan& p, int planes, int rad) {
+    if (p.planes == planes && p.rad == rad) return;
     std::vector<BlockMeta> gm = ctx->h_meta;
     const size_t per_plane = sizeof(double) * BLOCK_PTS;
     p.chunks.clear();
     size_t off = 0, max_ws = 0;
     Chunk cur{0, 0, 0, 0};
     for (int b = 0; b < ctx->nblk; ++b) {
-        const size_t need = per_plane * (size_t)gm[b].nbp * planes;
+        const size_t need = per_plane * ((size_t)gm[b].nbp * planes + (size_t)rad * gm[b].nsh);
         if (off + need > ctx->opt.workspace_bytes && b > cur.b0) {
             cur.b1 = b;
             cur.ws_bytes = off;
@@ -252,7 +253,7 @@ void ensure_plan(pdfxc_ctx* ctx, pdfxc::Plan& p, int planes) {
         }
         p.ws_bytes = max_ws;
     }
-    p.planes = planes;
+    p.planes = planes, p.rad = rad;
 }
 
 void free_grid(pdfxc_ctx* c) {
@@ -271,8 +272,8 @@ void free_grid(pdfxc_ctx* c) {
     dev_free(c->d_owner), dev_free(c->d_ao_atom), dev_free(c->d_grad);
     dev_free(c->d_fdens), dev_free(c->d_wslot), dev_free(c->d_brad), dev_free(c->d_pair);
     dev_free(c->d_wscratch);
-    dev_free(c->d_xtiles), dev_free(c->d_vtiles);
-    c->h_xtile0.clear(), c->h_vtile0.clear();
+    dev_free(c->d_xtiles), dev_free(c->d_vtiles), dev_free(c->d_ltiles);
+    c->h_xtile0.clear(), c->h_vtile0.clear(), c->h_ltile0.clear();
     free_plan(c->gplan);
     free_plan(c->uplan);
     dev_free(c->d_rho_b), dev_free(c->d_blk_sum_b);
@@ -901,18 +902,22 @@ void build_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* ato
     }
     upload(&ctx->d_seg_blk, ctx->seg_blk, s);
     {  // the FP64 contractions' tile lists (up to 64 of a block's nb AOs each)
-        std::vector<int2> xt, vt;
-        ctx->h_xtile0.assign(1, 0), ctx->h_vtile0.assign(1, 0);
+        std::vector<int2> xt, vt, lt;
+        ctx->h_xtile0.assign(1, 0), ctx->h_vtile0.assign(1, 0), ctx->h_ltile0.assign(1, 0);
         for (int b = 0; b < nblk; ++b) {
             const int nt = (ctx->h_meta[b].nb + 63) / 64;
             for (int i = 0; i < nt; ++i) xt.push_back(make_int2(b, i));
             for (int i = 0; i < nt; ++i)
                 for (int j = 0; j < nt; ++j) vt.push_back(make_int2(b, (i << 16) | j));
+            for (int i = 0; i < nt; ++i)
+                for (int j = i; j < nt; ++j) lt.push_back(make_int2(b, (i << 16) | j));
             ctx->h_xtile0.push_back((int64_t)xt.size());
             ctx->h_vtile0.push_back((int64_t)vt.size());
+            ctx->h_ltile0.push_back((int64_t)lt.size());
         }
         upload(&ctx->d_xtiles, xt, s);
         upload(&ctx->d_vtiles, vt, s);
+        upload(&ctx->d_ltiles, lt, s);
     }
     ctx->h_grp.assign(grp_blk.begin(), grp_blk.end() - 1);
     upload(&ctx->d_grp, ctx->h_grp, s);
@@ -1390,26 +1395,25 @@ void enqueue_build(pdfxc_ctx* ctx, int fn, const double* d_PA, bool incremental)
             for (int k = 0; k < 5; ++k) PDFXC_CUDA(cudaEventRecord(e[k], s));
             continue;
         }
-        // per block: phi, X (then Z), and for GGA the shells' radial sums (block_ws_doubles_rad)
+        // per block: phi, X (then Z; an LDA's rho sums), and for GGA the radial sums (block_ws_doubles_rad)
         PDFXC_CUDA(cudaEventRecord(e[0], s));
-        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, cb0, nb, ws, s);
+        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, cb0, nb, 2, ws, s);
         else pdfxc::launch_ao_eval(bv, gv, cb0, nb, false, ws, 0, s);
         PDFXC_LAUNCHED("k_ao_eval");
         PDFXC_CUDA(cudaEventRecord(e[1], s));
-        pdfxc::launch_gemm_x(gv, d_PA, nao, cb0, nb, c.max_nbp, 1, ws, s);
+        if (gga) pdfxc::launch_gemm_x_plane(gv, d_PA, nao, cb0, nb, c.max_nbp, 0, 1, ws, s);
+        else pdfxc::launch_gemm_x_lda(gv, d_PA, nao, cb0, nb, 1, ws, s);
         PDFXC_LAUNCHED("k_gemm_x");
         PDFXC_CUDA(cudaEventRecord(e[2], s));
-        if (gga) {
-            pdfxc::launch_rho_rad(bv, gv, cb0, nb, ws, ctx->d_rho_acc, s);
-            pdfxc::launch_functional_points(gv, cb0, nb, fn, incremental, ctx->opt.rho_cutoff, ctx->d_rho_acc,
-                                            ctx->d_rho, ctx->d_coef, ctx->d_blk_sum, s);
-            pdfxc::launch_z_rad(bv, gv, cb0, nb, ctx->d_coef, ws, s);
-        } else
-            pdfxc::launch_rho_functional(gv, cb0, nb, fn, incremental, ctx->opt.rho_cutoff, ws, ctx->d_rho,
-                                         ctx->d_coef, ctx->d_blk_sum, s);
-        PDFXC_LAUNCHED("k_rho_functional");
+        if (gga) pdfxc::launch_rho_rad(bv, gv, cb0, nb, 1, 2, ws, ctx->d_rho_acc, nullptr, s);
+        pdfxc::launch_functional(gv, cb0, nb, fn, incremental, ctx->opt.rho_cutoff,
+                                 pdfxc::RhoSource{gga ? ctx->d_rho_acc : nullptr, nullptr, ws, 1}, ctx->d_rho,
+                                 ctx->d_coef, ctx->d_blk_sum, s);
+        if (gga) pdfxc::launch_z_rad(bv, gv, cb0, nb, ctx->d_coef, nullptr, 1, 2, ws, s);
+        PDFXC_LAUNCHED("rho / functional / Z");
         PDFXC_CUDA(cudaEventRecord(e[3], s));
-        pdfxc::launch_gemm_v_plane(gv, cb0, nb, c.max_nbp, 1, ws, ctx->d_Vacc, nao, s);
+        if (gga) pdfxc::launch_gemm_v_plane(gv, cb0, nb, c.max_nbp, 1, ws, ctx->d_Vacc, nao, s);
+        else pdfxc::launch_gemm_v_lda(gv, cb0, nb, ctx->d_coef, ws, ctx->d_Vacc, nao, s);
         PDFXC_LAUNCHED("k_gemm_v");
         PDFXC_CUDA(cudaEventRecord(e[4], s));
         launches += gga ? 6 : 4;
@@ -1515,14 +1519,18 @@ void collect_profile(pdfxc_ctx* ctx) {
     p.finish_ms = dt(ctx->stage_ev[last - 1], ctx->stage_ev[last]);
 }
 
-// The open-shell build's launches on ctx->stream (FP64 path): per chunk phi (and grad phi), X_A
-// and X_B, the open-shell functional with Z_A and Z_B in place of X, and the two Vxc
-// contractions. P_A, P_B in ctx->d_P, d_P_b; Vacc, Vacc_b zeroed. Returns the launch count.
+// The open-shell build's launches on ctx->stream (FP64 path): per chunk phi (and the radial sums), the
+// X contractions of both spins, rho of both in one pass (an LDA: in the contractions), the open-shell
+// functional, the Z planes of both spins in one pass (GGA), and the two Vxc contractions. P_A, P_B in ctx->d_P, d_P_b; Vacc, Vacc_b zeroed.
+// Returns the launch count.
 int64_t enqueue_uks_fp64(pdfxc_ctx* ctx, int functional, bool incremental) {
     const bool gga = pdfxc::functional_is_gga(functional);
-    const int nao = ctx->nao, nphi = gga ? 4 : 1;
+    const int nao = ctx->nao;
     cudaStream_t s = ctx->stream;
-    ensure_plan(ctx, ctx->uplan, nphi + 2);  // phi planes, X_A, X_B
+    constexpr int planes = 3;  // phi, X_A (then Z_A), X_B (then Z_B)
+    ensure_plan(ctx, ctx->uplan, planes, gga ? 2 : 0);
+    if (!ctx->d_coef_b) dev_alloc(&ctx->d_coef_b, (size_t)ctx->nblk * BLOCK_PTS * 4);
+    if (gga && !ctx->d_rho_acc_b) dev_alloc(&ctx->d_rho_acc_b, (size_t)ctx->nblk * BLOCK_PTS * 4);
     pdfxc::GridView gv = grid_view(ctx);
     gv.meta = ctx->uplan.d_meta;
     const pdfxc::BasisView bv = basis_view(ctx);
@@ -1531,15 +1539,30 @@ int64_t enqueue_uks_fp64(pdfxc_ctx* ctx, int functional, bool incremental) {
     for (const Chunk& c : ctx->uplan.chunks) {
         const int b0 = std::max(c.b0, ctx->blk_lo), nb = std::min(c.b1, ctx->blk_hi) - b0;
         if (nb <= 0) continue;
-        pdfxc::launch_ao_eval(bv, gv, b0, nb, gga, ws, 0, s);
-        pdfxc::launch_gemm_x_planes(gv, ctx->d_P, nao, b0, nb, c.max_nbp, 0, nphi, 1, ws, s);
-        pdfxc::launch_gemm_x_planes(gv, ctx->d_P_b, nao, b0, nb, c.max_nbp, 0, nphi + 1, 1, ws, s);
-        pdfxc::launch_rho_functional_uks(gv, b0, nb, functional, incremental, ctx->opt.rho_cutoff, ws, ctx->d_rho,
-                                         ctx->d_rho_b, ctx->d_blk_sum, ctx->d_blk_sum_b, s);
-        pdfxc::launch_gemm_v_plane(gv, b0, nb, c.max_nbp, nphi, ws, ctx->d_Vacc, nao, s);
-        pdfxc::launch_gemm_v_plane(gv, b0, nb, c.max_nbp, nphi + 1, ws, ctx->d_Vacc_b, nao, s);
+        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, b0, nb, planes, ws, s);
+        else pdfxc::launch_ao_eval(bv, gv, b0, nb, false, ws, 0, s);
+        if (gga) {
+            pdfxc::launch_gemm_x_plane(gv, ctx->d_P, nao, b0, nb, c.max_nbp, 0, 1, ws, s);
+            pdfxc::launch_gemm_x_plane(gv, ctx->d_P_b, nao, b0, nb, c.max_nbp, 0, 2, ws, s);
+            pdfxc::launch_rho_rad(bv, gv, b0, nb, 1, planes, ws, ctx->d_rho_acc, ctx->d_rho_acc_b, s);
+        } else {
+            pdfxc::launch_gemm_x_lda(gv, ctx->d_P, nao, b0, nb, 1, ws, s);
+            pdfxc::launch_gemm_x_lda(gv, ctx->d_P_b, nao, b0, nb, 2, ws, s);
+        }
+        pdfxc::launch_functional_uks(
+            gv, b0, nb, functional, incremental, ctx->opt.rho_cutoff,
+            gga ? pdfxc::RhoSource{ctx->d_rho_acc, ctx->d_rho_acc_b} : pdfxc::RhoSource{nullptr, nullptr, ws, 1},
+            ctx->d_rho, ctx->d_rho_b, ctx->d_coef, ctx->d_coef_b, ctx->d_blk_sum, ctx->d_blk_sum_b, s);
+        if (gga) {
+            pdfxc::launch_z_rad(bv, gv, b0, nb, ctx->d_coef, ctx->d_coef_b, 1, planes, ws, s);
+            pdfxc::launch_gemm_v_plane(gv, b0, nb, c.max_nbp, 1, ws, ctx->d_Vacc, nao, s);
+            pdfxc::launch_gemm_v_plane(gv, b0, nb, c.max_nbp, 2, ws, ctx->d_Vacc_b, nao, s);
+        } else {
+            pdfxc::launch_gemm_v_lda(gv, b0, nb, ctx->d_coef, ws, ctx->d_Vacc, nao, s);
+            pdfxc::launch_gemm_v_lda(gv, b0, nb, ctx->d_coef_b, ws, ctx->d_Vacc_b, nao, s);
+        }
         PDFXC_CUDA(cudaGetLastError());
-        launches += 6;
+        launches += gga ? 8 : 6;
     }
     return launches;
 }
@@ -2013,7 +2036,7 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
         }
         if (!ctx->d_owner) upload(&ctx->d_owner, ctx->h_owner, s);
         // gradient workspace: its own per-block offsets and chunks
-        ensure_plan(ctx, ctx->gplan, pdfxc::grad_workspace_planes(gga));
+        ensure_plan(ctx, ctx->gplan, pdfxc::grad_workspace_planes(gga), 0);
         const size_t nslots = (size_t)ctx->nblk * BLOCK_PTS;
         if (!ctx->d_grad) dev_alloc(&ctx->d_grad, 6 * (size_t)natom);
         if (!ctx->d_fdens) dev_alloc(&ctx->d_fdens, nslots);

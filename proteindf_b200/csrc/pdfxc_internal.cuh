@@ -64,10 +64,13 @@ struct GridView {
     // X = P_sub phi, {block, M << 16 | N} (64 x 64 tiles) for Vacc += phi Z^T, block by block; and
     // each block's first tile (prefix sums, host memory: read by the launchers, not the kernels).
     // Null (the no-allocation build): the launch covers max_nbp tiles per block, surplus CTAs exit.
+    // ltiles: the tiles M <= N of vtiles (an LDA's symmetric contraction).
     const int2* xtiles;
     const int2* vtiles;
+    const int2* ltiles;
     const int64_t* h_xtile0;
     const int64_t* h_vtile0;
+    const int64_t* h_ltile0;
 };
 
 // One AO row of a block's screened basis: the atom of its shell and its blk_row_info entry.
@@ -93,6 +96,7 @@ struct Plan {
     void* d_ws = nullptr;
     size_t ws_bytes = 0;
     int planes = -1;
+    int rad = 0;  // with this many radial sums of every shell after the planes
 };
 
 }  // namespace pdfxc
@@ -188,8 +192,8 @@ struct pdfxc_ctx {
     double* d_brad = nullptr;   // [natom]
     double* d_pair = nullptr;   // [2 * natom^2] Becke pair constants
     double* d_wscratch = nullptr;  // weight-term atom rows in device memory (above 400 atoms)
-    int2 *d_xtiles = nullptr, *d_vtiles = nullptr;  // GridView::xtiles, vtiles
-    std::vector<int64_t> h_xtile0, h_vtile0;         // GridView::h_xtile0, h_vtile0 (nblk + 1 each)
+    int2 *d_xtiles = nullptr, *d_vtiles = nullptr, *d_ltiles = nullptr;  // GridView::xtiles, vtiles, ltiles
+    std::vector<int64_t> h_xtile0, h_vtile0, h_ltile0;  // GridView::h_xtile0, ... (nblk + 1 each)
 
     // open-shell build (pdfxc_build_vxc_uks): beta-spin buffers beside the alpha ones above
     pdfxc::Plan uplan;
@@ -224,22 +228,35 @@ void launch_ao_eval(const BasisView& b, const GridView& g, int blk0, int nblk, b
                     char* ws, int max_nsh, cudaStream_t s);
 void launch_gemm_x(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp,
                    int nplanes, char* ws, cudaStream_t s);
-// the same contraction over nz planes: plane dst0 + z = P_sub * plane src0 + z
-void launch_gemm_x_planes(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src0,
-                          int dst0, int nz, char* ws, cudaStream_t s);
-// the GGA closed-shell build from radial sums (layout block_ws_doubles_rad)
-void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, char* ws, cudaStream_t s);
-void launch_rho_functional_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int fn, bool incremental,
-                               double rho_cut, char* ws, double* rho, double* coef, double* blk_sum, cudaStream_t s);
-void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const char* ws, double* rho_acc,
-                    cudaStream_t s);
-void launch_z_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const double* coef, char* ws,
-                  cudaStream_t s);
-// per point: rho = rho_acc (+ stored, incremental), grad rho = 2 rho_acc[1..3] (+ stored), the
-// functional, the Vxc coefficients and the block sums (kernels_mixed.cu)
-void launch_functional_points(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
-                              const double* rho_acc, double* rho_store, double* coef, double* blk_sum,
-                              cudaStream_t s);
+// plane dst = P_sub * plane src
+void launch_gemm_x_plane(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src, int dst,
+                         char* ws, cudaStream_t s);
+// the builds: phi and (GGA) the radial sums after rad0 planes; an LDA's X = P_sub phi
+// reduced to each tile's rho sum, in row 4 tile of plane sum0; a GGA's rho sums of one or both spins (acc_b, X in planes xplane, xplane + 1); the Z planes
+// of one or both spins; the LDA's contraction
+void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, char* ws, cudaStream_t s);
+void launch_gemm_x_lda(const GridView& g, const double* P, int nao, int blk0, int nblk, int sum0, char* ws, cudaStream_t s);
+void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int xplane, int rad0, const char* ws,
+                    double* acc_a, double* acc_b, cudaStream_t s);
+void launch_z_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const double* coef_a, const double* coef_b,
+                  int zplane, int rad0, char* ws, cudaStream_t s);
+void launch_gemm_v_lda(const GridView& g, int blk0, int nblk, const double* coef, char* ws, double* Vacc, int nao,
+                       cudaStream_t s);
+// where a point's rho and sum grad phi X are: an accumulator array [slot][4] per spin, or (acc null) the
+// tiles' sums of launch_gemm_x_lda in planes sum0 (alpha) and sum0 + 1 (beta) of the workspace
+struct RhoSource {
+    const double *acc_a, *acc_b;
+    const char* ws;
+    int sum0;
+};
+// per point: the rho sums (+ the stored densities, incremental), the functional, the Vxc coefficients and
+// the block sums (kernels_mixed.cu); the open shell: blk_sum = (Exc, N_alpha) pairs, blk_sum_b =
+// (N_beta, 0) pairs
+void launch_functional(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
+                       const RhoSource& src, double* rho_store, double* coef, double* blk_sum, cudaStream_t s);
+void launch_functional_uks(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
+                           const RhoSource& src, double* rho_store_a, double* rho_store_b, double* coef_a,
+                           double* coef_b, double* blk_sum, double* blk_sum_b, cudaStream_t s);
 void launch_rho_functional(const GridView& g, int blk0, int nblk, int fn, bool incremental,
                            double rho_cut, char* ws, double* rho, double* coef, double* blk_sum,
                            cudaStream_t s);
@@ -254,11 +271,6 @@ void launch_unpack_upper(const double* packed, int n, double* V, cudaStream_t s)
 // Vacc += phi Z^T with Z in plane zplane of each block's workspace
 void launch_gemm_v_plane(const GridView& g, int blk0, int nblk, int max_nbp, int zplane, char* ws, double* Vacc,
                          int nao, cudaStream_t s);
-// open shell: rho/grad rho of X_A, X_B (the two planes after phi), the functional, Z_A/Z_B over X_A/X_B;
-// blk_sum = (Exc, N_alpha) pairs, blk_sum_b = (N_beta, 0) pairs
-void launch_rho_functional_uks(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
-                               char* ws, double* rho_a, double* rho_b, double* blk_sum, double* blk_sum_b,
-                               cudaStream_t s);
 void launch_block_sums(const double* blk_sum, int nblk, double* scalars, cudaStream_t s);
 // per grid segment: out[2 i], out[2 i + 1] = sums over blocks [seg_blk[i], seg_blk[i+1])
 void launch_segment_sums(const double* blk_sum, const int* seg_blk, int nseg, double* out, cudaStream_t s);
@@ -316,8 +328,7 @@ __host__ __device__ inline size_t block_ws_doubles(int nbp, bool gga) {
     return (size_t)nbp * BLOCK_PTS * (gga ? 5 : 2);
 }
 
-// The closed-shell FP64 build: phi and X (then Z) planes, then the shells' radial sums S0, S1
-// (the GGA form; the LDA form uses the two planes only).
+// The closed-shell FP64 build: phi and X (then Z) planes, then the shells' radial sums S0, S1 (the GGA form; an LDA uses the planes only).
 __host__ __device__ inline size_t block_ws_doubles_rad(int nbp, int nsh) {
     return (size_t)BLOCK_PTS * (2 * (size_t)nbp + 2 * (size_t)nsh);
 }
