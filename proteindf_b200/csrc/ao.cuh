@@ -80,6 +80,23 @@ __device__ __forceinline__ void shell_radial_staged(const BasisView& bas, const 
     }
 }
 
+// S0, S1 and S2 = sum_k c_k a_k^2 e^{-a_k r^2} of a staged shell (second derivatives)
+__device__ __forceinline__ void shell_radial2_staged(const BasisView& bas, const ShellRec& r, double d2, double& S0,
+                                                     double& S1, double& S2) {
+    const int np = r.np < 0 ? bas.sh_nprim[r.sh] : r.np, p0 = r.np < 0 ? bas.sh_p0[r.sh] : 0;
+    const double* al_ = r.np < 0 ? bas.p_exp + p0 : r.alpha;
+    const double* cf_ = r.np < 0 ? bas.p_coef + p0 : r.coef;
+    S0 = 0.0, S1 = 0.0, S2 = 0.0;
+    for (int k = 0; k < np; ++k) {  // exponents ascend within a shell: the rest are cut too
+        const double al = al_[k];
+        if (al * d2 > 30.0) break;
+        const double e = cf_[k] * exp(-al * d2), ae = al * e;
+        S0 += e;
+        S1 += ae;
+        S2 += al * ae;
+    }
+}
+
 // Value and (GGA) gradient of component t at displacement (x, y, z) from the shell's atom.
 template <bool GGA>
 __device__ __forceinline__ void ao_from_radial(int t, double x, double y, double z, double S0, double S1, double& v,
@@ -185,6 +202,38 @@ __device__ __forceinline__ void shell_rho(int L, double x, double y, double z, d
         gy += S0 * Py - y * w;
         gz += S0 * Pz - z * w;
     }
+}
+
+// sum_c X_c (H_c c), H_c the second derivatives of the shell's component c, added to g: with
+// d_k d_l phi = A_kl S0 - 2 (x_l A_k + x_k A_l + delta_kl A) S1 + 4 x_k x_l A S2 and the sums PA, PG of
+// shell_rho, PH = sum_c X_c A_c'' (constant), B = c . r, it is
+// S0 PH c - 2 S1 (r (c . PG) + B PG + c PA) + 4 S2 r B PA.
+__device__ __forceinline__ void shell_hess(int L, double x, double y, double z, double S0, double S1, double S2,
+                                           const double X[5], double cx, double cy, double cz, double& gx, double& gy,
+                                           double& gz) {
+    double PA, Px = 0.0, Py = 0.0, Pz = 0.0, Hx = 0.0, Hy = 0.0, Hz = 0.0;
+    if (L == 0) {
+        PA = X[0];
+    } else if (L == 1) {
+        PA = x * X[0] + y * X[1] + z * X[2];
+        Px = X[0], Py = X[1], Pz = X[2];
+    } else {
+        const double s3 = 0.57735026918962576451;  // 1/sqrt(3)
+        const double u = X[3] - s3 * X[4], v = X[3] + s3 * X[4], w = 2.0 * s3 * X[4];
+        PA = X[0] * (x * y) + X[1] * (z * x) + X[2] * (y * z) + X[3] * (0.5 * (x * x - y * y)) +
+             X[4] * (s3 * (z * z - 0.5 * (x * x + y * y)));
+        Px = X[0] * y + X[1] * z + u * x;
+        Py = X[0] * x + X[2] * z - v * y;
+        Pz = X[1] * x + X[2] * y + w * z;
+        Hx = X[0] * cy + X[1] * cz + u * cx;
+        Hy = X[0] * cx + X[2] * cz - v * cy;
+        Hz = X[1] * cx + X[2] * cy + w * cz;
+    }
+    const double B = cx * x + cy * y + cz * z, t1 = 2.0 * S1;
+    const double q = 4.0 * S2 * B * PA - t1 * (cx * Px + cy * Py + cz * Pz);  // along r
+    gx += S0 * Hx - t1 * (B * Px + cx * PA) + q * x;
+    gy += S0 * Hy - t1 * (B * Py + cy * PA) + q * y;
+    gz += S0 * Hz - t1 * (B * Pz + cz * PA) + q * z;
 }
 
 }  // namespace pdfxc

@@ -1,15 +1,17 @@
 // XC nuclear gradient on the device (FP64): DfCalcGridX::energyGradient /
 // energyGradient_part (src/libpdf/DfCalcGridX.cpp:1073-1415).
 //
-// AO-centre term, per block of 128 points with its screened AO list:
-//   ao_grad      phi, grad phi and (GGA) the six second derivatives of every
-//                screened AO (the reference's getAOs/getDAOs/getD2AOs, :667-863)
-//   gemm_x       X = P_sub phi and (GGA) Y_k = P_sub d_k phi on the FP64 tensor cores
-//   grad_point   rho, grad rho, the functional, and per AO i on atom B
-//                G_i = a grad phi_i X_i + sum_k c_k (grad d_k phi_i X_i + grad phi_i Y_ki),
-//                a = w vrho, c = w (2 vgAA + vgAB) grad rho_A;
-//                grad[B] -= 4 G_i (the reference's -2 w, doubled for the closed shell),
-//                grad[owner] += 4 G_i (the grid moves with its atom).
+// AO-centre term, per block of 128 points with its screened AO list: with X = P_sub phi, the
+// coefficients a = 0.5 w vrho and c = w (2 vgAA + vgAB) grad rho_A, and Z = a phi + c . grad phi, the
+// contribution of AO i on atom B is
+//   G_i = 2 a grad phi_i X_i + sum_k c_k (grad d_k phi_i X_i + grad phi_i Y_ki),  Y_k = P_sub d_k phi,
+// and sum_k c_k Y_k = P_sub (c . grad phi) = P_sub Z - a X =: Y - a X, so one contraction of Z, which the
+// adjoint needs anyway, stands for the three of the derivatives, and
+//   G_i = grad phi_i (a X_i + Y_i) + (grad grad phi_i c) X_i,
+// formed from the shells' radial sums (no plane of derivatives is stored; the reference evaluates
+// getAOs / getDAOs / getD2AOs, :667-863);
+// grad[B] -= 4 G_i (the reference's -2 w, doubled for the closed shell), grad[owner] += 4 G_i (the grid
+// moves with its atom).
 // Grid-weight term, per point with coefficient c = w_single f (f the energy density):
 //                the derivative of the Becke partition omega_A = P_A / sum_i P_i with
 //                respect to every nucleus (Johnson, Gill and Pople, J. Chem. Phys. 98,
@@ -18,115 +20,12 @@
 //                src/libpdf/DfGenerateGrid.cpp:2357-2372, returns 0 unless |mu| > 1).
 #include <cuda_runtime.h>
 
-#include "functional.cuh"
+#include "ao.cuh"
 #include "pdfxc_internal.cuh"
 
 namespace pdfxc {
 
 namespace {
-
-// Angular polynomial A of component t (s; px py pz; dxy dxz dyz d(x2-y2) dz2, the
-// reference's prefactors, :103-141), its gradient and its second derivatives
-// (xx xy xz yy yz zz).
-__device__ __forceinline__ void ang_poly(int t, double x, double y, double z, double& A, double* Ak, double* Akl) {
-    const double s3 = 0.57735026918962576451;  // 1/sqrt(3)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) Ak[k] = 0.0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) Akl[k] = 0.0;
-    switch (t) {
-        case 0: A = 1.0; break;
-        case 1: A = x; Ak[0] = 1.0; break;
-        case 2: A = y; Ak[1] = 1.0; break;
-        case 3: A = z; Ak[2] = 1.0; break;
-        case 4: A = x * y; Ak[0] = y; Ak[1] = x; Akl[1] = 1.0; break;
-        case 5: A = z * x; Ak[0] = z; Ak[2] = x; Akl[2] = 1.0; break;
-        case 6: A = y * z; Ak[1] = z; Ak[2] = y; Akl[4] = 1.0; break;
-        case 7: A = 0.5 * (x * x - y * y); Ak[0] = x; Ak[1] = -y; Akl[0] = 1.0; Akl[3] = -1.0; break;
-        default:
-            A = s3 * (z * z - 0.5 * (x * x + y * y));
-            Ak[0] = -s3 * x; Ak[1] = -s3 * y; Ak[2] = 2.0 * s3 * z;
-            Akl[0] = -s3; Akl[3] = -s3; Akl[5] = 2.0 * s3;
-    }
-}
-
-// Workspace planes of one block ([nbp][128] doubles each): 0 phi, 1-3 grad phi,
-// 4-9 second derivatives (GGA); then X (and Y_x, Y_y, Y_z for GGA).
-__host__ __device__ inline int grad_phi_planes(bool gga) { return gga ? 10 : 4; }
-
-// One CTA per block, 256 threads: the point is threadIdx.x % 128, the two halves
-// of the CTA take alternate shells. d_k d_l (A e^{-a r^2}) =
-// (A_kl - 2a (x_l A_k + x_k A_l) - 2a delta_kl A + 4a^2 x_k x_l A) e^{-a r^2}.
-template <bool GGA>
-__global__ void __launch_bounds__(256) k_ao_grad(BasisView bas, GridView g, int blk0, char* ws) {
-    const int blk = blk0 + blockIdx.x;
-    const BlockMeta m = g.meta[blk];
-    const int p = threadIdx.x & (BLOCK_PTS - 1);
-    const int half = threadIdx.x >> 7;
-    double* out = reinterpret_cast<double*>(ws + m.ws);
-    const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    const int gp = blk * BLOCK_PTS + p;
-    const double rx = g.px[gp], ry = g.py[gp], rz = g.pz[gp];
-    constexpr int KL[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
-    for (int i = half; i < m.nsh; i += 2) {
-        const int s = g.blk_shells[m.sh0 + i];
-        const int row0 = g.blk_shell_row[m.sh0 + i];
-        const int at = bas.sh_atom[s];
-        const double q[3] = {rx - bas.atom_xyz[3 * at], ry - bas.atom_xyz[3 * at + 1], rz - bas.atom_xyz[3 * at + 2]};
-        const double d2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2];
-        const int L = bas.sh_l[s], n = 2 * L + 1, np = bas.sh_nprim[s], p0 = bas.sh_p0[s];
-        double v[5], gd[5][3], hd[5][6];
-#pragma unroll
-        for (int c = 0; c < 5; ++c) {
-            v[c] = 0.0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) gd[c][k] = 0.0;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) hd[c][k] = 0.0;
-        }
-        for (int k = 0; k < np; ++k) {
-            const double al = bas.p_exp[p0 + k];
-            if (al * d2 > 30.0) continue;  // TOOBIG, DfCalcGridX.cpp:42, :690
-            const double e = bas.p_coef[p0 + k] * exp(-al * d2);
-            const double a2 = 2.0 * al;
-#pragma unroll
-            for (int c = 0; c < 5; ++c) {
-                if (c >= n) break;
-                double A, Ak[3], Akl[6];
-                ang_poly(L * L + c, q[0], q[1], q[2], A, Ak, Akl);
-                v[c] += A * e;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) gd[c][k] += (Ak[k] - a2 * q[k] * A) * e;
-                if (GGA) {
-#pragma unroll
-                    for (int h = 0; h < 6; ++h) {
-                        const int kk = KL[h][0], ll = KL[h][1];
-                        double t = Akl[h] - a2 * (q[ll] * Ak[kk] + q[kk] * Ak[ll]) + a2 * a2 * q[kk] * q[ll] * A;
-                        if (kk == ll) t -= a2 * A;
-                        hd[c][h] += t * e;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 5; ++c) {
-            if (c >= n) break;
-            const size_t o = (size_t)(row0 + c) * BLOCK_PTS + p;
-            out[o] = v[c];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) out[(1 + k) * plane + o] = gd[c][k];
-            if (GGA) {
-#pragma unroll
-                for (int h = 0; h < 6; ++h) out[(4 + h) * plane + o] = hd[c][h];
-            }
-        }
-    }
-    // zero the padding rows of every plane
-    for (int r = m.nb + half; r < m.nbp; r += 2) {
-        const size_t o = (size_t)r * BLOCK_PTS + p;
-        for (int k = 0; k < grad_phi_planes(GGA); ++k) out[k * plane + o] = 0.0;
-    }
-}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -164,92 +63,66 @@ __device__ __forceinline__ void warp_add3_by_owner(double* grad, int own, double
     }
 }
 
-// One CTA (128 threads, one per point) per block. fdens receives the energy density
-// f(rho) per point slot (0 below the density cut-off, for the weight term), blk_sum the
-// block's Exc and electron-count partials, grad the AO-centre term (natom x 3). Every
-// derivative is scaled by `seed`, the cotangent of Exc (1 for the plain gradient). With
-// want_z the adjoint of the density with respect to P replaces X in place:
-// Z_i = 0.5 a phi_i + c . grad phi_i (a = seed w vrho, c = seed w (2 vgAA + vgAB) grad rho),
-// so that phi Z^T + Z phi^T summed over the blocks is seed dExc/dP.
+// One CTA per block, 256 threads: the point is threadIdx.x % 128, the halves of the CTA take the
+// first and the second half of the block's shells (runs of one atom's shells stay together but for
+// one). Reads X, Y and the radial sums once; 16 warps per SM (its registers) do not cover the latency
+// (L1 prefetches of the shells ahead changed nothing). 30-atom PBE chain, 477k points: 0.97 ms, for 3.0 ms
+// of the stored second derivatives (1.2) and the pass over 14 planes (1.8), and three contractions less.
 template <bool GGA>
-__global__ void __launch_bounds__(BLOCK_PTS) k_grad_point(GridView g, const int* __restrict__ ao_atom,
-                                                          const int* __restrict__ owner, int blk0, int fn,
-                                                          double rho_cut, char* ws, double seed, int want_z,
-                                                          double* fdens, double* blk_sum, double* grad) {
+__global__ void __launch_bounds__(256, 2) k_grad_atoms(BasisView bas, GridView g, const int* __restrict__ owner,
+                                                       int blk0, const double* __restrict__ coef, const char* ws,
+                                                       double* grad) {
+    __shared__ double s_xyz[3][128];
+    __shared__ int s_row[128], s_l[128], s_at[128];
     const int blk = blk0 + blockIdx.x;
     const BlockMeta m = g.meta[blk];
-    const int p = threadIdx.x;
+    const int p = threadIdx.x & (BLOCK_PTS - 1), half = threadIdx.x >> 7;
     const size_t plane = (size_t)m.nbp * BLOCK_PTS;
-    const double* phi = reinterpret_cast<const double*>(ws + m.ws);
-    double* X = reinterpret_cast<double*>(ws + m.ws) + grad_phi_planes(GGA) * plane;
-    double rho = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-    for (int r = 0; r < m.nb; ++r) {
-        const size_t o = (size_t)r * BLOCK_PTS + p;
-        const double x = X[o];
-        rho = fma(phi[o], x, rho);
-        if (GGA) {
-            gx = fma(phi[plane + o], x, gx);
-            gy = fma(phi[2 * plane + o], x, gy);
-            gz = fma(phi[3 * plane + o], x, gz);
-        }
-    }
-    gx *= 2.0, gy *= 2.0, gz *= 2.0;
+    const double* base = reinterpret_cast<const double*>(ws + m.ws) + p;
+    const double* X = base + GRAD_X * plane;
+    const double* Y = base + GRAD_Y * plane;
+    const double* S0p = base + (GGA ? 4 : 3) * plane;
+    const double* S1p = S0p + (size_t)m.nsh * BLOCK_PTS;
+    const double* S2p = S1p + (size_t)m.nsh * BLOCK_PTS;
     const size_t gp = (size_t)blk * BLOCK_PTS + p;
-    const double w = g.pw[gp];
-    double f = 0.0, a = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
-    if (w != 0.0 && rho > rho_cut) {
-        const double gam = GGA ? gx * gx + gy * gy + gz * gz : 0.0;
-        const XcOut o = eval_functional(fn, rho, rho, gam, gam, gam);
-        f = o.f;
-        a = seed * w * o.va;
-        if (GGA) {
-            const double cc = seed * w * (2.0 * o.vgaa + o.vgab);
-            cx = cc * gx, cy = cc * gy, cz = cc * gz;
+    const double px = g.px[gp], py = g.py[gp], pz = g.pz[gp];
+    const double a = coef[gp * 4], cx = coef[gp * 4 + 1], cy = coef[gp * 4 + 2], cz = coef[gp * 4 + 3];
+    double tx = 0.0, ty = 0.0, tz = 0.0;  // all shells of this thread
+    for (int i0 = 0; i0 < m.nsh; i0 += 128) {
+        const int kn = min(128, m.nsh - i0);
+        __syncthreads();
+        for (int k = threadIdx.x; k < kn; k += 256) {
+            const int sh = g.blk_shells[m.sh0 + i0 + k], at = bas.sh_atom[sh];
+            s_row[k] = g.blk_shell_row[m.sh0 + i0 + k], s_l[k] = bas.sh_l[sh], s_at[k] = at;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s_xyz[c][k] = bas.atom_xyz[3 * at + c];
+        }
+        __syncthreads();
+        const int k1 = half ? kn : (kn + 1) / 2;
+        int k = half ? (kn + 1) / 2 : 0;
+        while (k < k1) {
+            const int at = s_at[k];  // uniform over a warp
+            const double x = px - s_xyz[0][k], y = py - s_xyz[1][k], z = pz - s_xyz[2][k];
+            double ax = 0.0, ay = 0.0, az = 0.0, unused = 0.0;
+            for (; k < k1 && s_at[k] == at; ++k) {
+                const int L = s_l[k], row0 = s_row[k];
+                const size_t o = (size_t)(i0 + k) * BLOCK_PTS;
+                const double S0 = S0p[o], S1 = S1p[o];
+                double xv[5], u[5];
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    xv[c] = c < 2 * L + 1 ? X[(size_t)(row0 + c) * BLOCK_PTS] : 0.0;
+                    if (GGA) u[c] = c < 2 * L + 1 ? fma(a, xv[c], Y[(size_t)(row0 + c) * BLOCK_PTS]) : 0.0;
+                    else u[c] = 2.0 * a * xv[c];
+                }
+                shell_rho<true>(L, x, y, z, S0, S1, u, unused, ax, ay, az);
+                if (GGA) shell_hess(L, x, y, z, S0, S1, S2p[o], xv, cx, cy, cz, ax, ay, az);
+            }
+            warp_add3(grad, at, -4.0, ax, ay, az);
+            tx += ax, ty += ay, tz += az;
         }
     }
-    fdens[gp] = seed * f;
-
-    // AO-centre term: the block's AO list is in shell order, so each atom's AOs form runs
-    const int* aos = g.blk_aos + m.ao0;
-    double ax = 0.0, ay = 0.0, az = 0.0, tx = 0.0, ty = 0.0, tz = 0.0;
-    int cur = m.nb > 0 ? ao_atom[aos[0]] : 0;
-    for (int r = 0; r < m.nb; ++r) {
-        const int at = ao_atom[aos[r]];  // the same for every thread of the CTA
-        if (at != cur) {
-            warp_add3(grad, cur, -4.0, ax, ay, az);
-            ax = ay = az = 0.0;
-            cur = at;
-        }
-        const size_t o = (size_t)r * BLOCK_PTS + p;
-        const double x = X[o];
-        const double d1x = phi[plane + o], d1y = phi[2 * plane + o], d1z = phi[3 * plane + o];
-        double Gx = a * d1x * x, Gy = a * d1y * x, Gz = a * d1z * x;
-        if (GGA) {
-            const double cY = cx * X[plane + o] + cy * X[2 * plane + o] + cz * X[3 * plane + o];
-            const double hxx = phi[4 * plane + o], hxy = phi[5 * plane + o], hxz = phi[6 * plane + o];
-            const double hyy = phi[7 * plane + o], hyz = phi[8 * plane + o], hzz = phi[9 * plane + o];
-            Gx += (cx * hxx + cy * hxy + cz * hxz) * x + d1x * cY;
-            Gy += (cx * hxy + cy * hyy + cz * hyz) * x + d1y * cY;
-            Gz += (cx * hxz + cy * hyz + cz * hzz) * x + d1z * cY;
-        }
-        ax += Gx, ay += Gy, az += Gz;
-        tx += Gx, ty += Gy, tz += Gz;
-        if (want_z) X[o] = 0.5 * a * phi[o] + (GGA ? cx * d1x + cy * d1y + cz * d1z : 0.0);
-    }
-    if (m.nb > 0) warp_add3(grad, cur, -4.0, ax, ay, az);
     warp_add3_by_owner(grad, owner[gp], 4.0, tx, ty, tz);
-
-    // block sums in FP64 (deterministic order): Exc, electron count
-    __shared__ double red[2][BLOCK_PTS / 32];
-    const double se = warp_sum(w * f), sn = warp_sum(w * rho);
-    if ((p & 31) == 0) red[0][p >> 5] = se, red[1][p >> 5] = sn;
-    __syncthreads();
-    if (p == 0) {
-        double E = 0.0, N = 0.0;
-        for (int i = 0; i < BLOCK_PTS / 32; ++i) E += red[0][i], N += red[1][i];
-        blk_sum[2 * blk] = E;
-        blk_sum[2 * blk + 1] = N;
-    }
 }
 
 __device__ __forceinline__ void becke_poly(double nu, double& p1, double& p2, double& p3) {
@@ -258,8 +131,8 @@ __device__ __forceinline__ void becke_poly(double nu, double& p1, double& p2, do
     p3 = 0.5 * p2 * (3.0 - p2 * p2);
 }
 
-// Grid-weight term. T points per CTA (one per thread); shared memory holds each
-// point's atom distances and partition products, [natom][T] each. Pair constants
+// Grid-weight term. 32 points per CTA (a lane each), the atoms divided over its four warps; shared
+// memory holds each point's atom distances and partition products, [natom][32] each. Pair constants
 // (1/R_ij and the size adjustment a_ij) come from the table k_becke_pairs writes.
 // For B != owner A and every other atom i, one evaluation of nu_iB gives
 // s_iB = (1 - f3)/2, s_Bi = (1 + f3)/2 (nu_Bi = -nu_iB), s'(nu_iB) = s'(nu_Bi) and
@@ -268,60 +141,90 @@ __device__ __forceinline__ void becke_poly(double nu, double& p1, double& p2, do
 //   grad_B P_A = s'(nu_AB) dnu grad_B mu_AB P_A / s_AB,
 // where P_i / s_iB is the product of P_i's other factors (taken as 0 when s_iB has
 // underflowed: the term is then below 1e-250).
+// A pair of atoms whose P_i and P_B both lie below 2^-80 Z at all of the CTA's points is left out: at
+// that size s' / s is at most 2e4 (s ~ (1 - nu)^8), so its terms are below 1e-19 of the others. The
+// points of a CTA are neighbours, so most pairs of a larger molecule go.
+// Bound by the FP64 pipe. 30-atom chain, 477k points: 1.90 ms (a thread per point, every pair: 4.09).
 //
-// ROWS_IN_DRAM: the two [natom] rows of every thread live in a scratch array in
-// device memory ([2][natom][gridDim.x * T], a thread's entries strided by the
-// grid's thread count, so a warp's accesses stay coalesced) instead of shared
-// memory; the form for systems whose rows do not fit shared memory.
-template <int T, bool ROWS_IN_DRAM>
-__global__ void __launch_bounds__(T) k_grad_weight(const double* __restrict__ atom_xyz, int natom,
-                                                   const double* __restrict__ inv, const double* __restrict__ adj,
-                                                   int64_t nslots, const double* __restrict__ px,
-                                                   const double* __restrict__ py, const double* __restrict__ pz,
-                                                   const int* __restrict__ owner, const double* __restrict__ wsingle,
-                                                   const double* __restrict__ fdens, double* grad,
-                                                   double* __restrict__ scratch) {
+// ROWS_IN_DRAM: the two [natom] rows of every point live in a scratch array in device memory
+// ([2][natom][32 gridDim.x], a warp's accesses coalesced) instead of shared memory; the form for
+// systems whose rows do not fit shared memory. The live atoms (a list and a flag per atom) follow in
+// shared memory.
+constexpr int GW_T = 32, GW_W = 4;
+template <bool ROWS_IN_DRAM>
+__global__ void __launch_bounds__(GW_T* GW_W) k_grad_weight(
+    const double* __restrict__ atom_xyz, int natom, const double* __restrict__ inv, const double* __restrict__ adj,
+    int64_t nslots, const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
+    const int* __restrict__ owner, const double* __restrict__ wsingle, const double* __restrict__ fdens, double* grad,
+    double* __restrict__ scratch) {
     extern __shared__ double sm[];
-    const size_t stride = ROWS_IN_DRAM ? (size_t)gridDim.x * T : (size_t)T;
-    double* rr = ROWS_IN_DRAM ? scratch + (size_t)blockIdx.x * T : sm;  // [natom][stride]
-    double* Pm = rr + (size_t)natom * stride;                            // [natom][stride]
-    const int t = threadIdx.x;
+    __shared__ double s_z[GW_W][GW_T];
+    __shared__ int s_n;
+    constexpr unsigned kAll = 0xffffffffu;
+    const size_t stride = ROWS_IN_DRAM ? (size_t)gridDim.x * GW_T : (size_t)GW_T;
+    double* rr = ROWS_IN_DRAM ? scratch + (size_t)blockIdx.x * GW_T : sm;  // [natom][stride]
+    double* Pm = rr + (size_t)natom * stride;                               // [natom][stride]
+    int* list = reinterpret_cast<int*>(sm + (ROWS_IN_DRAM ? 0 : 2 * (size_t)natom * GW_T));  // [natom] live atoms
+    int* live_at = list + natom;                                                              // [natom] 0 or 1
+    const int t = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr double kTiny = 1e-250;
-    for (int64_t i0 = blockIdx.x * (int64_t)T; i0 < nslots; i0 += (int64_t)gridDim.x * T) {
+    for (int64_t i0 = blockIdx.x * (int64_t)GW_T; i0 < nslots; i0 += (int64_t)gridDim.x * GW_T) {
         const int64_t i = i0 + t;
         const bool live = i < nslots;
         const double c = live ? wsingle[i] * fdens[i] : 0.0;
-        if (!__syncthreads_or(c != 0.0)) continue;
+        if (!__any_sync(kAll, c != 0.0)) continue;  // the same points in every warp: uniform over the CTA
         const double rx = live ? px[i] : 0.0, ry = live ? py[i] : 0.0, rz = live ? pz[i] : 0.0;
         const int A = live ? owner[i] : 0;
-        for (int m = 0; m < natom; ++m) {
+        for (int m = warp; m < natom; m += GW_W) {
             const double ax = __ldg(atom_xyz + 3 * m) - rx, ay = __ldg(atom_xyz + 3 * m + 1) - ry,
                          az = __ldg(atom_xyz + 3 * m + 2) - rz;
             rr[m * stride + t] = sqrt(ax * ax + ay * ay + az * az);
-            Pm[m * stride + t] = 1.0;
         }
-        // partition products, each unordered pair once
-        for (int m = 0; m < natom; ++m) {
+        __syncthreads();
+        // partition products
+        double z4 = 0.0;
+        for (int m = warp; m < natom; m += GW_W) {
             const double rm = rr[m * stride + t];
-            double pmv = Pm[m * stride + t];
-            for (int n = m + 1; n < natom; ++n) {
-                double mu = (rm - rr[n * stride + t]) * __ldg(inv + (size_t)m * natom + n);
-                const double nu = mu + __ldg(adj + (size_t)m * natom + n) * (1.0 - mu * mu);
+            const double *im = inv + (size_t)m * natom, *am = adj + (size_t)m * natom;
+            double p = 1.0;
+            for (int n = 0; n < natom; ++n) {
+                if (n == m) continue;
+                const double mu = (rm - rr[n * stride + t]) * __ldg(im + n);
                 double p1, p2, p3;
-                becke_poly(nu, p1, p2, p3);
-                pmv *= 0.5 * (1.0 - p3);
-                Pm[n * stride + t] *= 0.5 * (1.0 + p3);
+                becke_poly(mu + __ldg(am + n) * (1.0 - mu * mu), p1, p2, p3);
+                p *= 0.5 * (1.0 - p3);
             }
-            Pm[m * stride + t] = pmv;
+            Pm[m * stride + t] = p;
+            z4 += p;
         }
-        double Z = 0.0;
-        for (int m = 0; m < natom; ++m) Z += Pm[m * stride + t];
+        s_z[warp][t] = z4;
+        __syncthreads();
+        const double Z = (s_z[0][t] + s_z[1][t]) + (s_z[2][t] + s_z[3][t]);
         const bool act = c != 0.0 && Z > 0.0;
         const double invZ = act ? 1.0 / Z : 0.0;
+        for (int m = warp; m < natom; m += GW_W) {  // an atom is live where any point needs its P
+            const bool need = __any_sync(kAll, act && !(Pm[m * stride + t] < 8.271806125530277e-25 * Z));
+            if (t == 0) live_at[m] = need ? 1 : 0;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            int n = 0;
+            for (int m0 = 0; m0 < natom; m0 += 32) {
+                const bool f = m0 + t < natom && live_at[m0 + t];
+                const unsigned bits = __ballot_sync(kAll, f);
+                if (f) list[n + __popc(bits & ((1u << t) - 1))] = m0 + t;
+                n += __popc(bits);
+            }
+            if (t == 0) s_n = n;
+        }
+        __syncthreads();
+        const int nlive = s_n;
         const double PA = Pm[A * stride + t];
         const double omega = PA * invZ;
         double Tx = 0.0, Ty = 0.0, Tz = 0.0;
-        for (int B = 0; B < natom; ++B) {
+        for (int B = warp; B < natom; B += GW_W) {
+            const bool all = live_at[B] != 0;  // against every atom, or against the live ones
+            const int nn = all ? natom : nlive;
             double dx = 0.0, dy = 0.0, dz = 0.0;
             if (act && B != A) {
                 const double RBx = __ldg(atom_xyz + 3 * B), RBy = __ldg(atom_xyz + 3 * B + 1),
@@ -330,8 +233,11 @@ __global__ void __launch_bounds__(T) k_grad_weight(const double* __restrict__ at
                 const double irB = 1.0 / rB;
                 const double ux = (RBx - rx) * irB, uy = (RBy - ry) * irB, uz = (RBz - rz) * irB;
                 const double PB = Pm[B * stride + t];
-                double zx = 0.0, zy = 0.0, zz = 0.0, ax = 0.0, ay = 0.0, az = 0.0;
-                for (int n = 0; n < natom; ++n) {
+                // sum over n of h (u + mu e), h = -f / R_nB, e the unit vector from n to B: the u terms
+                // in one sum, the e terms by component
+                double hs = 0.0, ex = 0.0, ey = 0.0, ez = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+                for (int j = 0; j < nn; ++j) {
+                    const int n = all ? j : list[j];
                     if (n == B) continue;
                     const double iR = __ldg(inv + (size_t)n * natom + B);
                     const double a = __ldg(adj + (size_t)n * natom + B);
@@ -342,91 +248,70 @@ __global__ void __launch_bounds__(T) k_grad_weight(const double* __restrict__ at
                     const double s_nB = 0.5 * (1.0 - p3), s_Bn = 0.5 * (1.0 + p3);
                     const double k = -(27.0 / 16.0) * (1.0 - p2 * p2) * (1.0 - p1 * p1) * (1.0 - nu * nu) *
                                      (1.0 - 2.0 * a * mu);
-                    const double ex = (RBx - __ldg(atom_xyz + 3 * n)) * iR, ey = (RBy - __ldg(atom_xyz + 3 * n + 1)) * iR,
-                                 ez = (RBz - __ldg(atom_xyz + 3 * n + 2)) * iR;
-                    const double gmx = -(ux + mu * ex) * iR, gmy = -(uy + mu * ey) * iR, gmz = -(uz + mu * ez) * iR;
-                    const double rn = s_nB > kTiny ? Pm[n * stride + t] / s_nB : 0.0;
-                    const double rb = s_Bn > kTiny ? PB / s_Bn : 0.0;
-                    const double f = k * (rn - rb);
-                    zx += f * gmx, zy += f * gmy, zz += f * gmz;
-                    if (n == A) ax = k * rn * gmx, ay = k * rn * gmy, az = k * rn * gmz;
+                    // P_n / s_nB and P_B / s_Bn with one division (s_nB + s_Bn = 1: their product
+                    // underflows only where a quotient is dropped anyway)
+                    const bool okn = s_nB > kTiny, okb = s_Bn > kTiny;
+                    const double is = 1.0 / ((okn ? s_nB : 1.0) * (okb ? s_Bn : 1.0));
+                    const double rn = okn ? Pm[n * stride + t] * (okb ? s_Bn : 1.0) * is : 0.0;
+                    const double rb = okb ? PB * (okn ? s_nB : 1.0) * is : 0.0;
+                    const double h = -k * (rn - rb) * iR, q = h * mu * iR;
+                    const double ox = RBx - __ldg(atom_xyz + 3 * n), oy = RBy - __ldg(atom_xyz + 3 * n + 1),
+                                 oz = RBz - __ldg(atom_xyz + 3 * n + 2);
+                    hs += h;
+                    ex = fma(q, ox, ex), ey = fma(q, oy, ey), ez = fma(q, oz, ez);
+                    if (n == A) {
+                        const double ha = -k * rn * iR, qa = ha * mu * iR;
+                        gx = ha * ux + qa * ox, gy = ha * uy + qa * oy, gz = ha * uz + qa * oz;
+                    }
                 }
-                dx = c * (ax - omega * zx) * invZ;
-                dy = c * (ay - omega * zy) * invZ;
-                dz = c * (az - omega * zz) * invZ;
+                dx = c * (gx - omega * (hs * ux + ex)) * invZ;
+                dy = c * (gy - omega * (hs * uy + ey)) * invZ;
+                dz = c * (gz - omega * (hs * uz + ez)) * invZ;
             }
             warp_add3(grad, B, 1.0, dx, dy, dz);
             Tx += dx, Ty += dy, Tz += dz;
         }
         warp_add3_by_owner(grad, A, -1.0, Tx, Ty, Tz);
-        __syncthreads();  // shared rows are rewritten by the next tile of points
+        __syncthreads();  // the rows and lists are rewritten by the next tile of points
     }
 }
 
 }  // namespace
 
-int grad_workspace_planes(bool gga) { return grad_phi_planes(gga) + (gga ? 4 : 1); }
-
-void launch_ao_grad(const BasisView& b, const GridView& g, int blk0, int nblk, bool gga, char* ws, cudaStream_t s) {
+void launch_grad_atoms(const BasisView& b, const GridView& g, const int* owner, int blk0, int nblk, bool gga,
+                       const double* coef, const char* ws, double* grad, cudaStream_t s) {
     if (gga)
-        k_ao_grad<true><<<nblk, 256, 0, s>>>(b, g, blk0, ws);
+        k_grad_atoms<true><<<nblk, 256, 0, s>>>(b, g, owner, blk0, coef, ws, grad);
     else
-        k_ao_grad<false><<<nblk, 256, 0, s>>>(b, g, blk0, ws);
+        k_grad_atoms<false><<<nblk, 256, 0, s>>>(b, g, owner, blk0, coef, ws, grad);
 }
 
-void launch_grad_x(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, bool gga, char* ws,
-                   cudaStream_t s) {
-    // X = P_sub phi (LDA); X, Y_x, Y_y, Y_z = P_sub (phi, d_x phi, d_y phi, d_z phi) (GGA)
-    for (int z = 0; z < (gga ? 4 : 1); ++z)
-        launch_gemm_x_plane(g, P, nao, blk0, nblk, max_nbp, z, grad_phi_planes(gga) + z, ws, s);
-}
-
-void launch_grad_point(const GridView& g, const int* ao_atom, const int* owner, int blk0, int nblk, int fn,
-                       double rho_cut, char* ws, double seed, bool want_z, double* fdens, double* blk_sum,
-                       double* grad, cudaStream_t s) {
-    if (functional_is_gga(fn))
-        k_grad_point<true><<<nblk, BLOCK_PTS, 0, s>>>(g, ao_atom, owner, blk0, fn, rho_cut, ws, seed, want_z ? 1 : 0,
-                                                      fdens, blk_sum, grad);
-    else
-        k_grad_point<false><<<nblk, BLOCK_PTS, 0, s>>>(g, ao_atom, owner, blk0, fn, rho_cut, ws, seed,
-                                                       want_z ? 1 : 0, fdens, blk_sum, grad);
-}
-
-int grad_z_plane(bool gga) { return grad_phi_planes(gga); }
-
-// Shared memory per CTA: 2 * natom * T doubles; 64 points per CTA while that fits
-// 200 KiB, else 32; beyond 400 atoms the rows live in device memory
-// (grad_weight_scratch_doubles of scratch).
-int grad_weight_max_atoms() { return (int)((200u * 1024u) / (2 * sizeof(double) * 32)); }
+// Shared memory per CTA: 520 bytes per atom (two rows of 32 doubles, a list entry and a flag); beyond
+// 400 atoms the rows live in device memory (grad_weight_scratch_doubles of scratch).
+int grad_weight_max_atoms() { return (int)((200u * 1024u) / (2 * sizeof(double) * GW_T)); }
 
 namespace {
 constexpr int kWeightDramCtas = 148 * 4;
 }
 
-size_t grad_weight_scratch_doubles(int natom) { return (size_t)2 * natom * kWeightDramCtas * 32; }
+size_t grad_weight_scratch_doubles(int natom) { return (size_t)2 * natom * kWeightDramCtas * GW_T; }
 
 void launch_grad_weight(const double* atom_xyz, int natom, const double* inv, const double* adj, int64_t nslots,
                         const double* px, const double* py, const double* pz, const int* owner, const double* wsingle,
                         const double* fdens, double* grad, double* scratch, cudaStream_t s) {
-    const size_t smem64 = 2 * sizeof(double) * 64 * (size_t)natom;
-    const size_t smem32 = 2 * sizeof(double) * 32 * (size_t)natom;
+    const size_t lists = 2 * sizeof(int) * (size_t)natom;
+    int64_t blocks = (nslots + GW_T - 1) / GW_T;
     if (scratch) {
-        int64_t blocks = (nslots + 31) / 32;
         if (blocks > kWeightDramCtas) blocks = kWeightDramCtas;
-        k_grad_weight<32, true><<<(unsigned)blocks, 32, 0, s>>>(atom_xyz, natom, inv, adj, nslots, px, py, pz, owner,
-                                                               wsingle, fdens, grad, scratch);
-    } else if (smem64 <= 200u * 1024u) {
-        int64_t blocks = (nslots + 63) / 64;
-        if (blocks > 148 * 16) blocks = 148 * 16;
-        cudaFuncSetAttribute(k_grad_weight<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64);
-        k_grad_weight<64, false><<<(unsigned)blocks, 64, smem64, s>>>(atom_xyz, natom, inv, adj, nslots, px, py, pz,
-                                                                     owner, wsingle, fdens, grad, nullptr);
+        cudaFuncSetAttribute(k_grad_weight<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lists);
+        k_grad_weight<true><<<(unsigned)blocks, GW_T * GW_W, lists, s>>>(atom_xyz, natom, inv, adj, nslots, px, py, pz,
+                                                                        owner, wsingle, fdens, grad, scratch);
     } else {
-        int64_t blocks = (nslots + 31) / 32;
-        if (blocks > 148 * 16) blocks = 148 * 16;
-        cudaFuncSetAttribute(k_grad_weight<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem32);
-        k_grad_weight<32, false><<<(unsigned)blocks, 32, smem32, s>>>(atom_xyz, natom, inv, adj, nslots, px, py, pz,
-                                                                     owner, wsingle, fdens, grad, nullptr);
+        const size_t smem = 2 * sizeof(double) * GW_T * (size_t)natom + lists;
+        if (blocks > 148 * 32) blocks = 148 * 32;
+        cudaFuncSetAttribute(k_grad_weight<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_grad_weight<false><<<(unsigned)blocks, GW_T * GW_W, smem, s>>>(atom_xyz, natom, inv, adj, nslots, px, py, pz,
+                                                                         owner, wsingle, fdens, grad, nullptr);
     }
 }
 

@@ -105,7 +105,7 @@ __device__ __forceinline__ void fp64_tile(int nb, int T, int i, int& r8, int& n8
 // ring of three shared-memory stages filled by asynchronous copies (one barrier per step), 8 warps
 // of all the tile's rows x 16 points (up to 8 x 2 DMMA tiles), so that a trimmed tile shortens every
 // warp alike. Bound by the FP64 tensor pipe. Planes are [nbp][128] arrays of the block's workspace:
-// source plane src0, destination plane dst0 (the gradient: phi and its derivatives too).
+// source plane src0, destination plane dst0 (the adjoint: phi -> X, and Z -> P_sub Z).
 // MODE (bits): X_STORE writes X. X_PHI (LDA) reduces it: the tile goes to shared memory and each thread
 // sums rho for its point and half of the tile's rows; the tile's sums go to row 4 tile of plane sum0
 // (nb >= 1 AOs give ceil(nb / 64) tiles and at least 8 rows). An LDA build needs the sums only, which
@@ -336,6 +336,8 @@ __global__ void __launch_bounds__(BLOCK_PTS) k_rho_functional(GridView g, int bl
 // S1 [nsh][128]. k_ao_eval_rad writes phi and the radial sums; everything that needs grad phi forms
 // it from them (ao.cuh). The shells (rows, angular momenta, atoms, primitives) are staged in shared
 // memory, 64 at a time.
+// RAD2: also S2 = sum_k c_k a_k^2 e^{-a_k r^2} ([nsh][128] after S1), for second derivatives.
+template <bool RAD2>
 __global__ void __launch_bounds__(256) k_ao_eval_rad(BasisView bas, GridView g, int blk0, char* ws, int rad0) {
     const int blk = blk0 + blockIdx.x;
     const BlockMeta m = g.meta[blk];
@@ -358,7 +360,13 @@ __global__ void __launch_bounds__(256) k_ao_eval_rad(BasisView bas, GridView g, 
             const double x = rx - r.ax, y = ry - r.ay, z = rz - r.az;
             const int L = r.lq, n = 2 * L + 1;
             double S0, S1;
-            shell_radial_staged<true>(bas, r, x * x + y * y + z * z, S0, S1);
+            if (RAD2) {
+                double S2;
+                shell_radial2_staged(bas, r, x * x + y * y + z * z, S0, S1, S2);
+                S1p[(size_t)(m.nsh + i) * BLOCK_PTS + p] = S2;
+            } else {
+                shell_radial_staged<true>(bas, r, x * x + y * y + z * z, S0, S1);
+            }
             S0p[(size_t)i * BLOCK_PTS + p] = S0;
             S1p[(size_t)i * BLOCK_PTS + p] = S1;
             for (int c = 0; c < n; ++c) {
@@ -697,9 +705,10 @@ void launch_gemm_x_plane(const GridView& g, const double* P, int nao, int blk0, 
     run_gemm_x<X_STORE>(g, P, nao, blk0, nblk, max_nbp, src, dst, 0, ws, s);
 }
 
-void launch_gemm_x_lda(const GridView& g, const double* P, int nao, int blk0, int nblk, int sum0, char* ws,
+void launch_gemm_x_lda(const GridView& g, const double* P, int nao, int blk0, int nblk, int xplane, int sum0, char* ws,
                        cudaStream_t s) {
-    run_gemm_x<X_PHI>(g, P, nao, blk0, nblk, 0, 0, 0, sum0, ws, s);
+    if (xplane >= 0) run_gemm_x<X_PHI | X_STORE>(g, P, nao, blk0, nblk, 0, 0, xplane, sum0, ws, s);
+    else run_gemm_x<X_PHI>(g, P, nao, blk0, nblk, 0, 0, 0, sum0, ws, s);
 }
 
 void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int xplane, int rad0, const char* ws,
@@ -710,8 +719,12 @@ void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, i
         k_rho_rad<1><<<nblk, 256, 0, s>>>(b, g, blk0, ws, xplane, rad0, acc_a, nullptr);
 }
 
-void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, char* ws, cudaStream_t s) {
-    k_ao_eval_rad<<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
+void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, bool rad2, char* ws,
+                        cudaStream_t s) {
+    if (rad2)
+        k_ao_eval_rad<true><<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
+    else
+        k_ao_eval_rad<false><<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
 }
 
 void launch_z_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const double* coef_a, const double* coef_b,

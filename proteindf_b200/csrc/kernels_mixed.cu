@@ -182,28 +182,33 @@ __device__ __forceinline__ void load_rho(const GridView& g, int blk, int p, cons
 template <bool GGA>
 __global__ void __launch_bounds__(BLOCK_PTS) k_functional_mixed(GridView g, int blk0, int fn, int incremental,
                                                                 double rho_cut, RhoSource src,
-                                                                double* rho_store, double* coef, double* blk_sum) {
+                                                                double* rho_store, double* coef, double* blk_sum,
+                                                                double seed, double* fdens) {
     const int blk = blk0 + blockIdx.x;
     const int p = threadIdx.x;
     const size_t gp = (size_t)blk * BLOCK_PTS + p;
     double ra[4];
     load_rho<GGA>(g, blk, p, src, 0, ra);
     double rho = ra[0], gx = 2.0 * ra[1], gy = 2.0 * ra[2], gz = 2.0 * ra[3];
-    double* rs = rho_store + gp * 4;
-    if (incremental) rho += rs[0], gx += rs[1], gy += rs[2], gz += rs[3];
-    rs[0] = rho, rs[1] = gx, rs[2] = gy, rs[3] = gz;
-    const double w = g.pw[gp];
-    double e = 0.0, a = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
+    if (rho_store) {
+        double* rs = rho_store + gp * 4;
+        if (incremental) rho += rs[0], gx += rs[1], gy += rs[2], gz += rs[3];
+        rs[0] = rho, rs[1] = gx, rs[2] = gy, rs[3] = gz;
+    }
+    const double w = g.pw[gp], sw = seed * w;  // seed: the cotangent of Exc (1 in a build)
+    double e = 0.0, f = 0.0, a = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
     if (w != 0.0 && rho > rho_cut) {
         const double gam = gx * gx + gy * gy + gz * gz;
         const XcOut o = eval_functional(fn, rho, rho, gam, gam, gam);
+        f = o.f;
         e = w * o.f;
-        a = 0.5 * w * o.va;
+        a = 0.5 * sw * o.va;
         if (GGA) {
-            const double cc = w * (2.0 * o.vgaa + o.vgab);
+            const double cc = sw * (2.0 * o.vgaa + o.vgab);
             cx = cc * gx, cy = cc * gy, cz = cc * gz;
         }
     }
+    if (fdens) fdens[gp] = seed * f;
     double* cf = coef + gp * 4;
     cf[0] = a, cf[1] = cx, cf[2] = cy, cf[3] = cz;
     __shared__ double red[2][BLOCK_PTS / 32];
@@ -1390,10 +1395,20 @@ void launch_functional(const GridView& g, int blk0, int nblk, int fn, bool incre
                        const RhoSource& src, double* rho_store, double* coef, double* blk_sum, cudaStream_t s) {
     if (functional_is_gga(fn))
         k_functional_mixed<true><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, src, rho_store, coef,
-                                                            blk_sum);
+                                                            blk_sum, 1.0, nullptr);
     else
         k_functional_mixed<false><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, incremental, rho_cut, src, rho_store, coef,
-                                                             blk_sum);
+                                                             blk_sum, 1.0, nullptr);
+}
+
+void launch_functional_adjoint(const GridView& g, int blk0, int nblk, int fn, double rho_cut, const RhoSource& src,
+                               double seed, double* fdens, double* coef, double* blk_sum, cudaStream_t s) {
+    if (functional_is_gga(fn))
+        k_functional_mixed<true><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, 0, rho_cut, src, nullptr, coef, blk_sum, seed,
+                                                            fdens);
+    else
+        k_functional_mixed<false><<<nblk, BLOCK_PTS, 0, s>>>(g, blk0, fn, 0, rho_cut, src, nullptr, coef, blk_sum,
+                                                             seed, fdens);
 }
 
 void launch_functional_uks(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,

@@ -269,7 +269,7 @@ void free_grid(pdfxc_ctx* c) {
     if (c->d_ws) cudaFree(c->d_ws);
     c->d_ws = nullptr;
     c->h_owner.clear();
-    dev_free(c->d_owner), dev_free(c->d_ao_atom), dev_free(c->d_grad);
+    dev_free(c->d_owner), dev_free(c->d_grad);
     dev_free(c->d_fdens), dev_free(c->d_wslot), dev_free(c->d_brad), dev_free(c->d_pair);
     dev_free(c->d_wscratch);
     dev_free(c->d_xtiles), dev_free(c->d_vtiles), dev_free(c->d_ltiles);
@@ -1397,12 +1397,12 @@ void enqueue_build(pdfxc_ctx* ctx, int fn, const double* d_PA, bool incremental)
         }
         // per block: phi, X (then Z; an LDA's rho sums), and for GGA the radial sums (block_ws_doubles_rad)
         PDFXC_CUDA(cudaEventRecord(e[0], s));
-        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, cb0, nb, 2, ws, s);
+        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, cb0, nb, 2, false, ws, s);
         else pdfxc::launch_ao_eval(bv, gv, cb0, nb, false, ws, 0, s);
         PDFXC_LAUNCHED("k_ao_eval");
         PDFXC_CUDA(cudaEventRecord(e[1], s));
         if (gga) pdfxc::launch_gemm_x_plane(gv, d_PA, nao, cb0, nb, c.max_nbp, 0, 1, ws, s);
-        else pdfxc::launch_gemm_x_lda(gv, d_PA, nao, cb0, nb, 1, ws, s);
+        else pdfxc::launch_gemm_x_lda(gv, d_PA, nao, cb0, nb, -1, 1, ws, s);
         PDFXC_LAUNCHED("k_gemm_x");
         PDFXC_CUDA(cudaEventRecord(e[2], s));
         if (gga) pdfxc::launch_rho_rad(bv, gv, cb0, nb, 1, 2, ws, ctx->d_rho_acc, nullptr, s);
@@ -1539,15 +1539,15 @@ int64_t enqueue_uks_fp64(pdfxc_ctx* ctx, int functional, bool incremental) {
     for (const Chunk& c : ctx->uplan.chunks) {
         const int b0 = std::max(c.b0, ctx->blk_lo), nb = std::min(c.b1, ctx->blk_hi) - b0;
         if (nb <= 0) continue;
-        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, b0, nb, planes, ws, s);
+        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, b0, nb, planes, false, ws, s);
         else pdfxc::launch_ao_eval(bv, gv, b0, nb, false, ws, 0, s);
         if (gga) {
             pdfxc::launch_gemm_x_plane(gv, ctx->d_P, nao, b0, nb, c.max_nbp, 0, 1, ws, s);
             pdfxc::launch_gemm_x_plane(gv, ctx->d_P_b, nao, b0, nb, c.max_nbp, 0, 2, ws, s);
             pdfxc::launch_rho_rad(bv, gv, b0, nb, 1, planes, ws, ctx->d_rho_acc, ctx->d_rho_acc_b, s);
         } else {
-            pdfxc::launch_gemm_x_lda(gv, ctx->d_P, nao, b0, nb, 1, ws, s);
-            pdfxc::launch_gemm_x_lda(gv, ctx->d_P_b, nao, b0, nb, 2, ws, s);
+            pdfxc::launch_gemm_x_lda(gv, ctx->d_P, nao, b0, nb, -1, 1, ws, s);
+            pdfxc::launch_gemm_x_lda(gv, ctx->d_P_b, nao, b0, nb, -1, 2, ws, s);
         }
         pdfxc::launch_functional_uks(
             gv, b0, nb, functional, incremental, ctx->opt.rho_cutoff,
@@ -2001,10 +2001,10 @@ pdfxc_status pdfxc_set_rho_uks(pdfxc_ctx* ctx, int gga, const double* rho) {
 namespace {
 
 // The XC nuclear gradient (pdfxc_xc_gradient) and the adjoint of Exc (pdfxc_xc_backward): per
-// chunk phi, grad phi and the second derivatives are recomputed (k_ao_grad), X = P_sub phi
-// (k_gemm_x), then the functional and the AO-centre term per point (k_grad_point); with
-// dexc_dP, the density adjoint Z replaces X and Vacc += phi Z^T (k_gemm_v), then
-// dexc_dP = Vacc + Vacc^T. Every derivative is scaled by `seed`.
+// chunk phi and the radial sums are recomputed, X = P_sub phi is stored and reduced to rho, the
+// functional gives the energy density and the coefficients scaled by `seed`, Z = 0.5 a phi + c . grad phi
+// is formed, Y = P_sub Z (GGA), and the AO-centre term follows from X, Y and the radial sums
+// (k_grad_atoms); with dexc_dP, Vacc += phi Z^T, then dexc_dP = Vacc + Vacc^T.
 pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, const double* PA,
                             const double* w_single, const double* becke_radius, int size_adjust, double seed,
                             double* grad_orbital, double* grad_weight, double* dexc_dP, double* exc) {
@@ -2028,15 +2028,10 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
         const bool gga = pdfxc::functional_is_gga(functional);
         const int nao = ctx->nao, natom = ctx->natom;
         cudaStream_t s = ctx->stream;
-        if (!ctx->d_ao_atom) {
-            std::vector<int> ao_atom(nao);
-            for (int sh = 0; sh < ctx->nshell; ++sh)
-                for (int c = 0; c < 2 * ctx->h_sh_l[sh] + 1; ++c) ao_atom[ctx->h_sh_ao0[sh] + c] = ctx->h_sh_atom[sh];
-            upload(&ctx->d_ao_atom, ao_atom, s);
-        }
         if (!ctx->d_owner) upload(&ctx->d_owner, ctx->h_owner, s);
         // gradient workspace: its own per-block offsets and chunks
-        ensure_plan(ctx, ctx->gplan, pdfxc::grad_workspace_planes(gga), 0);
+        const int planes = pdfxc::grad_planes(gga), rad0 = planes;
+        ensure_plan(ctx, ctx->gplan, planes, gga ? 3 : 2);
         const size_t nslots = (size_t)ctx->nblk * BLOCK_PTS;
         if (!ctx->d_grad) dev_alloc(&ctx->d_grad, 6 * (size_t)natom);
         if (!ctx->d_fdens) dev_alloc(&ctx->d_fdens, nslots);
@@ -2050,12 +2045,26 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
         for (const Chunk& ch : ctx->gplan.chunks) {
             const int b0 = std::max(ch.b0, ctx->blk_lo), n = std::min(ch.b1, ctx->blk_hi) - b0;
             if (n <= 0) continue;
-            pdfxc::launch_ao_grad(bv, gv, b0, n, gga, ws, s);
-            pdfxc::launch_grad_x(gv, ctx->d_P, nao, b0, n, ch.max_nbp, gga, ws, s);
-            pdfxc::launch_grad_point(gv, ctx->d_ao_atom, ctx->d_owner, b0, n, functional, ctx->opt.rho_cutoff, ws,
-                                     seed, dexc_dP != nullptr, ctx->d_fdens, ctx->d_blk_sum, ctx->d_grad, s);
-            if (dexc_dP)
-                pdfxc::launch_gemm_v_plane(gv, b0, n, ch.max_nbp, pdfxc::grad_z_plane(gga), ws, ctx->d_Vacc, nao, s);
+            pdfxc::launch_ao_eval_rad(bv, gv, b0, n, rad0, gga, ws, s);
+            if (gga) {
+                pdfxc::launch_gemm_x_plane(gv, ctx->d_P, nao, b0, n, ch.max_nbp, 0, pdfxc::GRAD_X, ws, s);
+                pdfxc::launch_rho_rad(bv, gv, b0, n, pdfxc::GRAD_X, rad0, ws, ctx->d_rho_acc, nullptr, s);
+            } else {
+                pdfxc::launch_gemm_x_lda(gv, ctx->d_P, nao, b0, n, pdfxc::GRAD_X, pdfxc::GRAD_Z, ws, s);
+            }
+            pdfxc::launch_functional_adjoint(
+                gv, b0, n, functional, ctx->opt.rho_cutoff,
+                pdfxc::RhoSource{gga ? ctx->d_rho_acc : nullptr, nullptr, ws, pdfxc::GRAD_Z}, seed, ctx->d_fdens,
+                ctx->d_coef, ctx->d_blk_sum, s);
+            if (gga) {
+                pdfxc::launch_z_rad(bv, gv, b0, n, ctx->d_coef, nullptr, pdfxc::GRAD_Z, rad0, ws, s);
+                pdfxc::launch_gemm_x_plane(gv, ctx->d_P, nao, b0, n, ch.max_nbp, pdfxc::GRAD_Z, pdfxc::GRAD_Y, ws, s);
+            }
+            pdfxc::launch_grad_atoms(bv, gv, ctx->d_owner, b0, n, gga, ctx->d_coef, ws, ctx->d_grad, s);
+            if (dexc_dP && gga)
+                pdfxc::launch_gemm_v_plane(gv, b0, n, ch.max_nbp, pdfxc::GRAD_Z, ws, ctx->d_Vacc, nao, s);
+            else if (dexc_dP)
+                pdfxc::launch_gemm_v_lda(gv, b0, n, ctx->d_coef, ws, ctx->d_Vacc, nao, s);
             PDFXC_CUDA(cudaGetLastError());
         }
         pdfxc::launch_block_sums(ctx->d_blk_sum + 2 * (size_t)ctx->blk_lo, ctx->blk_hi - ctx->blk_lo, ctx->d_scalars, s);

@@ -184,7 +184,6 @@ struct pdfxc_ctx {
     // XC nuclear gradient (pdfxc_xc_gradient); freed with the grid
     std::vector<int> h_owner;              // owner atom per point slot (empty: set_grid had no atoms)
     int* d_owner = nullptr;
-    int* d_ao_atom = nullptr;              // [n_ao]
     pdfxc::Plan gplan;                     // gradient workspace layout
     double* d_grad = nullptr;   // [2 * natom * 3]: AO-centre term, grid-weight term
     double* d_fdens = nullptr;  // [nblk * BLOCK_PTS] energy density per slot
@@ -231,11 +230,14 @@ void launch_gemm_x(const GridView& g, const double* P, int nao, int blk0, int nb
 // plane dst = P_sub * plane src
 void launch_gemm_x_plane(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src, int dst,
                          char* ws, cudaStream_t s);
-// the builds: phi and (GGA) the radial sums after rad0 planes; an LDA's X = P_sub phi
-// reduced to each tile's rho sum, in row 4 tile of plane sum0; a GGA's rho sums of one or both spins (acc_b, X in planes xplane, xplane + 1); the Z planes
+// the builds: phi and (GGA) the radial sums after rad0 planes (rad2: with S2); an LDA's X = P_sub phi
+// reduced to each tile's rho sum, in row 4 tile of plane sum0 (and stored in plane xplane, if not
+// negative); a GGA's rho sums of one or both spins (acc_b, X in planes xplane, xplane + 1); the Z planes
 // of one or both spins; the LDA's contraction
-void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, char* ws, cudaStream_t s);
-void launch_gemm_x_lda(const GridView& g, const double* P, int nao, int blk0, int nblk, int sum0, char* ws, cudaStream_t s);
+void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, bool rad2, char* ws,
+                        cudaStream_t s);
+void launch_gemm_x_lda(const GridView& g, const double* P, int nao, int blk0, int nblk, int xplane, int sum0, char* ws,
+                       cudaStream_t s);
 void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int xplane, int rad0, const char* ws,
                     double* acc_a, double* acc_b, cudaStream_t s);
 void launch_z_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const double* coef_a, const double* coef_b,
@@ -251,9 +253,12 @@ struct RhoSource {
 };
 // per point: the rho sums (+ the stored densities, incremental), the functional, the Vxc coefficients and
 // the block sums (kernels_mixed.cu); the open shell: blk_sum = (Exc, N_alpha) pairs, blk_sum_b =
-// (N_beta, 0) pairs
+// (N_beta, 0) pairs; the adjoint: coefficients scaled by seed, fdens = seed * energy density per slot
+// (0 below the density cut-off), no stored densities
 void launch_functional(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
                        const RhoSource& src, double* rho_store, double* coef, double* blk_sum, cudaStream_t s);
+void launch_functional_adjoint(const GridView& g, int blk0, int nblk, int fn, double rho_cut, const RhoSource& src,
+                               double seed, double* fdens, double* coef, double* blk_sum, cudaStream_t s);
 void launch_functional_uks(const GridView& g, int blk0, int nblk, int fn, bool incremental, double rho_cut,
                            const RhoSource& src, double* rho_store_a, double* rho_store_b, double* coef_a,
                            double* coef_b, double* blk_sum, double* blk_sum_b, cudaStream_t s);
@@ -275,17 +280,12 @@ void launch_block_sums(const double* blk_sum, int nblk, double* scalars, cudaStr
 // per grid segment: out[2 i], out[2 i + 1] = sums over blocks [seg_blk[i], seg_blk[i+1])
 void launch_segment_sums(const double* blk_sum, const int* seg_blk, int nseg, double* out, cudaStream_t s);
 
-// gradient.cu: XC nuclear gradient (FP64)
-int grad_workspace_planes(bool gga);  // [nbp][BLOCK_PTS] double planes per block
-void launch_ao_grad(const BasisView& b, const GridView& g, int blk0, int nblk, bool gga, char* ws, cudaStream_t s);
-void launch_grad_x(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, bool gga, char* ws,
-                   cudaStream_t s);
-// seed: the cotangent of Exc that scales every derivative; want_z: the density adjoint
-// Z = 0.5 a phi + c . grad phi replaces X (plane grad_z_plane) for the dExc/dP contraction
-void launch_grad_point(const GridView& g, const int* ao_atom, const int* owner, int blk0, int nblk, int fn,
-                       double rho_cut, char* ws, double seed, bool want_z, double* fdens, double* blk_sum,
-                       double* grad, cudaStream_t s);
-int grad_z_plane(bool gga);
+// gradient.cu: XC nuclear gradient (FP64). Planes: phi, X = P_sub phi, Z, Y = P_sub Z (GGA), then the
+// radial sums S0, S1 and (GGA) S2 of the block's shells.
+constexpr int GRAD_X = 1, GRAD_Z = 2, GRAD_Y = 3;
+inline int grad_planes(bool gga) { return gga ? 4 : 3; }
+void launch_grad_atoms(const BasisView& b, const GridView& g, const int* owner, int blk0, int nblk, bool gga,
+                       const double* coef, const char* ws, double* grad, cudaStream_t s);
 // the weight term keeps each point's atom rows in shared memory up to grad_weight_max_atoms()
 // atoms; above that (or when scratch is given) in grad_weight_scratch_doubles(natom) of device memory
 int grad_weight_max_atoms();
