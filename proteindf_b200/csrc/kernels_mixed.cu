@@ -607,8 +607,10 @@ __device__ __forceinline__ double warp_max_d(double v) {
 // to four blocks). Pass 1: the radial sums S0, S1 of every shell of the group's basis at the
 // thread's point (stored for the later stages) and the point's exponent of phi^T rows (the
 // max over the AOs: max_c |A_c S0| = |S0| max_c |A_c|, the rounding being monotone). Pass 2,
-// per tile of 16 AO rows: every thread forms phi of its point row by row from S0 and cuts its
-// 16 digits with the point's scale (one 16-byte store per digit plane). These are the only
+// per tile of 16 AO rows: every thread forms phi of its point shell by shell from S0 (a branch per
+// shell, not per row), cuts the digits with the point's scale into its own column of a shared-memory
+// tile, and stores its 16 rows' digits (one 16-byte store per digit plane; INT8 builds 1.2 to
+// 1.6 % faster than row by row in registers). These are the only
 // phi digits: the Vxc contraction reads them as an MN-major operand and takes the point scale
 // into Z' = 2^e_pt Z.
 constexpr int kGroupPts = 4 * BLOCK_PTS;
@@ -649,9 +651,25 @@ __device__ __forceinline__ double ang_max_abs(int L, double x, double y, double 
 }
 
 // Shared memory of k_phi_group: the group's shell table (pass 1), then its rows' geometry
-// (pass 2); a group whose table or rows do not fit reads them from global.
-constexpr size_t kPhiGroupBytes = 64 * 1024;
-constexpr int kPhiRowsCap = (int)(kPhiGroupBytes / sizeof(RowGeom));
+// (pass 2); a group whose table or rows do not fit reads them from global. After it the digit words of
+// a tile (pass 2).
+constexpr size_t kPhiTableBytes = 64 * 1024;
+constexpr size_t kPhiGroupBytes = kPhiTableBytes + 16 * kGroupPts * sizeof(uint32_t);
+constexpr int kPhiRowsCap = (int)(kPhiTableBytes / sizeof(RowGeom));
+
+// phi of every component of a shell of angular momentum L (the expressions of ang_poly1)
+__device__ __forceinline__ void shell_phi(int L, double x, double y, double z, double S0, double v[5]) {
+    if (L == 0) {
+        v[0] = S0;
+    } else if (L == 1) {
+        v[0] = x * S0, v[1] = y * S0, v[2] = z * S0;
+    } else {
+        const double s3 = 0.57735026918962576451;  // 1/sqrt(3)
+        v[0] = x * y * S0, v[1] = z * x * S0, v[2] = y * z * S0;
+        v[3] = 0.5 * (x * x - y * y) * S0;
+        v[4] = s3 * (z * z - 0.5 * (x * x + y * y)) * S0;
+    }
+}
 
 template <bool GGA>
 __global__ void __launch_bounds__(kGroupPts, 2) k_phi_group(BasisView bas, GridView g, const int* __restrict__ grp,
@@ -666,7 +684,7 @@ __global__ void __launch_bounds__(kGroupPts, 2) k_phi_group(BasisView bas, GridV
     double* rad = reinterpret_cast<double*>(base + L.rad);
     ShellRec* recs = reinterpret_cast<ShellRec*>(psm);
     RowGeom* rows = reinterpret_cast<RowGeom*>(psm);
-    const bool staged = (size_t)m.nsh * sizeof(ShellRec) <= kPhiGroupBytes;  // uniform over the CTA
+    const bool staged = (size_t)m.nsh * sizeof(ShellRec) <= kPhiTableBytes;  // uniform over the CTA
     if (staged)
         for (int i = tid; i < m.nsh; i += blockDim.x) stage_shell(bas, g.blk_shells[m.sh0 + i], 0, recs[i]);
     __syncthreads();
@@ -706,23 +724,27 @@ __global__ void __launch_bounds__(kGroupPts, 2) k_phi_group(BasisView bas, GridV
     if (!live) return;
     const RowGeom* rg = rows_staged ? rows : g.blk_row_geom + m.ao0;
     const double sc = oz_digit_scale(ept);
+    uint32_t* words = reinterpret_cast<uint32_t*>(psm + kPhiTableBytes) + tid;  // this thread's column
     oz_prefetch_rows<false>(rg, 0, m, rad, q);
     for (int mu0 = 0; mu0 < m.nbp; mu0 += 16) {
         if (mu0 + 16 < m.nb) oz_prefetch_rows<false>(rg + mu0 + 16, mu0 + 16, m, rad, q);  // the next tile's S0
-        // row by row (uniform over the CTA; the rows of one shell read the same S0 from L1), phi = A S0,
-        // cut at once: the tile's 16 values stay in registers
+        const int nr = min(16, m.nb - mu0);
+        for (int r = 0; r < nr;) {  // shell by shell (uniform over the CTA)
+            const RowGeom& gq = rg[mu0 + r];
+            const int t = gq.info & 15;
+            const int Lq = t == 0 ? 0 : (t < 4 ? 1 : 2);
+            const int u0 = t - Lq * Lq;                  // the component of row r
+            const int n = min(2 * Lq + 1 - u0, nr - r);  // the shell's rows in this tile from r
+            double v[5];
+            shell_phi(Lq, rx - gq.ax, ry - gq.ay, rz - gq.az, rad[(size_t)(gq.info >> 4) * BLOCK_PTS + q], v);
+#pragma unroll
+            for (int k = 0; k < 5; ++k)
+                if (k >= u0 && k < u0 + n) words[(r + k - u0) * kGroupPts] = oz_word(v[k], sc);
+            r += n;
+        }
         uint32_t w[16];
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            double v = 0.0;
-            if (mu0 + r < m.nb) {
-                const RowGeom gq = rg[mu0 + r];
-                double A, Ax, Ay, Az;
-                ang_poly1(gq.info & 15, rx - gq.ax, ry - gq.ay, rz - gq.az, A, Ax, Ay, Az);
-                v = A * rad[(size_t)(gq.info >> 4) * BLOCK_PTS + q];
-            }
-            w[r] = oz_word(v, sc);
-        }
+        for (int r = 0; r < 16; ++r) w[r] = r < nr ? words[r * kGroupPts] : 0u;
         oz_store16_words(base + L.phi1, kOzPlanesA, oz_off_a(q, mu0, m.nbp), w);
     }
 }
