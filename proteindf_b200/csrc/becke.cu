@@ -156,9 +156,9 @@ __global__ void __launch_bounds__(128) k_becke_near_tables(const double* __restr
 //      of all P_m; when they do not (a rounding boundary within 2^-73 of the sum) the point is summed
 //      over all atoms.
 // Bound by the issue of the FP32 filter and the FP64 pipe in step 3. Seeded chains on USER 75 x 302
-// grids, ncu (this form / one point per thread up to 48 atoms, a warp per point above): 30 atoms 0.57 /
-// 0.94 ms, 43 atoms 1.28 / 3.58, 77 atoms 5.9 / 17.4, 100 atoms 12.6 / 39.
-constexpr int kNearPts = 32, kNearThreads = 128, kNearCap = 1024;
+// grids, ncu (this form / one point per thread up to 48 atoms, a warp per point above): 30 atoms 0.56 /
+// 0.94 ms, 43 atoms 1.14 / 3.58, 100 atoms 8.7 / 39.
+constexpr int kNearPts = 32, kNearCap = 1024;
 
 // P_m at the point whose distances are r[n * kNearPts]: the factors in ascending partner order, up
 // to a product of zero. Four factors are formed ahead of the products.
@@ -199,7 +199,8 @@ __device__ __forceinline__ float becke_s32(float rm, float rn, float2 c, float& 
     return fmaf(-0.5f, nu, 0.5f);
 }
 
-__global__ void __launch_bounds__(kNearThreads) k_becke_near(const double* __restrict__ atom_xyz, int natom,
+template <int kNearW>
+__global__ void __launch_bounds__(32 * kNearW) k_becke_near(const double* __restrict__ atom_xyz, int natom,
                                                              const double2* __restrict__ pair,
                                                              const float2* __restrict__ pairf,
                                                              const int* __restrict__ near, int64_t npts,
@@ -213,8 +214,8 @@ __global__ void __launch_bounds__(kNearThreads) k_becke_near(const double* __res
     float* rf = reinterpret_cast<float*>(pe + kNearCap);           // [natom][32]: FP32 copy of rr
     uint32_t* mask = reinterpret_cast<uint32_t*>(rf + (size_t)natom * kNearPts);  // [natom]: points that keep m
     int* off = reinterpret_cast<int*>(mask + natom);               // [natom + 1]: pairs before m
-    __shared__ float s_min[4][kNearPts], s_prod[4][kNearPts];
-    __shared__ int s_arg[4][kNearPts], s_c[kNearPts], s_end;
+    __shared__ float s_min[kNearW][kNearPts], s_prod[kNearW][kNearPts];
+    __shared__ int s_arg[kNearW][kNearPts], s_c[kNearPts], s_end;
     constexpr unsigned kAll = 0xffffffffu;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int nlist = min(kNearList, natom);
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kNearThreads) k_becke_near(const double* __res
         const double rx = live ? xyz[3 * i] : 0.0, ry = live ? xyz[3 * i + 1] : 0.0, rz = live ? xyz[3 * i + 2] : 0.0;
         float best = 3e38f;
         int arg = 0;
-        for (int m = warp; m < natom; m += 4) {
+        for (int m = warp; m < natom; m += kNearW) {
             const double ax = atom_xyz[3 * m] - rx, ay = atom_xyz[3 * m + 1] - ry, az = atom_xyz[3 * m + 2] - rz;
             const double d = sqrt(ax * ax + ay * ay + az * az);
             rr[m * kNearPts + lane] = d;
@@ -236,16 +237,16 @@ __global__ void __launch_bounds__(kNearThreads) k_becke_near(const double* __res
         s_min[warp][lane] = best, s_arg[warp][lane] = arg;
         __syncthreads();
         if (warp == 0) {
-            for (int w = 1; w < 4; ++w)
+            for (int w = 1; w < kNearW; ++w)
                 if (s_min[w][lane] < best) best = s_min[w][lane], arg = s_arg[w][lane];
             s_c[lane] = arg;
         }
         __syncthreads();
         const int c = s_c[lane];
-        {  // P_c in FP32, a quarter of its factors per warp
+        {  // P_c in FP32, its factors divided over the warps
             const float rc = rf[c * kNearPts + lane];
             float p = 1.0f;
-            for (int n = warp; n < natom; n += 4) {
+            for (int n = warp; n < natom; n += kNearW) {
                 float e;
                 const float s = becke_s32(rc, rf[n * kNearPts + lane], __ldg(pairf + (size_t)c * natom + n), e);
                 p *= n == c ? 1.0f : s;
@@ -254,18 +255,35 @@ __global__ void __launch_bounds__(kNearThreads) k_becke_near(const double* __res
         }
         __syncthreads();
         // the drop threshold: 2^-80 P_c, and nothing dropped where P_c is near the end of the FP32 range
-        const float pc = s_prod[0][lane] * s_prod[1][lane] * s_prod[2][lane] * s_prod[3][lane];
+        float pc = 1.0f;
+#pragma unroll
+        for (int w = 0; w < kNearW; ++w) pc *= s_prod[w][lane];
         const float thr = pc > 1e-10f ? pc * 8.271806e-25f : 0.0f;
-        // 2. the filter
-        for (int m = warp; m < natom; m += 4) {
+        // 2. the filter: c's nearest atoms and their distances in registers, four factors at a time
+        int nn[kNearList];
+        float rn[kNearList];
+#pragma unroll
+        for (int k = 0; k < kNearList; ++k) {
+            nn[k] = __ldg(near + c * kNearList + min(k, nlist - 1));
+            rn[k] = rf[nn[k] * kNearPts + lane];
+        }
+        for (int m = warp; m < natom; m += kNearW) {
             const float rm = rf[m * kNearPts + lane];
+            const float2* pm = pairf + (size_t)m * natom;
             float p = 1.0f;
             bool drop = !live;
-            for (int k = 0; k < nlist; ++k) {
-                const int n = __ldg(near + c * kNearList + k);
-                float e;
-                const float s = becke_s32(rm, rf[n * kNearPts + lane], __ldg(pairf + (size_t)m * natom + n), e);
-                if (n != m) p *= s + e;
+#pragma unroll
+            for (int k0 = 0; k0 < kNearList; k0 += 4) {
+                float2 pc4[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) pc4[k] = __ldg(pm + nn[k0 + k]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float e;
+                    const float s = becke_s32(rm, rn[k0 + k], pc4[k], e);
+                    // (a list shorter than kNearList repeats its last atom: not a factor twice)
+                    p *= nn[k0 + k] != m && k0 + k < nlist ? s + e : 1.0f;
+                }
                 drop = drop || p < thr;
                 if (__all_sync(kAll, drop)) break;
             }
@@ -308,7 +326,7 @@ __global__ void __launch_bounds__(kNearThreads) k_becke_near(const double* __res
             }
             __syncthreads();
             const int me = s_end, e0 = off[ms], ne = off[me] - e0;
-            for (int e = t; e < ne; e += kNearThreads) {
+            for (int e = t; e < ne; e += 32 * kNearW) {
                 int a = ms, b = me;  // the atom of pair e0 + e: the last m with off[m] <= e0 + e
                 while (b - a > 1) {
                     const int mid = (a + b) / 2;
@@ -494,6 +512,11 @@ __global__ void k_transpose_n2(const double* __restrict__ a, double* __restrict_
 // Above this many atoms (32 points' distances and lists past 200 KiB of shared memory) the warp form.
 size_t becke_near_max_atoms() { return 480; }
 
+// Warps per CTA: at 100 atoms eight warps share what shared memory lets four CTAs hold (12.6 -> 8.7 ms with
+// the lists in registers); few atoms leave eight warps too little each (30 atoms:
+// 0.56 ms with four, 0.61 with eight; 43 atoms 1.14 with four).
+constexpr int kNearSmall = 48;
+
 size_t becke_near_table_bytes(int natom) {
     return (size_t)natom * natom * (sizeof(double2) + sizeof(float2)) + sizeof(int) * kNearList * (size_t)natom;
 }
@@ -512,9 +535,15 @@ void launch_becke_near(const double* atom_xyz, const double* brad, const int* gh
     int64_t blocks = (npts + kNearPts - 1) / kNearPts;
     if (blocks > 148 * 64) blocks = 148 * 64;
     if (blocks < 1) blocks = 1;
-    cudaFuncSetAttribute(k_becke_near, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_becke_near<<<(unsigned)blocks, kNearThreads, smem, s>>>(atom_xyz, natom, pair, pairf, near, npts, xyz, owner,
-                                                              w_single, w_out);
+    if (natom <= kNearSmall) {
+        cudaFuncSetAttribute(k_becke_near<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_becke_near<4><<<(unsigned)blocks, 128, smem, s>>>(atom_xyz, natom, pair, pairf, near, npts, xyz, owner,
+                                                            w_single, w_out);
+    } else {
+        cudaFuncSetAttribute(k_becke_near<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_becke_near<8><<<(unsigned)blocks, 256, smem, s>>>(atom_xyz, natom, pair, pairf, near, npts, xyz, owner,
+                                                            w_single, w_out);
+    }
 }
 
 size_t becke_warp_max_atoms() { return (200u * 1024u) / (2 * sizeof(double) * BECKE_WW); }
