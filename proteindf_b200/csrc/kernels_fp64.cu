@@ -508,14 +508,16 @@ __global__ void __launch_bounds__(256, 3) k_z_rad(BasisView bas, GridView g, int
 }
 
 // Vacc[aos[m]][aos[n]] += sum_p phi[m][p] Z[n][p]: CTA tile up to 64 x 64 AOs (fp64_tile in both
-// dimensions), K = 128 points in steps of 16 through a ring of three shared-memory stages, 4 warps as
-// 2 x 2 of up to 4 x 4 DMMA tiles. Bound by the FP64 tensor pipe. A tile of an odd number of rows of
+// dimensions), K = 128 points in steps of 16 through two shared-memory stages, 4 warps as 2 x 2 of up
+// to 4 x 4 DMMA tiles. Bound by the FP64 tensor pipe; two stages and 128 registers let four CTAs share
+// an SM, which hide one another's first loads and atomics (three CTAs of three stages: 100-atom build
+// 21.8 ms against 20.9; a persistent form with the ring running on across tiles was slower still). A tile of an odd number of rows of
 // eight gives its first warps more work, and a warp stays on its quarter of the SM, so the warps'
 // places in the tile rotate with the CTA. Rows at nb and beyond are not read.
 // LDA: Z = a phi with a = 0.5 w vrho per point, so there is no Z plane: B is phi again, scaled by a as
 // its fragments are loaded, and phi diag(a) phi^T is symmetric: only the tiles tm <= tn are computed
 // (the list ltiles), those off the diagonal counted twice (the finish adds Vacc^T).
-constexpr int GV_B = 64, GV_BK = 16, GV_S = 3, GV_AS = GV_BK + 4;
+constexpr int GV_B = 64, GV_BK = 16, GV_S = 2, GV_AS = GV_BK + 4;
 constexpr int GV_STAGE = 2 * GV_B * GV_AS;  // doubles: A [m][k], B [n][k]
 constexpr int GV_SMEM = GV_S * GV_STAGE * 8;
 
@@ -547,7 +549,7 @@ __device__ __forceinline__ void gv_step_n(int nj, const double* As, const double
 }
 
 template <bool LDA>
-__global__ void __launch_bounds__(128, 3) k_gemm_v(GridView g, int blk0, char* ws, int zplane, const double* coef,
+__global__ void __launch_bounds__(128, 4) k_gemm_v(GridView g, int blk0, char* ws, int zplane, const double* coef,
                                                 double* Vacc, int nao, int tiles, int64_t t0) {
     extern __shared__ __align__(16) double gv_sm[];
     __shared__ double s_a[LDA ? BLOCK_PTS : 1];
