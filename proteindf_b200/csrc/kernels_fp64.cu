@@ -178,10 +178,11 @@ __global__ void __launch_bounds__(256, 2) k_gemm_x(GridView g, const double* __r
         prow[q] = r < 8 * mc && m0 + r < m.nb ? P + (size_t)aos[m0 + r] * nao : nullptr;
     }
     const int nk = (m.nb + GX_BK - 1) / GX_BK;
+    int next = (t & 15) < m.nb ? aos[t & 15] : -1;  // the AO of this thread's A column, a step ahead of its use
     auto issue = [&](int kt) {
         double* st = gx_sm + (kt % GX_S) * GX_STAGE;
-        const int k = kt * GX_BK + (t & 15);
-        const int col = k < m.nb ? aos[k] : -1;
+        const int col = next, k = (kt + 1) * GX_BK + (t & 15);
+        next = k < m.nb ? aos[k] : -1;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const bool ok = col >= 0 && prow[q];
@@ -331,13 +332,13 @@ __global__ void __launch_bounds__(BLOCK_PTS) k_rho_functional(GridView g, int bl
     }
 }
 
-// GGA builds without stored AO gradients. Layout of a block (doubles): phi [nbp][128], one plane per
-// spin [nbp][128] (X, then Z), then the radial sums S0 [nsh][128] and
-// S1 [nsh][128]. k_ao_eval_rad writes phi and the radial sums; everything that needs grad phi forms
+// Builds without stored AO gradients. Layout of a block (doubles): phi [nbp][128], one plane per
+// spin [nbp][128] (X, then Z), then, for a GGA, the radial sums S0 [nsh][128] and S1 [nsh][128]. k_ao_eval_rad writes phi and the radial sums; everything that needs grad phi forms
 // it from them (ao.cuh). The shells (rows, angular momenta, atoms, primitives) are staged in shared
 // memory, 64 at a time.
-// RAD2: also S2 = sum_k c_k a_k^2 e^{-a_k r^2} ([nsh][128] after S1), for second derivatives.
-template <bool RAD2>
+// NR: the radial sums stored, 0 (an LDA: phi only), 2, or 3 with S2 = sum_k c_k a_k^2 e^{-a_k r^2}
+// ([nsh][128] after S1, for second derivatives).
+template <int NR>
 __global__ void __launch_bounds__(256) k_ao_eval_rad(BasisView bas, GridView g, int blk0, char* ws, int rad0) {
     const int blk = blk0 + blockIdx.x;
     const BlockMeta m = g.meta[blk];
@@ -359,16 +360,11 @@ __global__ void __launch_bounds__(256) k_ao_eval_rad(BasisView bas, GridView g, 
             const ShellRec& r = recs[i - i0];
             const double x = rx - r.ax, y = ry - r.ay, z = rz - r.az;
             const int L = r.lq, n = 2 * L + 1;
-            double S0, S1;
-            if (RAD2) {
-                double S2;
-                shell_radial2_staged(bas, r, x * x + y * y + z * z, S0, S1, S2);
-                S1p[(size_t)(m.nsh + i) * BLOCK_PTS + p] = S2;
-            } else {
-                shell_radial_staged<true>(bas, r, x * x + y * y + z * z, S0, S1);
-            }
-            S0p[(size_t)i * BLOCK_PTS + p] = S0;
-            S1p[(size_t)i * BLOCK_PTS + p] = S1;
+            double S0, S1 = 0.0, S2 = 0.0;
+            if (NR == 3) shell_radial2_staged(bas, r, x * x + y * y + z * z, S0, S1, S2);
+            else shell_radial_staged<NR != 0>(bas, r, x * x + y * y + z * z, S0, S1);
+            if (NR >= 2) S0p[(size_t)i * BLOCK_PTS + p] = S0, S1p[(size_t)i * BLOCK_PTS + p] = S1;
+            if (NR == 3) S1p[(size_t)(m.nsh + i) * BLOCK_PTS + p] = S2;
             for (int c = 0; c < n; ++c) {
                 double v, gx, gy, gz;
                 ao_from_radial<false>(L * L + c, x, y, z, S0, S1, v, gx, gy, gz);
@@ -721,12 +717,11 @@ void launch_rho_rad(const BasisView& b, const GridView& g, int blk0, int nblk, i
         k_rho_rad<1><<<nblk, 256, 0, s>>>(b, g, blk0, ws, xplane, rad0, acc_a, nullptr);
 }
 
-void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, bool rad2, char* ws,
+void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, int nrad, char* ws,
                         cudaStream_t s) {
-    if (rad2)
-        k_ao_eval_rad<true><<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
-    else
-        k_ao_eval_rad<false><<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
+    if (nrad == 0) k_ao_eval_rad<0><<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
+    else if (nrad == 2) k_ao_eval_rad<2><<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
+    else k_ao_eval_rad<3><<<nblk, 256, 0, s>>>(b, g, blk0, ws, rad0);
 }
 
 void launch_z_rad(const BasisView& b, const GridView& g, int blk0, int nblk, const double* coef_a, const double* coef_b,

@@ -1397,8 +1397,7 @@ void enqueue_build(pdfxc_ctx* ctx, int fn, const double* d_PA, bool incremental)
         }
         // per block: phi, X (then Z; an LDA's rho sums), and for GGA the radial sums (block_ws_doubles_rad)
         PDFXC_CUDA(cudaEventRecord(e[0], s));
-        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, cb0, nb, 2, false, ws, s);
-        else pdfxc::launch_ao_eval(bv, gv, cb0, nb, false, ws, 0, s);
+        pdfxc::launch_ao_eval_rad(bv, gv, cb0, nb, 2, gga ? 2 : 0, ws, s);
         PDFXC_LAUNCHED("k_ao_eval");
         PDFXC_CUDA(cudaEventRecord(e[1], s));
         if (gga) pdfxc::launch_gemm_x_plane(gv, d_PA, nao, cb0, nb, c.max_nbp, 0, 1, ws, s);
@@ -1539,8 +1538,7 @@ int64_t enqueue_uks_fp64(pdfxc_ctx* ctx, int functional, bool incremental) {
     for (const Chunk& c : ctx->uplan.chunks) {
         const int b0 = std::max(c.b0, ctx->blk_lo), nb = std::min(c.b1, ctx->blk_hi) - b0;
         if (nb <= 0) continue;
-        if (gga) pdfxc::launch_ao_eval_rad(bv, gv, b0, nb, planes, false, ws, s);
-        else pdfxc::launch_ao_eval(bv, gv, b0, nb, false, ws, 0, s);
+        pdfxc::launch_ao_eval_rad(bv, gv, b0, nb, planes, gga ? 2 : 0, ws, s);
         if (gga) {
             pdfxc::launch_gemm_x_plane(gv, ctx->d_P, nao, b0, nb, c.max_nbp, 0, 1, ws, s);
             pdfxc::launch_gemm_x_plane(gv, ctx->d_P_b, nao, b0, nb, c.max_nbp, 0, 2, ws, s);
@@ -1842,7 +1840,7 @@ pdfxc_status pdfxc_density(pdfxc_ctx* ctx, const double* P, int64_t npts, const 
         char* ws = static_cast<char*>(d->d_ws);
         for (const Chunk& c : d->chunks) {
             const int nb = c.b1 - c.b0;
-            pdfxc::launch_ao_eval(bv, gv, c.b0, nb, false, ws, 0, s);
+            pdfxc::launch_ao_eval_rad(bv, gv, c.b0, nb, 2, 0, ws, s);
             pdfxc::launch_gemm_x(gv, d->d_P, nao, c.b0, nb, c.max_nbp, 1, ws, s);
             pdfxc::launch_rho_functional(gv, c.b0, nb, PDFXC_SVWN, false, d->opt.rho_cutoff, ws, d->d_rho, d->d_coef,
                                          d->d_blk_sum, s);
@@ -2045,7 +2043,7 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
         for (const Chunk& ch : ctx->gplan.chunks) {
             const int b0 = std::max(ch.b0, ctx->blk_lo), n = std::min(ch.b1, ctx->blk_hi) - b0;
             if (n <= 0) continue;
-            pdfxc::launch_ao_eval_rad(bv, gv, b0, n, rad0, gga, ws, s);
+            pdfxc::launch_ao_eval_rad(bv, gv, b0, n, rad0, gga ? 3 : 2, ws, s);
             if (gga) {
                 pdfxc::launch_gemm_x_plane(gv, ctx->d_P, nao, b0, n, ch.max_nbp, 0, pdfxc::GRAD_X, ws, s);
                 pdfxc::launch_rho_rad(bv, gv, b0, n, pdfxc::GRAD_X, rad0, ws, ctx->d_rho_acc, nullptr, s);

@@ -230,11 +230,11 @@ void launch_gemm_x(const GridView& g, const double* P, int nao, int blk0, int nb
 // plane dst = P_sub * plane src
 void launch_gemm_x_plane(const GridView& g, const double* P, int nao, int blk0, int nblk, int max_nbp, int src, int dst,
                          char* ws, cudaStream_t s);
-// the builds: phi and (GGA) the radial sums after rad0 planes (rad2: with S2); an LDA's X = P_sub phi
+// the builds: phi and nrad (0, 2 or 3) radial sums after rad0 planes; an LDA's X = P_sub phi
 // reduced to each tile's rho sum, in row 4 tile of plane sum0 (and stored in plane xplane, if not
 // negative); a GGA's rho sums of one or both spins (acc_b, X in planes xplane, xplane + 1); the Z planes
 // of one or both spins; the LDA's contraction
-void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, bool rad2, char* ws,
+void launch_ao_eval_rad(const BasisView& b, const GridView& g, int blk0, int nblk, int rad0, int nrad, char* ws,
                         cudaStream_t s);
 void launch_gemm_x_lda(const GridView& g, const double* P, int nao, int blk0, int nblk, int xplane, int sum0, char* ws,
                        cudaStream_t s);
