@@ -929,7 +929,7 @@ void build_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* ato
         for (const Chunk& c : ctx->chunks) {
             std::vector<std::pair<int, int2>> it;
             for (int b = c.b0; b < c.b1; ++b)  // rho: (block, 64-AO output tile); cost ~ K = nbp
-                for (int nt = 0; nt < ctx->h_meta[b].nbp / 64; ++nt) it.push_back({ctx->h_meta[b].nbp, make_int2(b, nt)});
+                for (int nt = 0; nt < ctx->h_meta[b].nbp / 64; ++nt) it.push_back({ctx->h_meta[b].nbp, make_int2(b, (b - ctx->h_meta[b].lead) << 16 | nt)});
             std::stable_sort(it.begin(), it.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
             ctx->items_off_rho.push_back((int)items.size());
             ctx->items_n_rho.push_back((int)it.size());
@@ -939,7 +939,7 @@ void build_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* ato
                 const BlockMeta& m = ctx->h_meta[b];
                 if (m.lead != b) continue;
                 for (int mt = 0; mt < (m.nbp + 127) / 128; ++mt)
-                    for (int nt = 0; nt < m.nbp / 64; ++nt) it.push_back({m.gn, make_int2(b, (mt << 16) | nt)});
+                    for (int nt = 0; nt < m.nbp / 64; ++nt) it.push_back({m.gn, make_int2(b, (int)((unsigned)(m.gn - 1) << 28 | mt << 16 | nt))});
             }
             std::stable_sort(it.begin(), it.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
             ctx->items_off_vxc.push_back((int)items.size());
