@@ -439,8 +439,9 @@ __global__ void __launch_bounds__(128) k_ss(const double* __restrict__ atom_xyz,
 
 void launch_ss(const double* atom_xyz, int natom, double* inv, double* adj, const int* nbr_idx,
                const double* nbr_dist, int64_t npts, const double* xyz, const int* owner, const double* w_single,
-               double* w_out, cudaStream_t s) {
-    k_becke_pairs<<<(natom * natom + 255) / 256, 256, 0, s>>>(atom_xyz, atom_xyz, nullptr, natom, 0, inv, adj);
+               double* w_out, bool tables, cudaStream_t s) {
+    if (tables)
+        k_becke_pairs<<<(natom * natom + 255) / 256, 256, 0, s>>>(atom_xyz, atom_xyz, nullptr, natom, 0, inv, adj);
     const int threads = 128;
     int64_t blocks = (npts + threads - 1) / threads;
     if (blocks > 148 * 64) blocks = 148 * 64;
@@ -523,13 +524,14 @@ size_t becke_near_table_bytes(int natom) {
 
 void launch_becke_near(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
                        void* tab, int64_t npts, const double* xyz, const int* owner, const double* w_single,
-                       double* w_out, cudaStream_t s) {
+                       double* w_out, bool tables, cudaStream_t s) {
     const size_t n2 = (size_t)natom * natom;
     double2* pair = static_cast<double2*>(tab);
     float2* pairf = reinterpret_cast<float2*>(pair + n2);
     int* near = reinterpret_cast<int*>(pairf + n2);
-    k_becke_near_tables<<<natom, 128, sizeof(double) * natom, s>>>(atom_xyz, brad, ghost, natom, size_adjust, pair,
-                                                                    pairf, near);
+    if (tables)
+        k_becke_near_tables<<<natom, 128, sizeof(double) * natom, s>>>(atom_xyz, brad, ghost, natom, size_adjust, pair,
+                                                                       pairf, near);
     const size_t smem = (size_t)natom * kNearPts * (sizeof(double) + sizeof(float)) + sizeof(double) * kNearCap +
                         sizeof(int) * (2 * (size_t)natom + 1);
     int64_t blocks = (npts + kNearPts - 1) / kNearPts;
@@ -551,13 +553,15 @@ size_t becke_warp_max_atoms() { return (200u * 1024u) / (2 * sizeof(double) * BE
 // tab: 4 n_atom^2 doubles (the pair table, then its transpose)
 void launch_becke_warp(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
                        double* tab, int64_t npts, const double* xyz, const int* owner, const double* w_single,
-                       double* w_out, cudaStream_t s) {
+                       double* w_out, bool tables, cudaStream_t s) {
     const size_t n2 = (size_t)natom * natom;
     double *inv = tab, *adj = tab + n2, *invT = tab + 2 * n2, *adjT = tab + 3 * n2;
-    k_becke_pairs<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(atom_xyz, brad, ghost, natom, size_adjust, inv, adj);
-    const unsigned tb = (unsigned)std::min<size_t>((n2 + 255) / 256, 148 * 8);
-    k_transpose_n2<<<tb, 256, 0, s>>>(inv, invT, natom);
-    k_transpose_n2<<<tb, 256, 0, s>>>(adj, adjT, natom);
+    if (tables) {
+        k_becke_pairs<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(atom_xyz, brad, ghost, natom, size_adjust, inv, adj);
+        const unsigned tb = (unsigned)std::min<size_t>((n2 + 255) / 256, 148 * 8);
+        k_transpose_n2<<<tb, 256, 0, s>>>(inv, invT, natom);
+        k_transpose_n2<<<tb, 256, 0, s>>>(adj, adjT, natom);
+    }
     int64_t blocks = (npts + BECKE_WW - 1) / BECKE_WW;
     if (blocks > 148 * 64) blocks = 148 * 64;
     if (blocks < 1) blocks = 1;

@@ -999,61 +999,57 @@ pdfxc_status pdfxc_set_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, co
 
 namespace {
 
-// Partition weights on the device: Becke (ss = false) or Stratmann-Scuseria (ss = true).
-// Partition weights of device-resident points: d_wo = d_ws * P_owner / sum_m P_m (Becke or
-// Stratmann-Scuseria), enqueued on the context's stream; d_br (natom Becke radii) only for Becke.
+// Partition weights of device-resident points: d_wo = d_ws * P_owner / sum_m P_m (Becke, or
+// Stratmann-Scuseria with ss), enqueued on the context's stream; d_br (natom Becke radii) only for Becke.
+// d_tab: the pair tables, allocated and filled by the call with `first` (of several parts of the
+// points), freed by the caller once the stream has drained.
 void partition_weights_device(pdfxc_ctx* ctx, bool ss, int64_t npts, const double* d_xyz, const int* d_own,
-                              const double* d_ws, const double* d_br, int size_adjust, double* d_wo) {
+                              const double* d_ws, const double* d_br, int size_adjust, double* d_wo, double*& d_tab,
+                              bool first) {
     cudaStream_t s = ctx->stream;
-    double* d_pair = nullptr;
-    try {
-        if (ss) {
-            const int na = ctx->natom, nn = na - 1;
-            if (!ctx->d_nbr_idx && nn > 0) {  // once per system: neighbour lists by distance
-                std::vector<int> idx((size_t)na * nn);
-                std::vector<double> dst((size_t)na * nn);
-                std::vector<std::pair<double, int>> row(nn);
-                for (int m = 0; m < na; ++m) {
-                    const double* A = &ctx->h_atom_xyz[3 * m];
-                    int k = 0;
-                    for (int n = 0; n < na; ++n) {
-                        if (n == m) continue;
-                        const double* B = &ctx->h_atom_xyz[3 * n];
-                        row[k++] = {std::sqrt((A[0] - B[0]) * (A[0] - B[0]) + (A[1] - B[1]) * (A[1] - B[1]) +
-                                              (A[2] - B[2]) * (A[2] - B[2])),
-                                    n};
-                    }
-                    std::sort(row.begin(), row.end());
-                    for (int j = 0; j < nn; ++j) idx[(size_t)m * nn + j] = row[j].second, dst[(size_t)m * nn + j] = row[j].first;
+    const size_t natom = ctx->natom;
+    if (ss) {
+        const int na = ctx->natom, nn = na - 1;
+        if (!ctx->d_nbr_idx && nn > 0) {  // once per system: neighbour lists by distance
+            std::vector<int> idx((size_t)na * nn);
+            std::vector<double> dst((size_t)na * nn);
+            std::vector<std::pair<double, int>> row(nn);
+            for (int m = 0; m < na; ++m) {
+                const double* A = &ctx->h_atom_xyz[3 * m];
+                int k = 0;
+                for (int n = 0; n < na; ++n) {
+                    if (n == m) continue;
+                    const double* B = &ctx->h_atom_xyz[3 * n];
+                    row[k++] = {std::sqrt((A[0] - B[0]) * (A[0] - B[0]) + (A[1] - B[1]) * (A[1] - B[1]) +
+                                          (A[2] - B[2]) * (A[2] - B[2])),
+                                n};
                 }
-                upload(&ctx->d_nbr_idx, idx, s);
-                upload(&ctx->d_nbr_dist, dst, s);
+                std::sort(row.begin(), row.end());
+                for (int j = 0; j < nn; ++j) idx[(size_t)m * nn + j] = row[j].second, dst[(size_t)m * nn + j] = row[j].first;
             }
-            dev_alloc(&d_pair, 2 * (size_t)ctx->natom * ctx->natom);
-            pdfxc::launch_ss(ctx->d_atom_xyz, ctx->natom, d_pair, d_pair + (size_t)ctx->natom * ctx->natom,
-                             ctx->d_nbr_idx, ctx->d_nbr_dist, npts, d_xyz, d_own, d_ws, d_wo, s);
-        } else if ((size_t)ctx->natom <= pdfxc::becke_near_max_atoms()) {
-            dev_alloc(&d_pair, (pdfxc::becke_near_table_bytes(ctx->natom) + sizeof(double) - 1) / sizeof(double));
-            pdfxc::launch_becke_near(ctx->d_atom_xyz, d_br, ctx->d_ghost, ctx->natom, size_adjust, d_pair, npts, d_xyz,
-                                     d_own, d_ws, d_wo, s);
-        } else if ((size_t)ctx->natom <= pdfxc::becke_warp_max_atoms()) {
-            dev_alloc(&d_pair, 4 * (size_t)ctx->natom * ctx->natom);
-            pdfxc::launch_becke_warp(ctx->d_atom_xyz, d_br, ctx->d_ghost, ctx->natom, size_adjust, d_pair, npts, d_xyz,
-                                     d_own, d_ws, d_wo, s);
-        } else if ((size_t)ctx->natom <= pdfxc::becke_max_atoms()) {
-            pdfxc::launch_becke(ctx->d_atom_xyz, d_br, ctx->d_ghost, ctx->natom, size_adjust, npts, d_xyz, d_own,
-                                d_ws, d_wo, s);
-        } else {
-            throw std::runtime_error("Becke partition: at most " + std::to_string(pdfxc::becke_max_atoms()) +
-                                     " atoms (use the Stratmann-Scuseria partition)");
+            upload(&ctx->d_nbr_idx, idx, s);
+            upload(&ctx->d_nbr_dist, dst, s);
+            PDFXC_CUDA(cudaStreamSynchronize(s));  // idx and dst leave scope
         }
-        PDFXC_CUDA(cudaGetLastError());
-        PDFXC_CUDA(cudaStreamSynchronize(s));
-    } catch (...) {
-        dev_free(d_pair);
-        throw;
+        if (first) dev_alloc(&d_tab, 2 * natom * natom);
+        pdfxc::launch_ss(ctx->d_atom_xyz, ctx->natom, d_tab, d_tab + natom * natom, ctx->d_nbr_idx, ctx->d_nbr_dist,
+                         npts, d_xyz, d_own, d_ws, d_wo, first, s);
+    } else if (natom <= pdfxc::becke_near_max_atoms()) {
+        if (first) dev_alloc(&d_tab, (pdfxc::becke_near_table_bytes(ctx->natom) + sizeof(double) - 1) / sizeof(double));
+        pdfxc::launch_becke_near(ctx->d_atom_xyz, d_br, ctx->d_ghost, ctx->natom, size_adjust, d_tab, npts, d_xyz, d_own,
+                                 d_ws, d_wo, first, s);
+    } else if (natom <= pdfxc::becke_warp_max_atoms()) {
+        if (first) dev_alloc(&d_tab, 4 * natom * natom);
+        pdfxc::launch_becke_warp(ctx->d_atom_xyz, d_br, ctx->d_ghost, ctx->natom, size_adjust, d_tab, npts, d_xyz, d_own,
+                                 d_ws, d_wo, first, s);
+    } else if (natom <= pdfxc::becke_max_atoms()) {
+        pdfxc::launch_becke(ctx->d_atom_xyz, d_br, ctx->d_ghost, ctx->natom, size_adjust, npts, d_xyz, d_own, d_ws,
+                            d_wo, s);
+    } else {
+        throw std::runtime_error("Becke partition: at most " + std::to_string(pdfxc::becke_max_atoms()) +
+                                 " atoms (use the Stratmann-Scuseria partition)");
     }
-    dev_free(d_pair);
+    PDFXC_CUDA(cudaGetLastError());
 }
 
 pdfxc_status partition_weights(pdfxc_ctx* ctx, bool ss, int64_t npts, const double* xyz, const int* atom,
@@ -1078,27 +1074,58 @@ pdfxc_status partition_weights(pdfxc_ctx* ctx, bool ss, int64_t npts, const doub
                 return PDFXC_ERR_ARG;
             }
         cudaStream_t s = ctx->stream;
-        double *d_xyz = nullptr, *d_ws = nullptr, *d_wo = nullptr, *d_br = nullptr;
+        // The points in up to eight parts of at least 64 Ki: a part's copies to the device (from pageable
+        // memory, on a stream of their own) run under the kernel of the part before it, and its weights
+        // come back under the kernels of the parts after it. (100 atoms, 1.5 M points: call 20.0 -> 13.7 ms.)
+        const int64_t part = std::max<int64_t>((npts + 7) / 8, 1 << 16);
+        const int np = (int)((npts + part - 1) / part);
+        if (np > 1 && !ctx->copy_stream)
+            PDFXC_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+        cudaStream_t cs = np > 1 ? ctx->copy_stream : s;
+        double *d_xyz = nullptr, *d_ws = nullptr, *d_wo = nullptr, *d_br = nullptr, *d_tab = nullptr;
         int* d_own = nullptr;
+        std::vector<cudaEvent_t> ev(np > 1 ? 2 * (size_t)np : 0, nullptr);  // per part: inputs there, weights there
+        auto release = [&]() {
+            cudaStreamSynchronize(cs), cudaStreamSynchronize(s);  // nothing in flight uses the buffers
+            for (cudaEvent_t e : ev)
+                if (e) cudaEventDestroy(e);
+            dev_free(d_xyz), dev_free(d_ws), dev_free(d_wo), dev_free(d_br), dev_free(d_own), dev_free(d_tab);
+        };
+        auto hand_over = [&](cudaEvent_t e, cudaStream_t from, cudaStream_t to) {  // `to` waits for `from`
+            if (from == to) return;
+            PDFXC_CUDA(cudaEventRecord(e, from));
+            PDFXC_CUDA(cudaStreamWaitEvent(to, e, 0));
+        };
         try {
+            for (cudaEvent_t& e : ev) PDFXC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             dev_alloc(&d_xyz, 3 * (size_t)npts);
             dev_alloc(&d_ws, (size_t)npts);
             dev_alloc(&d_wo, (size_t)npts);
             dev_alloc(&d_br, (size_t)ctx->natom);
             dev_alloc(&d_own, (size_t)npts);
-            PDFXC_CUDA(cudaMemcpyAsync(d_xyz, xyz, 3 * sizeof(double) * npts, cudaMemcpyHostToDevice, s));
-            PDFXC_CUDA(cudaMemcpyAsync(d_ws, w_single, sizeof(double) * npts, cudaMemcpyHostToDevice, s));
             if (!ss)
                 PDFXC_CUDA(cudaMemcpyAsync(d_br, becke_radius, sizeof(double) * ctx->natom, cudaMemcpyHostToDevice, s));
-            PDFXC_CUDA(cudaMemcpyAsync(d_own, atom, sizeof(int) * npts, cudaMemcpyHostToDevice, s));
-            partition_weights_device(ctx, ss, npts, d_xyz, d_own, d_ws, d_br, size_adjust, d_wo);
-            PDFXC_CUDA(cudaMemcpyAsync(w_out, d_wo, sizeof(double) * npts, cudaMemcpyDeviceToHost, s));
-            PDFXC_CUDA(cudaStreamSynchronize(s));
+            for (int k = 0; k < np; ++k) {
+                const int64_t i0 = k * part, n = std::min(part, npts - i0);
+                PDFXC_CUDA(cudaMemcpyAsync(d_xyz + 3 * i0, xyz + 3 * i0, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, cs));
+                PDFXC_CUDA(cudaMemcpyAsync(d_ws + i0, w_single + i0, sizeof(double) * n, cudaMemcpyHostToDevice, cs));
+                PDFXC_CUDA(cudaMemcpyAsync(d_own + i0, atom + i0, sizeof(int) * n, cudaMemcpyHostToDevice, cs));
+                hand_over(np > 1 ? ev[2 * k] : nullptr, cs, s);
+                partition_weights_device(ctx, ss, n, d_xyz + 3 * i0, d_own + i0, d_ws + i0, d_br, size_adjust, d_wo + i0,
+                                         d_tab, k == 0);
+                if (np > 1) PDFXC_CUDA(cudaEventRecord(ev[2 * k + 1], s));
+            }
+            for (int k = 0; k < np; ++k) {
+                const int64_t i0 = k * part, n = std::min(part, npts - i0);
+                if (np > 1) PDFXC_CUDA(cudaStreamWaitEvent(cs, ev[2 * k + 1], 0));
+                PDFXC_CUDA(cudaMemcpyAsync(w_out + i0, d_wo + i0, sizeof(double) * n, cudaMemcpyDeviceToHost, cs));
+            }
+            PDFXC_CUDA(cudaStreamSynchronize(cs));
         } catch (...) {
-            dev_free(d_xyz), dev_free(d_ws), dev_free(d_wo), dev_free(d_br), dev_free(d_own);
+            release();
             throw;
         }
-        dev_free(d_xyz), dev_free(d_ws), dev_free(d_wo), dev_free(d_br), dev_free(d_own);
+        release();
         return PDFXC_OK;
     });
 }
@@ -1242,6 +1269,7 @@ pdfxc_status pdfxc_generate_grid(pdfxc_ctx* ctx, const pdfxc_grid_params* prm, i
         std::vector<double> O(prm->orientation ? prm->orientation : ident, (prm->orientation ? prm->orientation : ident) + 9);
         pdfxc::GridShell* d_sh = nullptr;
         double *d_unit = nullptr, *d_O = nullptr, *d_xyz = nullptr, *d_ws = nullptr, *d_wo = nullptr, *d_br = nullptr;
+        double* d_tab = nullptr;
         int* d_own = nullptr;
         std::vector<double> xyz(3 * (size_t)np), w((size_t)np);
         std::vector<int> own((size_t)np);
@@ -1258,18 +1286,18 @@ pdfxc_status pdfxc_generate_grid(pdfxc_ctx* ctx, const pdfxc_grid_params* prm, i
             if (prm->partition == PDFXC_PARTITION_BECKE)
                 upload(&d_br, std::vector<double>(prm->becke_radius, prm->becke_radius + natom), s);
             partition_weights_device(ctx, prm->partition == PDFXC_PARTITION_SS, np, d_xyz, d_own, d_ws, d_br,
-                                     prm->size_adjust, d_wo);
+                                     prm->size_adjust, d_wo, d_tab, true);
             PDFXC_CUDA(cudaMemcpyAsync(xyz.data(), d_xyz, sizeof(double) * xyz.size(), cudaMemcpyDeviceToHost, s));
             PDFXC_CUDA(cudaMemcpyAsync(w.data(), d_wo, sizeof(double) * w.size(), cudaMemcpyDeviceToHost, s));
             PDFXC_CUDA(cudaMemcpyAsync(own.data(), d_own, sizeof(int) * own.size(), cudaMemcpyDeviceToHost, s));
             PDFXC_CUDA(cudaStreamSynchronize(s));
         } catch (...) {
             dev_free(d_sh), dev_free(d_unit), dev_free(d_O), dev_free(d_xyz), dev_free(d_ws), dev_free(d_wo);
-            dev_free(d_br), dev_free(d_own);
+            dev_free(d_br), dev_free(d_own), dev_free(d_tab);
             throw;
         }
         dev_free(d_sh), dev_free(d_unit), dev_free(d_O), dev_free(d_xyz), dev_free(d_ws), dev_free(d_wo);
-        dev_free(d_br), dev_free(d_own);
+        dev_free(d_br), dev_free(d_own), dev_free(d_tab);
         // the weight screen, in point order
         std::vector<double> xyzw;
         std::vector<int> atom;
@@ -2513,6 +2541,7 @@ void pdfxc_destroy(pdfxc_ctx* ctx) {
         if (e) cudaEventDestroy(e);
     for (auto& e : ctx->stage_ev) cudaEventDestroy(e);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }

@@ -104,6 +104,7 @@ struct Plan {
 struct pdfxc_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t copy_stream = nullptr;  // copies beside the kernels (partition weights), made on first use
     pdfxc_options opt{};
     std::string err;
 
@@ -295,11 +296,12 @@ void launch_grad_weight(const double* atom_xyz, int natom, const double* inv, co
                         const double* fdens, double* grad, double* scratch, cudaStream_t s);
 
 // becke.cu
-// Stratmann-Scuseria weights (n_atom <= 6000: atoms in shared memory); inv/adj: n_atom^2 scratch each
+// Partition weights; `tables`: fill the pair tables first (else they are there from a call before).
+// Stratmann-Scuseria weights (n_atom <= 6000); inv/adj: n_atom^2 scratch each
 // nbr_idx / nbr_dist: per atom the other atoms in ascending distance, natom x (natom - 1)
 void launch_ss(const double* atom_xyz, int natom, double* inv, double* adj, const int* nbr_idx,
                const double* nbr_dist, int64_t npts, const double* xyz, const int* owner, const double* w_single,
-               double* w_out, cudaStream_t s);
+               double* w_out, bool tables, cudaStream_t s);
 void launch_becke_pairs(const double* atom_xyz, const double* brad, int natom, int size_adjust, double* inv,
                         double* adj, cudaStream_t s);
 // ghost (n_atom ints, may be null): partner atoms left out of every product (atomic number <= 0)
@@ -311,13 +313,13 @@ size_t becke_max_atoms();
 // tab: becke_near_table_bytes(n_atom) of device memory
 void launch_becke_near(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
                        void* tab, int64_t npts, const double* xyz, const int* owner, const double* w_single,
-                       double* w_out, cudaStream_t s);
+                       double* w_out, bool tables, cudaStream_t s);
 size_t becke_near_max_atoms();
 size_t becke_near_table_bytes(int natom);
 // the same weights with a warp per point (lanes over the atoms); tab: 4 n_atom^2 doubles
 void launch_becke_warp(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
                        double* tab, int64_t npts, const double* xyz, const int* owner, const double* w_single,
-                       double* w_out, cudaStream_t s);
+                       double* w_out, bool tables, cudaStream_t s);
 size_t becke_warp_max_atoms();
 
 // Intermediates of one block inside its chunk workspace (doubles):
