@@ -105,21 +105,17 @@ pdfxc_status guarded(pdfxc_ctx* ctx, F&& f) {
     }
 }
 
-// Distances beyond which a shell's value and gradient bounds both stay below `cutoff` (first) and
-// below share * cutoff (second), share <= 1:
-// bound(r) = sum_k |c_k| e^{-a_k r^2} max(r^L, L r^(L-1) + 2 a_k r^(L+1)).
-std::pair<double, double> shell_cutoff_radius(int L, const double* e, const double* c, int np, double cutoff,
-                                              double share) {
-    double outer = 0.0;
+// Distance beyond which a shell's value and gradient bounds both stay below
+// `cutoff`: bound(r) = sum_k |c_k| e^{-a_k r^2} max(r^L, L r^(L-1) + 2 a_k r^(L+1)).
+double shell_cutoff_radius(int L, const double* e, const double* c, int np, double cutoff) {
     for (double r = 60.0; r > 0.0; r -= 0.01) {
         const double rl = std::pow(r, L), dl = L > 0 ? L * std::pow(r, L - 1) : 0.0;
         double b = 0.0;
         for (int k = 0; k < np; ++k)
             b += std::fabs(c[k]) * std::exp(-e[k] * r * r) * std::max(rl, dl + 2.0 * e[k] * rl * r);
-        if (outer == 0.0 && b >= share * cutoff) outer = r + 0.01;
-        if (b >= cutoff) return {r + 0.01, outer};
+        if (b >= cutoff) return r + 0.01;
     }
-    return {0.0, outer};
+    return 0.0;
 }
 
 uint64_t spread3(uint64_t v) {
@@ -489,8 +485,8 @@ void resolve_shapes(pdfxc_ctx* ctx, int64_t npts, size_t nseg) {
 // Spatial blocks and basis screening, once per geometry: within each segment the points
 // are put in Morton order over the segment's bounding box and cut into groups of up to
 // group_blocks x block_points consecutive points, each group into blocks of block_points;
-// every group keeps the shells of its segment whose value/gradient envelope reaches
-// ao_cutoff at the nearest point of its bounding sphere and 0.3 of it at its own nearest point.
+// every group keeps the shells of its segment whose value/gradient envelope reaches 0.2 of
+// ao_cutoff at the group's nearest point.
 // The host side of a blocked grid (plan_grid), before it is uploaded.
 struct HostGrid {
     std::vector<double> px, py, pz, pw;
@@ -623,15 +619,16 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
     });
     // 2. per-shell screening radius, then the per-block shell lists
     // (once per distinct shell: the shells of one element's basis repeat on every such atom)
-    // Rs: where the envelope falls below ao_cutoff, tested against the group's bounding sphere; Rn: where
-    // it falls below kNearShare of it, tested against the group's nearest point. (The sphere test alone
-    // keeps shells that no point reaches. Without the share the results at a loose cut-off would lie
-    // further from the unscreened ones than with the sphere test alone; 90-atom B3LYP chain, cut-off
-    // 1e-10, relative error of Vxc: sphere 3.4e-12; nearest point at 1.0, 0.5, 0.3 of the cut-off
-    // 9.3e-12, 4.5e-12, 2.6e-12.)
-    constexpr double kNearShare = 0.3;
-    std::vector<double> Rs(ctx->nshell), Rn(ctx->nshell);
-    std::map<std::vector<double>, std::pair<double, double>> radius_of;
+    // Rs: where the envelope falls below kNearShare of ao_cutoff, tested against the group's nearest
+    // point. (The group's bounding sphere as the nearest point keeps shells that no point reaches, and at
+    // a loose cut-off the many shells just below it at its surface make most of the error. Relative error
+    // of Vxc against the unscreened sum and mean nb^2, B3LYP chain of 150 atoms, cut-off 1e-10, groups of
+    // 128 points: sphere at the cut-off 5.1e-12, 54,900; nearest point at 1, 0.3, 0.2 and 0.1 of it
+    // 13.2e-12, 43,200; 3.8e-12, 47,300; 2.4e-12, 48,600; 1.2e-12, 51,000. With groups of 512 points a
+    // share of 0.3 can be less exact than the sphere (1.38e-12 against 1.24e-12 at 90 atoms), 0.2 was not.)
+    constexpr double kNearShare = 0.2;
+    std::vector<double> Rs(ctx->nshell);
+    std::map<std::vector<double>, double> radius_of;
     for (int sh = 0; sh < ctx->nshell; ++sh) {
         const int p0 = ctx->h_sh_p0[sh], np = ctx->h_sh_nprim[sh];
         std::vector<double> k = {(double)ctx->h_sh_l[sh]};
@@ -640,8 +637,8 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
         auto it = radius_of.find(k);
         if (it == radius_of.end())
             it = radius_of.emplace(k, shell_cutoff_radius(ctx->h_sh_l[sh], &ctx->h_p_exp[p0], &ctx->h_p_coef[p0], np,
-                                                          ctx->opt.ao_cutoff, kNearShare)).first;
-        Rs[sh] = it->second.first, Rn[sh] = it->second.second;
+                                                          kNearShare * ctx->opt.ao_cutoff)).first;
+        Rs[sh] = it->second;
     }
     std::vector<int>&shells = G.shells, &rows = G.rows, &aos = G.aos, &row_info = G.row_info;
     shells.clear(), rows.clear(), aos.clear(), row_info.clear();
@@ -740,9 +737,9 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
             const int sh0 = (int)P.shells.size(), ao0 = (int)P.aos.size();
             int row = 0;
             candidates(si, (int)gi, cand_sh, ats);
-            // A shell must pass both tests (Rs, Rn above). The sphere settles the shells that every point
-            // reaches and the bounding box most of those that none reaches; for the rest the points are
-            // looked through, as far as the first one inside, once per atom.
+            // The sphere settles the shells that every point reaches or none does, the bounding box most of
+            // the others that none reaches; for the rest the points are looked through, as far as the first
+            // one inside, once per atom.
             double blo[3] = {1e300, 1e300, 1e300}, bhi[3] = {-1e300, -1e300, -1e300};
             const size_t slot0 = (size_t)grp_blk[gi] * BLOCK_PTS;  // the group's slots; only its last block may be padded
             const size_t slot1 = (size_t)(grp_blk[gi + 1] - 1) * BLOCK_PTS + ctx->h_meta[grp_blk[gi + 1] - 1].npts;
@@ -778,7 +775,7 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
                                            (A[1] - cen[3 * gi + 1]) * (A[1] - cen[3 * gi + 1]) +
                                            (A[2] - cen[3 * gi + 2]) * (A[2] - cen[3 * gi + 2]));
                 if (d - rad[gi] > Rs[sh]) continue;
-                if (d + rad[gi] > Rn[sh] && beyond(at, Rn[sh])) continue;
+                if (d + rad[gi] > Rs[sh] && beyond(at, Rs[sh])) continue;
                 P.shells.push_back(sh);
                 P.rows.push_back(row);
                 const int L = ctx->h_sh_l[sh], nc = 2 * L + 1;
