@@ -100,27 +100,32 @@ __global__ void k_becke_pairs(const double* __restrict__ atom_xyz, const double*
         becke_pair(atom_xyz, brad, ghost, size_adjust, e / natom, e % natom, inv[e], adj[e]);
 }
 
-// The tables of k_becke_near, one CTA per atom m: (inv, adj) of its row in FP64 and in FP32, and
-// its kNearList nearest atoms by distance, itself first (ties by index).
+// The tables of k_becke_near, one CTA per atom m: (inv, adj) of its row in FP64 and in FP32, whether
+// any of them is not finite (two atoms in one place, radii of zero), and its kNearList nearest atoms by
+// distance, itself first (ties by index).
 constexpr int kNearList = 16;
 __global__ void __launch_bounds__(128) k_becke_near_tables(const double* __restrict__ atom_xyz,
                                                            const double* __restrict__ brad,
                                                            const int* __restrict__ ghost, int natom, int size_adjust,
                                                            double2* __restrict__ pair, float2* __restrict__ pairf,
-                                                           int* __restrict__ near) {
+                                                           int* __restrict__ near, int* __restrict__ odd) {
     extern __shared__ double nd[];  // [natom] squared distance to m
     __shared__ double bd[128];
     __shared__ int bi[128];
     const int m = blockIdx.x, t = threadIdx.x;
+    bool wild = false;
     for (int n = t; n < natom; n += blockDim.x) {
         double inv, adj;
         becke_pair(atom_xyz, brad, ghost, size_adjust, m, n, inv, adj);
         pair[(size_t)m * natom + n] = make_double2(inv, adj);
         pairf[(size_t)m * natom + n] = make_float2((float)inv, (float)adj);
+        wild = wild || !isfinite((float)inv) || !isfinite((float)adj);
         const double dx = atom_xyz[3 * m] - atom_xyz[3 * n], dy = atom_xyz[3 * m + 1] - atom_xyz[3 * n + 1],
                      dz = atom_xyz[3 * m + 2] - atom_xyz[3 * n + 2];
         nd[n] = n == m ? -1.0 : dx * dx + dy * dy + dz * dz;
     }
+    wild = __syncthreads_or(wild);
+    if (t == 0) odd[m] = wild ? 1 : 0;
     for (int k = 0; k < kNearList && k < natom; ++k) {
         __syncthreads();
         double d = 1e300;
@@ -148,7 +153,8 @@ __global__ void __launch_bounds__(128) k_becke_near_tables(const double* __restr
 //      estimate of P_c;
 //   2. the filter, a warp per m with a lane per point: an FP32 upper bound of P_m from the factors of
 //      c's nearest atoms alone (every factor is at most 1 and carries a margin for the FP32 rounding);
-//      m is dropped when the bound falls below 2^-80 of P_c;
+//      m is dropped when the bound falls below 2^-80 of P_c. Nothing is dropped where a pair constant of
+//      the molecule is not finite: P_m may then be a NaN, which the sum has to show;
 //   3. P_m of the kept (m, point) pairs (about 10 of 100 atoms), packed over the CTA's threads in the
 //      order of m, with the operations and the order of k_becke;
 //   4. per point the sum over m in ascending order, twice: with every dropped P_m at its lower and at
@@ -203,7 +209,8 @@ template <int kNearW>
 __global__ void __launch_bounds__(32 * kNearW) k_becke_near(const double* __restrict__ atom_xyz, int natom,
                                                              const double2* __restrict__ pair,
                                                              const float2* __restrict__ pairf,
-                                                             const int* __restrict__ near, int64_t npts,
+                                                             const int* __restrict__ near,
+                                                             const int* __restrict__ odd, int64_t npts,
                                                              const double* __restrict__ xyz,
                                                              const int* __restrict__ owner,
                                                              const double* __restrict__ w_single,
@@ -219,6 +226,9 @@ __global__ void __launch_bounds__(32 * kNearW) k_becke_near(const double* __rest
     constexpr unsigned kAll = 0xffffffffu;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int nlist = min(kNearList, natom);
+    bool wild = false;
+    for (int m = t; m < natom; m += 32 * kNearW) wild = wild || odd[m] != 0;
+    const bool keep_all = __syncthreads_or(wild);
     for (int64_t i0 = blockIdx.x * (int64_t)kNearPts; i0 < npts; i0 += (int64_t)gridDim.x * kNearPts) {
         const int64_t i = i0 + lane;
         const bool live = i < npts;
@@ -258,7 +268,7 @@ __global__ void __launch_bounds__(32 * kNearW) k_becke_near(const double* __rest
         float pc = 1.0f;
 #pragma unroll
         for (int w = 0; w < kNearW; ++w) pc *= s_prod[w][lane];
-        const float thr = pc > 1e-10f ? pc * 8.271806e-25f : 0.0f;
+        const float thr = pc > 1e-10f && !keep_all ? pc * 8.271806e-25f : 0.0f;
         // 2. the filter: c's nearest atoms and their distances in registers, four factors at a time
         int nn[kNearList];
         float rn[kNearList];
@@ -521,7 +531,7 @@ size_t becke_near_max_atoms() { return 480; }
 constexpr int kNearSmall = 48;
 
 size_t becke_near_table_bytes(int natom) {
-    return (size_t)natom * natom * (sizeof(double2) + sizeof(float2)) + sizeof(int) * kNearList * (size_t)natom;
+    return (size_t)natom * natom * (sizeof(double2) + sizeof(float2)) + sizeof(int) * (kNearList + 1) * (size_t)natom;
 }
 
 void launch_becke_near(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
@@ -531,9 +541,10 @@ void launch_becke_near(const double* atom_xyz, const double* brad, const int* gh
     double2* pair = static_cast<double2*>(tab);
     float2* pairf = reinterpret_cast<float2*>(pair + n2);
     int* near = reinterpret_cast<int*>(pairf + n2);
+    int* odd = near + kNearList * (size_t)natom;
     if (tables)
         k_becke_near_tables<<<natom, 128, sizeof(double) * natom, s>>>(atom_xyz, brad, ghost, natom, size_adjust, pair,
-                                                                       pairf, near);
+                                                                       pairf, near, odd);
     const size_t smem = (size_t)natom * kNearPts * (sizeof(double) + sizeof(float)) + sizeof(double) * kNearCap +
                         sizeof(int) * (2 * (size_t)natom + 1);
     int64_t blocks = (npts + kNearPts - 1) / kNearPts;
@@ -541,11 +552,11 @@ void launch_becke_near(const double* atom_xyz, const double* brad, const int* gh
     if (blocks < 1) blocks = 1;
     if (natom <= kNearSmall) {
         cudaFuncSetAttribute(k_becke_near<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_becke_near<4><<<(unsigned)blocks, 128, smem, s>>>(atom_xyz, natom, pair, pairf, near, npts, xyz, owner,
+        k_becke_near<4><<<(unsigned)blocks, 128, smem, s>>>(atom_xyz, natom, pair, pairf, near, odd, npts, xyz, owner,
                                                             w_single, w_out);
     } else {
         cudaFuncSetAttribute(k_becke_near<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_becke_near<8><<<(unsigned)blocks, 256, smem, s>>>(atom_xyz, natom, pair, pairf, near, npts, xyz, owner,
+        k_becke_near<8><<<(unsigned)blocks, 256, smem, s>>>(atom_xyz, natom, pair, pairf, near, odd, npts, xyz, owner,
                                                             w_single, w_out);
     }
 }

@@ -1,0 +1,49 @@
+"""Becke partition weights bit for bit against the CPU restatement, where the near form's filter, sums
+and tables can go wrong."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def chain(n, seed):
+    from proteindf_b200 import basis, grids, systems
+    syms, xyz = systems.peptide_chain(n, seed=seed)
+    sh = basis.ShellTable(syms, xyz, basis.load_basis("cc-pVDZ"))
+    return sh, np.array([grids.BECKE_RADIUS[int(z)] for z in sh.atom_z])
+
+
+def weights(sh, brad, pts, owner, **kw):
+    from proteindf_b200.xc import XcEngine
+    eng = XcEngine()
+    eng.set_system(sh)
+    w = eng.becke_weights(pts, owner, np.ones(len(pts)), brad, **kw)
+    eng.close()
+    return w
+
+
+def near_points(sh, n, seed, spread=1.5):
+    """Points around seeded atoms, each with its atom as the owner."""
+    rng = np.random.default_rng(seed)
+    owner = rng.integers(0, sh.natom, n).astype(np.int32)
+    return sh.atom_xyz[owner] + spread * rng.standard_normal((n, 3)), owner
+
+
+@pytest.mark.parametrize("n", [30, 60])
+@pytest.mark.parametrize("what", ["place", "radius"])
+def test_non_finite_pair_constants_show_in_every_weight(n, what):
+    """Two atoms in one place (1/R_mn infinite) or of radius zero (a_mn 0/0): P of the first is a NaN at
+    every point, and so is every weight, however far the two are from the point."""
+    from oracle import oracle
+    from proteindf_b200 import basis
+    sh, brad = chain(n, seed=11)
+    if what == "place":
+        xyz = sh.atom_xyz.copy()
+        xyz[1] = xyz[0]
+        sh = basis.ShellTable(sh.symbols, xyz, basis.load_basis("cc-pVDZ"))
+    else:
+        brad[:2] = 0.0
+    pts, owner = near_points(sh, 500, seed=n)
+    ref = oracle.becke(sh.atom_xyz, brad, pts, owner)
+    assert np.isnan(ref).all()
+    assert np.isnan(weights(sh, brad, pts, owner)).all()
