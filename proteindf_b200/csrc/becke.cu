@@ -195,7 +195,10 @@ __device__ __forceinline__ double becke_product(const double* r, const double2* 
 }
 
 // FP32 factor s(nu_mn) and a bound of its rounding error: |d mu| <= 1.8e-7 (r_m + r_n) / R_mn, at most
-// 3.4 times that in s, and 1e-6 for the polynomial.
+// 3.4 times that in s, and 1e-6 for the polynomial. That holds while mu stays near [-1, 1]: from a margin of
+// 0.25 on the polynomial may be anything. max(s, 0) + margin still bounds the factor from above there (up
+// to a margin of 1 the cubics map what lies beyond 1 back into [-1, 1], and above it the sum is past 1); s
+// alone says nothing.
 __device__ __forceinline__ float becke_s32(float rm, float rn, float2 c, float& margin) {
     const float u = (rm - rn) * c.x;
     float nu = fmaf(c.y, fmaf(-u, u, 1.0f), u);
@@ -259,12 +262,13 @@ __global__ void __launch_bounds__(32 * kNearW) k_becke_near(const double* __rest
             for (int n = warp; n < natom; n += kNearW) {
                 float e;
                 const float s = becke_s32(rc, rf[n * kNearPts + lane], __ldg(pairf + (size_t)c * natom + n), e);
-                p *= n == c ? 1.0f : s;
+                p *= n == c ? 1.0f : (e <= 0.25f ? s : 0.0f);
             }
             s_prod[warp][lane] = p;
         }
         __syncthreads();
-        // the drop threshold: 2^-80 P_c, and nothing dropped where P_c is near the end of the FP32 range
+        // the drop threshold: 2^-80 P_c, and nothing dropped where P_c is near the end of the FP32 range or a
+        // point is so far away that FP32 does not tell the distances apart (from 1e5 to 1e6 bohr on)
         float pc = 1.0f;
 #pragma unroll
         for (int w = 0; w < kNearW; ++w) pc *= s_prod[w][lane];
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(32 * kNearW) k_becke_near(const double* __rest
                     float e;
                     const float s = becke_s32(rm, rn[k0 + k], pc4[k], e);
                     // (a list shorter than kNearList repeats its last atom: not a factor twice)
-                    p *= nn[k0 + k] != m && k0 + k < nlist ? s + e : 1.0f;
+                    p *= nn[k0 + k] != m && k0 + k < nlist ? fmaxf(s, 0.0f) + e : 1.0f;
                 }
                 drop = drop || p < thr;
                 if (__all_sync(kAll, drop)) break;

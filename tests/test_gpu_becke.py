@@ -47,3 +47,19 @@ def test_non_finite_pair_constants_show_in_every_weight(n, what):
     ref = oracle.becke(sh.atom_xyz, brad, pts, owner)
     assert np.isnan(ref).all()
     assert np.isnan(weights(sh, brad, pts, owner)).all()
+
+
+@pytest.mark.parametrize("n", [40, 100])
+def test_far_points_equal_oracle_bit_for_bit(n):
+    """Points at 1e3 to 1e9 bohr and beyond the range of FP32, where FP32 no longer tells the atoms'
+    distances apart: the filter must not drop an atom that carries the sum."""
+    from oracle import oracle
+    sh, brad = chain(n, seed=1)
+    rng = np.random.default_rng(n)
+    far = np.repeat([1e3, 1e5, 3e5, 1e6, 1e7, 2e7, 5e7, 1e8, 1e9, 1e12, 1e39], 60)
+    u = rng.standard_normal((len(far), 3))
+    pts = far[:, None] * u / np.linalg.norm(u, axis=1)[:, None]
+    owner = rng.integers(0, n, len(far)).astype(np.int32)
+    w = weights(sh, brad, pts, owner)
+    ref = oracle.becke(sh.atom_xyz, brad, pts, owner)
+    assert np.array_equal(w, ref, equal_nan=True)
