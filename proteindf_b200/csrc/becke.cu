@@ -538,6 +538,11 @@ size_t becke_near_table_bytes(int natom) {
     return (size_t)natom * natom * (sizeof(double2) + sizeof(float2)) + sizeof(int) * (kNearList + 1) * (size_t)natom;
 }
 
+static size_t becke_near_smem(int natom) {
+    return (size_t)natom * kNearPts * (sizeof(double) + sizeof(float)) + sizeof(double) * kNearCap +
+           sizeof(int) * (2 * (size_t)natom + 1);
+}
+
 void launch_becke_near(const double* atom_xyz, const double* brad, const int* ghost, int natom, int size_adjust,
                        void* tab, int64_t npts, const double* xyz, const int* owner, const double* w_single,
                        double* w_out, bool tables, cudaStream_t s) {
@@ -549,17 +554,19 @@ void launch_becke_near(const double* atom_xyz, const double* brad, const int* gh
     if (tables)
         k_becke_near_tables<<<natom, 128, sizeof(double) * natom, s>>>(atom_xyz, brad, ghost, natom, size_adjust, pair,
                                                                        pairf, near, odd);
-    const size_t smem = (size_t)natom * kNearPts * (sizeof(double) + sizeof(float)) + sizeof(double) * kNearCap +
-                        sizeof(int) * (2 * (size_t)natom + 1);
+    const size_t smem = becke_near_smem(natom);
+    // the limit belongs to the function in the whole process: the largest size, whatever this call's (calls
+    // on other threads would lower one another's; so in every launcher whose size varies)
+    const int limit = (int)becke_near_smem((int)becke_near_max_atoms());
     int64_t blocks = (npts + kNearPts - 1) / kNearPts;
     if (blocks > 148 * 64) blocks = 148 * 64;
     if (blocks < 1) blocks = 1;
     if (natom <= kNearSmall) {
-        cudaFuncSetAttribute(k_becke_near<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_becke_near<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
         k_becke_near<4><<<(unsigned)blocks, 128, smem, s>>>(atom_xyz, natom, pair, pairf, near, odd, npts, xyz, owner,
                                                             w_single, w_out);
     } else {
-        cudaFuncSetAttribute(k_becke_near<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_becke_near<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
         k_becke_near<8><<<(unsigned)blocks, 256, smem, s>>>(atom_xyz, natom, pair, pairf, near, odd, npts, xyz, owner,
                                                             w_single, w_out);
     }
@@ -583,7 +590,8 @@ void launch_becke_warp(const double* atom_xyz, const double* brad, const int* gh
     if (blocks > 148 * 64) blocks = 148 * 64;
     if (blocks < 1) blocks = 1;
     const size_t smem = 2 * sizeof(double) * BECKE_WW * natom;
-    cudaFuncSetAttribute(k_becke_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_becke_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(2 * sizeof(double) * BECKE_WW * becke_warp_max_atoms()));
     k_becke_warp<<<(unsigned)blocks, 32 * BECKE_WW, smem, s>>>(atom_xyz, natom, invT, adjT, npts, xyz, owner, w_single,
                                                                w_out);
 }
@@ -596,7 +604,8 @@ void launch_becke(const double* atom_xyz, const double* brad, const int* ghost, 
     if (blocks > 148 * 64) blocks = 148 * 64;
     if (blocks < 1) blocks = 1;
     const size_t smem = sizeof(double4) * natom;
-    cudaFuncSetAttribute(k_becke, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_becke, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(double4) * becke_max_atoms()));
     k_becke<<<(unsigned)blocks, threads, smem, s>>>(atom_xyz, brad, ghost, natom, size_adjust, npts, xyz, owner,
                                                     w_single, w_out);
 }

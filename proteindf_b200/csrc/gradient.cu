@@ -292,6 +292,10 @@ int grad_weight_max_atoms() { return (int)((200u * 1024u) / (2 * sizeof(double) 
 
 namespace {
 constexpr int kWeightDramCtas = 148 * 4;
+// Limits of the dynamic shared memory (the functions' for the whole process, so not by this call's size): the
+// most atoms of the shared form; for the other an SM's 227 KiB less the kernel's own 1040 bytes
+constexpr int kWeightSmem = 400 * (2 * (int)sizeof(double) * GW_T + 2 * (int)sizeof(int));
+constexpr int kWeightListSmem = 227 * 1024 - 1040;
 }
 
 size_t grad_weight_scratch_doubles(int natom) { return (size_t)2 * natom * kWeightDramCtas * GW_T; }
@@ -303,13 +307,13 @@ void launch_grad_weight(const double* atom_xyz, int natom, const double* inv, co
     int64_t blocks = (nslots + GW_T - 1) / GW_T;
     if (scratch) {
         if (blocks > kWeightDramCtas) blocks = kWeightDramCtas;
-        cudaFuncSetAttribute(k_grad_weight<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lists);
+        cudaFuncSetAttribute(k_grad_weight<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWeightListSmem);
         k_grad_weight<true><<<(unsigned)blocks, GW_T * GW_W, lists, s>>>(atom_xyz, natom, inv, adj, nslots, px, py, pz,
                                                                         owner, wsingle, fdens, grad, scratch);
     } else {
         const size_t smem = 2 * sizeof(double) * GW_T * (size_t)natom + lists;
         if (blocks > 148 * 32) blocks = 148 * 32;
-        cudaFuncSetAttribute(k_grad_weight<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_grad_weight<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWeightSmem);
         k_grad_weight<false><<<(unsigned)blocks, GW_T * GW_W, smem, s>>>(atom_xyz, natom, inv, adj, nslots, px, py, pz,
                                                                          owner, wsingle, fdens, grad, nullptr);
     }

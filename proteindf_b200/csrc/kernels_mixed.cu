@@ -20,6 +20,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "ao.cuh"
 #include "functional.cuh"
 #include "pdfxc_internal.cuh"
@@ -1596,6 +1598,9 @@ size_t umma_smem_bytes(int nterms) {
     return (size_t)S * 2 * nA * umma::SLAB_BYTES + (2 * S + 1) * 8 + 16;
 }
 
+// k_umma's limit of shared memory, the same for every call (it is the function's for the whole process)
+static int umma_smem_limit() { return (int)std::max(umma_smem_bytes(3), umma_smem_bytes(6)); }
+
 static UmmaParams umma_params(const MixedArgs& a) { return UmmaParams{a.nterms, a.nterms == 3 ? 3 : 2, a.err, nullptr}; }
 
 void mixed_prepare(const MixedArgs& a, cudaStream_t s) {
@@ -1610,11 +1615,11 @@ void mixed_rho(const MixedArgs& a, cudaStream_t s) {
     const int tiles = a.max_nbp / umma::TILE_ROWS;
     const size_t smem = umma_smem_bytes(a.nterms);
     if (functional_is_gga(a.fn)) {
-        cudaFuncSetAttribute(k_umma<MODE_RHO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_umma<MODE_RHO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma_smem_limit());
         k_umma<MODE_RHO, true><<<dim3(tiles, a.nblk), 128, smem, s>>>(a.g, a.blk0, a.ws, umma_params(a), tiles,
                                                                      a.rho_acc, a.Vacc, a.nao);
     } else {
-        cudaFuncSetAttribute(k_umma<MODE_RHO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_umma<MODE_RHO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma_smem_limit());
         k_umma<MODE_RHO, false><<<dim3(tiles, a.nblk), 128, smem, s>>>(a.g, a.blk0, a.ws, umma_params(a), tiles,
                                                                       a.rho_acc, a.Vacc, a.nao);
     }
@@ -1632,7 +1637,7 @@ void mixed_functional(const MixedArgs& a, cudaStream_t s) {
 void mixed_vxc(const MixedArgs& a, cudaStream_t s) {
     const int tiles = a.max_nbp / umma::TILE_ROWS;
     const size_t smem = umma_smem_bytes(a.nterms);
-    cudaFuncSetAttribute(k_umma<MODE_VXC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_umma<MODE_VXC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma_smem_limit());
     k_umma<MODE_VXC, false><<<dim3(tiles * tiles, a.nblk), 128, smem, s>>>(a.g, a.blk0, a.ws, umma_params(a), tiles,
                                                                           a.rho_acc, a.Vacc, a.nao);
 }

@@ -63,3 +63,36 @@ def test_far_points_equal_oracle_bit_for_bit(n):
     w = weights(sh, brad, pts, owner)
     ref = oracle.becke(sh.atom_xyz, brad, pts, owner)
     assert np.array_equal(w, ref, equal_nan=True)
+
+
+def test_contexts_of_different_sizes_in_several_threads():
+    """The near form's shared memory depends on the atom count, its limit is the function's for the whole
+    process: contexts of 60 and of 400 atoms on four host threads must not lower it for one another."""
+    import threading
+    from proteindf_b200.xc import XcEngine
+    work, bad = [], []
+    for n in (400, 60, 400, 60):
+        sh, brad = chain(n, seed=9)
+        eng = XcEngine()
+        eng.set_system(sh)
+        pts, owner = near_points(sh, 1, seed=n)
+        work.append((eng, brad, pts, owner, eng.becke_weights(pts, owner, np.ones(1), brad)))
+    start = threading.Barrier(len(work))
+
+    def calls(eng, brad, pts, owner, want):
+        start.wait()
+        try:
+            for _ in range(700):
+                if not np.array_equal(eng.becke_weights(pts, owner, np.ones(1), brad), want):
+                    bad.append("weights")
+        except RuntimeError as e:
+            bad.append(str(e))
+
+    threads = [threading.Thread(target=calls, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for w in work:
+        w[0].close()
+    assert not bad, bad[:3]
