@@ -1,5 +1,6 @@
-"""Becke partition weights bit for bit against the CPU restatement, where the near form's filter, sums
-and tables can go wrong."""
+"""Partition weights bit for bit against the CPU restatement: the forms of the Becke weights by atom count
+(near to 480, a warp per point to 1600, a thread per point above), the parts of a long call, and where the
+near form's filter, sums and tables can go wrong."""
 import numpy as np
 import pytest
 
@@ -96,3 +97,33 @@ def test_contexts_of_different_sizes_in_several_threads():
     for w in work:
         w[0].close()
     assert not bad, bad[:3]
+
+
+@pytest.mark.parametrize("n", [480, 481, 500, 1600, 1601])
+def test_forms_at_their_ends_equal_oracle_bit_for_bit(n):
+    """The last atom count of the near form, the first ones and the last of the warp form, the first of the
+    form with a thread per point; 300 points, of which one is far outside."""
+    from oracle import oracle
+    sh, brad = chain(n, seed=3)
+    pts, owner = near_points(sh, 300, seed=n)
+    pts[7] += 400.0
+    assert np.array_equal(weights(sh, brad, pts, owner), oracle.becke(sh.atom_xyz, brad, pts, owner))
+
+
+@pytest.mark.parametrize("form,n", [("near", 20), ("near", 60), ("warp", 481), ("ss", 60)])
+def test_parts_of_a_long_call_equal_short_calls(form, n):
+    """More than 65,536 points go through the kernels in parts that share the pair tables of the first; every
+    point's weight is that of a call of its own part."""
+    from proteindf_b200.xc import XcEngine
+    sh, brad = chain(n, seed=4)
+    npts = 65536 * 2 + 77 if n < 100 else 65536 + 77
+    pts, owner = near_points(sh, npts, seed=n)
+    w = 1.0 + np.arange(npts) / npts
+    eng = XcEngine()
+    eng.set_system(sh)
+    call = eng.ss_weights if form == "ss" else lambda p, o, v: eng.becke_weights(p, o, v, brad)
+    whole = call(pts, owner, w)
+    for i in range(0, npts, 30000):
+        s = slice(i, i + 30000)
+        assert np.array_equal(call(pts[s], owner[s], w[s]), whole[s])
+    eng.close()

@@ -90,7 +90,7 @@ def test_becke_vs_reference(water2):
 def test_becke_equals_oracle_bit_for_bit():
     """The device's Becke weights (compiled without fused multiply-adds) equal the CPU
     restatement's bit for bit, so both sides keep the same points under the 1e-16 weight screen;
-    a 30-atom chain on a USER 40 x 110 grid, the warp-per-point table form."""
+    a 30-atom chain on a USER 40 x 110 grid, the near form with four warps."""
     from oracle import oracle
     from proteindf_b200 import basis, grids, systems
     from proteindf_b200.xc import XcEngine
@@ -106,9 +106,8 @@ def test_becke_equals_oracle_bit_for_bit():
     eng.close()
 
 
-def test_becke_warp_form_equals_oracle_bit_for_bit():
-    """Above 48 atoms the Becke weights come from the warp-per-point kernel (its lanes over the
-    atoms); they equal the CPU restatement's bit for bit too: a 56-atom chain on a USER 20 x 50 grid."""
+def test_becke_near_form_of_eight_warps_equals_oracle_bit_for_bit():
+    """Above 48 atoms the near form runs with eight warps per CTA: a 56-atom chain on a USER 20 x 50 grid."""
     from oracle import oracle
     from proteindf_b200 import basis, grids, systems
     from proteindf_b200.xc import XcEngine
