@@ -127,3 +127,36 @@ def test_parts_of_a_long_call_equal_short_calls(form, n):
         s = slice(i, i + 30000)
         assert np.array_equal(call(pts[s], owner[s], w[s]), whole[s])
     eng.close()
+
+
+def lattice(k, seed=0):
+    """k^3 hydrogen atoms on a shaken lattice of 1.4 bohr, radii of two kinds: most P_m count at most points."""
+    from proteindf_b200 import basis
+    rng = np.random.default_rng(seed + k)
+    n = k ** 3
+    xyz = 1.4 * np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    sh = basis.ShellTable(["H"] * n, xyz + rng.uniform(-0.2, 0.2, (n, 3)), {"H": [{"shell": "s", "prims": [[0.6, 1.0]]}]})
+    return sh, np.where(np.arange(n) % 3 == 0, 0.35, 0.70)
+
+
+@pytest.mark.parametrize("k", [3, 4, 5])
+@pytest.mark.parametrize("spread", [0.7, 10.0, 100.0])
+def test_many_kept_pairs_equal_oracle_bit_for_bit(k, spread):
+    """125 atoms with points far outside keep 37 of them a point: more pairs than a CTA's 1,024 at once, so its
+    points are summed in several runs of atoms. The last CTA has 13 points."""
+    from oracle import oracle
+    sh, brad = lattice(k)
+    pts, owner = near_points(sh, 301, seed=k, spread=spread)
+    assert np.array_equal(weights(sh, brad, pts, owner), oracle.becke(sh.atom_xyz, brad, pts, owner))
+
+
+@pytest.mark.parametrize("share", ["2.8e-14", "1e-9", "1e-4"])
+@pytest.mark.parametrize("k", [3, 5])
+def test_second_sum_equals_oracle_bit_for_bit(k, share, monkeypatch):
+    """A looser drop threshold leaves the sum's last bits open at nearly every point (297 to 301 of the 301); they
+    are summed over all atoms, to the same bits."""
+    from oracle import oracle
+    monkeypatch.setenv("PDFXC_BECKE_SHARE", share)
+    sh, brad = lattice(k)
+    pts, owner = near_points(sh, 301, seed=k)
+    assert np.array_equal(weights(sh, brad, pts, owner), oracle.becke(sh.atom_xyz, brad, pts, owner))
