@@ -122,7 +122,12 @@ __global__ void __launch_bounds__(256, 2) k_grad_atoms(BasisView bas, GridView g
             tx += ax, ty += ay, tz += az;
         }
     }
-    warp_add3_by_owner(grad, owner[gp], 4.0, tx, ty, tz);
+    // the halves' sums of a point first: every addition to an owner's running sum, which is larger than the
+    // gradient (it cancels against the atoms' terms), rounds once
+    __syncthreads();
+    if (half) s_xyz[0][p] = tx, s_xyz[1][p] = ty, s_xyz[2][p] = tz;
+    __syncthreads();
+    if (!half) warp_add3_by_owner(grad, owner[gp], 4.0, tx + s_xyz[0][p], ty + s_xyz[1][p], tz + s_xyz[2][p]);
 }
 
 __device__ __forceinline__ void becke_poly(double nu, double& p1, double& p2, double& p3) {
@@ -271,8 +276,17 @@ __global__ void __launch_bounds__(GW_T* GW_W) k_grad_weight(
             warp_add3(grad, B, 1.0, dx, dy, dz);
             Tx += dx, Ty += dy, Tz += dz;
         }
-        warp_add3_by_owner(grad, A, -1.0, Tx, Ty, Tz);
-        __syncthreads();  // the rows and lists are rewritten by the next tile of points
+        // the warps' sums of a point first, as in k_grad_atoms; after the last barrier the rows and lists are
+        // rewritten by the next tile of points
+        double T[3] = {Tx, Ty, Tz};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s_z[warp][t] = T[k];
+            __syncthreads();
+            T[k] = (s_z[0][t] + s_z[1][t]) + (s_z[2][t] + s_z[3][t]);
+            __syncthreads();
+        }
+        if (warp == 0) warp_add3_by_owner(grad, A, -1.0, T[0], T[1], T[2]);
     }
 }
 
