@@ -30,9 +30,8 @@ namespace fdetail {
 // functional. (The functional kernels are bound by the FP64 pipe; pow costs several times cbrt. B3LYP
 // over 3.5 M points: 0.88 -> 0.25 ms.)
 __device__ __forceinline__ void slater(double ra, double rb, double ca, double cb, double& f, double& va, double& vb) {
-    const double ck = 0.62035049089940001667;  // (3 / (4 pi))^(1/3)
-    const double coef = -(9.0 / 4.0) * ck * (2.0 / 3.0);
-    const double dcoef = -3.0 * ck * (2.0 / 3.0);
+    const double coef = -0.93052573634910002500;   // -(3/2) (3 / (4 pi))^(1/3)
+    const double dcoef = -1.24070098179880003333;  // 4/3 of it
     f = coef * (ra * ca + rb * cb);
     va = dcoef * ca;
     vb = dcoef * cb;
