@@ -70,12 +70,13 @@ __device__ __forceinline__ void warp_add3_by_owner(double* grad, int own, double
 // of the stored second derivatives (1.2) and the pass over 14 planes (1.8), and three contractions less.
 template <bool GGA>
 __global__ void __launch_bounds__(256, 2) k_grad_atoms(BasisView bas, GridView g, const int* __restrict__ owner,
-                                                       int blk0, const double* __restrict__ coef, const char* ws,
-                                                       double* grad) {
+                                                       int natom, int blk0, const double* __restrict__ coef,
+                                                       const char* ws, double* grad) {
     __shared__ double s_xyz[3][128];
     __shared__ int s_row[128], s_l[128], s_at[128];
     const int blk = blk0 + blockIdx.x;
     const BlockMeta m = g.meta[blk];
+    grad += (size_t)6 * natom * (blk % GRAD_COPIES);
     const int p = threadIdx.x & (BLOCK_PTS - 1), half = threadIdx.x >> 7;
     const size_t plane = (size_t)m.nbp * BLOCK_PTS;
     const double* base = reinterpret_cast<const double*>(ws + m.ws) + p;
@@ -122,12 +123,7 @@ __global__ void __launch_bounds__(256, 2) k_grad_atoms(BasisView bas, GridView g
             tx += ax, ty += ay, tz += az;
         }
     }
-    // the halves' sums of a point first: every addition to an owner's running sum, which is larger than the
-    // gradient (it cancels against the atoms' terms), rounds once
-    __syncthreads();
-    if (half) s_xyz[0][p] = tx, s_xyz[1][p] = ty, s_xyz[2][p] = tz;
-    __syncthreads();
-    if (!half) warp_add3_by_owner(grad, owner[gp], 4.0, tx + s_xyz[0][p], ty + s_xyz[1][p], tz + s_xyz[2][p]);
+    warp_add3_by_owner(grad, owner[gp], 4.0, tx, ty, tz);
 }
 
 __device__ __forceinline__ void becke_poly(double nu, double& p1, double& p2, double& p3) {
@@ -172,6 +168,7 @@ __global__ void __launch_bounds__(GW_T* GW_W) k_grad_weight(
     int* list = reinterpret_cast<int*>(sm + (ROWS_IN_DRAM ? 0 : 2 * (size_t)natom * GW_T));  // [natom] live atoms
     int* live_at = list + natom;                                                              // [natom] 0 or 1
     const int t = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    grad += (size_t)6 * natom * (blockIdx.x % GRAD_COPIES);
     constexpr double kTiny = 1e-250;
     for (int64_t i0 = blockIdx.x * (int64_t)GW_T; i0 < nslots; i0 += (int64_t)gridDim.x * GW_T) {
         const int64_t i = i0 + t;
@@ -276,28 +273,19 @@ __global__ void __launch_bounds__(GW_T* GW_W) k_grad_weight(
             warp_add3(grad, B, 1.0, dx, dy, dz);
             Tx += dx, Ty += dy, Tz += dz;
         }
-        // the warps' sums of a point first, as in k_grad_atoms; after the last barrier the rows and lists are
-        // rewritten by the next tile of points
-        double T[3] = {Tx, Ty, Tz};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            s_z[warp][t] = T[k];
-            __syncthreads();
-            T[k] = (s_z[0][t] + s_z[1][t]) + (s_z[2][t] + s_z[3][t]);
-            __syncthreads();
-        }
-        if (warp == 0) warp_add3_by_owner(grad, A, -1.0, T[0], T[1], T[2]);
+        warp_add3_by_owner(grad, A, -1.0, Tx, Ty, Tz);
+        __syncthreads();  // the rows and lists are rewritten by the next tile of points
     }
 }
 
 }  // namespace
 
-void launch_grad_atoms(const BasisView& b, const GridView& g, const int* owner, int blk0, int nblk, bool gga,
+void launch_grad_atoms(const BasisView& b, const GridView& g, const int* owner, int natom, int blk0, int nblk, bool gga,
                        const double* coef, const char* ws, double* grad, cudaStream_t s) {
     if (gga)
-        k_grad_atoms<true><<<nblk, 256, 0, s>>>(b, g, owner, blk0, coef, ws, grad);
+        k_grad_atoms<true><<<nblk, 256, 0, s>>>(b, g, owner, natom, blk0, coef, ws, grad);
     else
-        k_grad_atoms<false><<<nblk, 256, 0, s>>>(b, g, owner, blk0, coef, ws, grad);
+        k_grad_atoms<false><<<nblk, 256, 0, s>>>(b, g, owner, natom, blk0, coef, ws, grad);
 }
 
 // Shared memory per CTA: 520 bytes per atom (two rows of 32 doubles, a list entry and a flag); beyond

@@ -2056,9 +2056,9 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
         const int planes = pdfxc::grad_planes(gga), rad0 = planes;
         ensure_plan(ctx, ctx->gplan, planes, gga ? 3 : 2);
         const size_t nslots = (size_t)ctx->nblk * BLOCK_PTS;
-        if (!ctx->d_grad) dev_alloc(&ctx->d_grad, 6 * (size_t)natom);
+        if (!ctx->d_grad) dev_alloc(&ctx->d_grad, pdfxc::GRAD_COPIES * 6 * (size_t)natom);
         if (!ctx->d_fdens) dev_alloc(&ctx->d_fdens, nslots);
-        PDFXC_CUDA(cudaMemsetAsync(ctx->d_grad, 0, sizeof(double) * 6 * natom, s));
+        PDFXC_CUDA(cudaMemsetAsync(ctx->d_grad, 0, sizeof(double) * pdfxc::GRAD_COPIES * 6 * natom, s));
         PDFXC_CUDA(cudaMemcpyAsync(ctx->d_P, PA, sizeof(double) * nao * nao, cudaMemcpyHostToDevice, s));
         if (dexc_dP) memset_async(ctx->d_Vacc, sizeof(double) * (size_t)nao * nao, s);
         pdfxc::GridView gv = grid_view(ctx);
@@ -2083,7 +2083,7 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
                 pdfxc::launch_z_rad(bv, gv, b0, n, ctx->d_coef, nullptr, pdfxc::GRAD_Z, rad0, ws, s);
                 pdfxc::launch_gemm_x_plane(gv, ctx->d_P, nao, b0, n, ch.max_nbp, pdfxc::GRAD_Z, pdfxc::GRAD_Y, ws, s);
             }
-            pdfxc::launch_grad_atoms(bv, gv, ctx->d_owner, b0, n, gga, ctx->d_coef, ws, ctx->d_grad, s);
+            pdfxc::launch_grad_atoms(bv, gv, ctx->d_owner, natom, b0, n, gga, ctx->d_coef, ws, ctx->d_grad, s);
             if (dexc_dP && gga)
                 pdfxc::launch_gemm_v_plane(gv, b0, n, ch.max_nbp, pdfxc::GRAD_Z, ws, ctx->d_Vacc, nao, s);
             else if (dexc_dP)
@@ -2116,7 +2116,7 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
                                       ctx->d_grad + 3 * natom, dram_rows ? ctx->d_wscratch : nullptr, s);
             PDFXC_CUDA(cudaGetLastError());
         }
-        std::vector<double> g(6 * (size_t)natom);
+        std::vector<double> copies(pdfxc::GRAD_COPIES * 6 * (size_t)natom), g(6 * (size_t)natom, 0.0);
         double sc[2];
         if (dexc_dP) {
             pdfxc::launch_finish(ctx->d_Vacc, ctx->d_V, nao, ctx->d_blk_sum + 2 * (size_t)ctx->blk_lo,
@@ -2124,9 +2124,10 @@ pdfxc_status xc_derivatives(pdfxc_ctx* ctx, const char* name, int functional, co
             PDFXC_LAUNCHED("dExc/dP symmetrisation");
             PDFXC_CUDA(cudaMemcpyAsync(dexc_dP, ctx->d_V, sizeof(double) * (size_t)nao * nao, cudaMemcpyDeviceToHost, s));
         }
-        PDFXC_CUDA(cudaMemcpyAsync(g.data(), ctx->d_grad, sizeof(double) * g.size(), cudaMemcpyDeviceToHost, s));
+        PDFXC_CUDA(cudaMemcpyAsync(copies.data(), ctx->d_grad, sizeof(double) * copies.size(), cudaMemcpyDeviceToHost, s));
         PDFXC_CUDA(cudaMemcpyAsync(sc, ctx->d_scalars, sizeof(sc), cudaMemcpyDeviceToHost, s));
         PDFXC_CUDA(cudaStreamSynchronize(s));
+        for (size_t k = 0; k < copies.size(); ++k) g[k % g.size()] += copies[k];
         std::copy(g.begin(), g.begin() + 3 * natom, grad_orbital);
         if (w_single) std::copy(g.begin() + 3 * natom, g.end(), grad_weight);
         if (exc) *exc = sc[0];

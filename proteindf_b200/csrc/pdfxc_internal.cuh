@@ -186,7 +186,7 @@ struct pdfxc_ctx {
     std::vector<int> h_owner;              // owner atom per point slot (empty: set_grid had no atoms)
     int* d_owner = nullptr;
     pdfxc::Plan gplan;                     // gradient workspace layout
-    double* d_grad = nullptr;   // [2 * natom * 3]: AO-centre term, grid-weight term
+    double* d_grad = nullptr;   // [GRAD_COPIES][2 * natom * 3]: AO-centre term, grid-weight term
     double* d_fdens = nullptr;  // [nblk * BLOCK_PTS] energy density per slot
     double* d_wslot = nullptr;  // [nblk * BLOCK_PTS] single-centre weight per slot
     double* d_brad = nullptr;   // [natom]
@@ -284,8 +284,12 @@ void launch_segment_sums(const double* blk_sum, const int* seg_blk, int nseg, do
 // gradient.cu: XC nuclear gradient (FP64). Planes: phi, X = P_sub phi, Z, Y = P_sub Z (GGA), then the
 // radial sums S0, S1 and (GGA) S2 of the block's shells.
 constexpr int GRAD_X = 1, GRAD_Z = 2, GRAD_Y = 3;
+// CTAs add to one of this many copies of the gradient ([2 * natom * 3] each), which the host sums: an
+// atom's terms cancel, and every addition rounds at the size of the running sum, an eighth as large so
+constexpr int GRAD_COPIES = 8;
 inline int grad_planes(bool gga) { return gga ? 4 : 3; }
-void launch_grad_atoms(const BasisView& b, const GridView& g, const int* owner, int blk0, int nblk, bool gga,
+// grad: the first copy's AO-centre (grid-weight) term
+void launch_grad_atoms(const BasisView& b, const GridView& g, const int* owner, int natom, int blk0, int nblk, bool gga,
                        const double* coef, const char* ws, double* grad, cudaStream_t s);
 // the weight term keeps each point's atom rows in shared memory up to grad_weight_max_atoms()
 // atoms; above that (or when scratch is given) in grad_weight_scratch_doubles(natom) of device memory

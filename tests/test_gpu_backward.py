@@ -96,3 +96,20 @@ def test_autograd_matches_finite_differences(cfg3):
     print(f"cfg3 PBE finite differences: max |dE/dR - FD| = {max(errR):.3e} (h = 1e-4 bohr, 10 coordinates, "
           f"max |dE/dR| {np.abs(gR).max():.3e}); max |dE/dP_A - FD| = {max(errP):.3e} (h = 1e-5, 20 entries)")
     assert max(errR) <= FD_TOL and max(errP) <= FD_TOL
+
+
+def test_gradient_sums_to_zero_over_the_atoms(cfg3):
+    """The grid moves with its atoms, so each term's sum over the atoms is zero but for the roundings of the
+    additions to the atoms' sums, whose terms cancel. Root mean square of the sum over that of the gradient,
+    over eight densities: 5e-15 as eight copies of the sums are added to, 3e-14 with a single one."""
+    from proteindf_b200 import systems
+    c = cfg3
+    c["system"].place(c["xyz"])
+    off = []
+    for seed in range(8):
+        P = 0.5 * systems.density_matrix(c["sh"].nao, 60, seed=seed)
+        go, gw, _ = c["eng"].xc_gradient("PBE", P, w_single=c["ws"], becke_radius=c["brad"])
+        off.append([np.sqrt((g.sum(0) ** 2).mean() / (g ** 2).mean()) for g in (go, gw)])
+    off = np.sqrt((np.array(off) ** 2).mean(0))
+    print(f"sum of the gradient over the atoms: AO-centre term {off[0]:.1e}, weight term {off[1]:.1e}")
+    assert off.max() <= 1.2e-14
