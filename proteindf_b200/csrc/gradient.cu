@@ -66,8 +66,9 @@ __device__ __forceinline__ void warp_add3_by_owner(double* grad, int own, double
 // One CTA per block, 256 threads: the point is threadIdx.x % 128, the halves of the CTA take the
 // first and the second half of the block's shells (runs of one atom's shells stay together but for
 // one). Reads X, Y and the radial sums once; 16 warps per SM (its registers) do not cover the latency
-// (L1 prefetches of the shells ahead changed nothing). 30-atom PBE chain, 477k points: 0.97 ms, for 3.0 ms
-// of the stored second derivatives (1.2) and the pass over 14 planes (1.8), and three contractions less.
+// (L1 prefetches of the shells ahead changed nothing). 30-atom PBE chain, 477k points: 0.52 ms (0.97 with
+// the atomics on one copy of the gradient), for 3.0 ms of the stored second derivatives (1.2) and the pass
+// over 14 planes (1.8), and three contractions less.
 template <bool GGA>
 __global__ void __launch_bounds__(256, 2) k_grad_atoms(BasisView bas, GridView g, const int* __restrict__ owner,
                                                        int natom, int blk0, const double* __restrict__ coef,
@@ -145,7 +146,7 @@ __device__ __forceinline__ void becke_poly(double nu, double& p1, double& p2, do
 // A pair of atoms whose P_i and P_B both lie below 2^-80 Z at all of the CTA's points is left out: at
 // that size s' / s is at most 2e4 (s ~ (1 - nu)^8), so its terms are below 1e-19 of the others. The
 // points of a CTA are neighbours, so most pairs of a larger molecule go.
-// Bound by the FP64 pipe. 30-atom chain, 477k points: 1.90 ms (a thread per point, every pair: 4.09).
+// Bound by the FP64 pipe. 30-atom chain, 477k points: 1.88 ms (a thread per point, every pair: 4.09).
 //
 // ROWS_IN_DRAM: the two [natom] rows of every point live in a scratch array in device memory
 // ([2][natom][32 gridDim.x], a warp's accesses coalesced) instead of shared memory; the form for

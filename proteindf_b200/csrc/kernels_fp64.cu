@@ -92,9 +92,9 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // The FP64 contractions cover a block's nb AOs with T = ceil(nb / 64) tiles per dimension, tile i
 // taking an equal share of the 16-row pairs of DMMA rows, cut at the last row of eight: nb rounded up
-// to 8, not to 64, is what the tensor pipe works for. (nb averages 231 on the 100-atom chain, 256 with
-// 64-row padding: sum of nb^2 29 % less together with the last rows' trim.) r8, n8: first row of
-// eight and their number (at most 8).
+// to 8, not to 64, is what the tensor pipe works for. (On the benchmark's 100-atom chain nb averages 218,
+// 221 rounded up to 8 and 250 rounded up to 64: 21 % off the sum of nb^2.) r8, n8: first row of eight and
+// their number (at most 8).
 __device__ __forceinline__ void fp64_tile(int nb, int T, int i, int& r8, int& n8) {
     const int pairs = (nb + 15) / 16;
     r8 = 2 * (i * pairs / T);
@@ -333,9 +333,10 @@ __global__ void __launch_bounds__(BLOCK_PTS) k_rho_functional(GridView g, int bl
 }
 
 // Builds without stored AO gradients. Layout of a block (doubles): phi [nbp][128], one plane per
-// spin [nbp][128] (X, then Z), then, for a GGA, the radial sums S0 [nsh][128] and S1 [nsh][128]. k_ao_eval_rad writes phi and the radial sums; everything that needs grad phi forms
-// it from them (ao.cuh). The shells (rows, angular momenta, atoms, primitives) are staged in shared
-// memory, 64 at a time.
+// spin [nbp][128] (X, then Z), then, for a GGA, the radial sums S0 [nsh][128] and S1 [nsh][128].
+// k_ao_eval_rad writes phi and the radial sums; everything that needs grad phi forms it from them
+// (ao.cuh). The shells (rows, angular momenta, atoms, primitives) are staged in shared memory, 64 at a
+// time. (k_ao_eval above, with stored gradients, serves the no-allocation build alone.)
 // NR: the radial sums stored, 0 (an LDA: phi only), 2, or 3 with S2 = sum_k c_k a_k^2 e^{-a_k r^2}
 // ([nsh][128] after S1, for second derivatives).
 template <int NR>
@@ -506,10 +507,10 @@ __global__ void __launch_bounds__(256, 3) k_z_rad(BasisView bas, GridView g, int
 // Vacc[aos[m]][aos[n]] += sum_p phi[m][p] Z[n][p]: CTA tile up to 64 x 64 AOs (fp64_tile in both
 // dimensions), K = 128 points in steps of 16 through two shared-memory stages, 4 warps as 2 x 2 of up
 // to 4 x 4 DMMA tiles. Bound by the FP64 tensor pipe; two stages and 128 registers let four CTAs share
-// an SM, which hide one another's first loads and atomics (three CTAs of three stages: 100-atom build
-// 21.8 ms against 20.9; a persistent form with the ring running on across tiles was slower still). A tile of an odd number of rows of
-// eight gives its first warps more work, and a warp stays on its quarter of the SM, so the warps'
-// places in the tile rotate with the CTA. Rows at nb and beyond are not read.
+// an SM, which hide one another's first loads and atomics (three CTAs of three stages: a 100-atom build
+// 21.8 ms against 20.9; a persistent form with the ring running on across tiles was slower still). A tile of
+// an odd number of rows of eight gives its first warps more work, and a warp stays on its quarter of the
+// SM, so the warps' places in the tile rotate with the CTA. Rows at nb and beyond are not read.
 // LDA: Z = a phi with a = 0.5 w vrho per point, so there is no Z plane: B is phi again, scaled by a as
 // its fragments are loaded, and phi diag(a) phi^T is symmetric: only the tiles tm <= tn are computed
 // (the list ltiles), those off the diagonal counted twice (the finish adds Vacc^T).

@@ -578,7 +578,7 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
     ctx->h_meta.assign(nblk, BlockMeta{});
     parallel_ranges(ngrp, 256, [&](int64_t glo, int64_t ghi, int) {
         for (int64_t gi = glo; gi < ghi; ++gi) {
-            // the group's centre and radius (screening)
+            // the group's centre and bounding radius (screening: what they alone settle)
             const int64_t g0 = runs[grp_blk[gi]].first, g1 = runs[grp_blk[gi + 1] - 1].second;
             double gc[3] = {0, 0, 0};
             for (int64_t i = g0; i < g1; ++i)
@@ -741,7 +741,8 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
             // the others that none reaches; for the rest the points are looked through, as far as the first
             // one inside, once per atom.
             double blo[3] = {1e300, 1e300, 1e300}, bhi[3] = {-1e300, -1e300, -1e300};
-            const size_t slot0 = (size_t)grp_blk[gi] * BLOCK_PTS;  // the group's slots; only its last block may be padded
+            // the group's slots; only its last block may be padded
+            const size_t slot0 = (size_t)grp_blk[gi] * BLOCK_PTS;
             const size_t slot1 = (size_t)(grp_blk[gi + 1] - 1) * BLOCK_PTS + ctx->h_meta[grp_blk[gi + 1] - 1].npts;
             const bool padded = bp < BLOCK_PTS;  // smaller blocks: every block is padded
             for (size_t i = slot0; i < slot1; ++i) {
@@ -791,8 +792,8 @@ void plan_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* atom
                 m.nsh = (int)P.shells.size() - sh0;
                 m.nb = row;
                 // FP64: rows of eight; BF16 split: its 128 x 128 tiles; INT8: 64, the width of an output
-                // tile and of a K slab (nb averages 228 on the 100-atom chain: 128-row padding adds a
-                // quarter to the slabs that the contractions copy and multiply)
+                // tile and of a K slab (on the benchmark's 100-atom chain nb averages 227, and 128-row
+                // padding adds 28 % to the slabs of the rho contraction and 14 % to the Vxc one's)
                 const int q = !mixed ? 8 : (ctx->opt.split_terms == 10 ? 64 : 128);
                 m.nbp = std::max(q, (row + q - 1) / q * q);
                 blk_flops[bb] = 4.0 * double(m.nb) * m.nb * m.npts;
@@ -926,7 +927,8 @@ void build_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* ato
         for (const Chunk& c : ctx->chunks) {
             std::vector<std::pair<int, int2>> it;
             for (int b = c.b0; b < c.b1; ++b)  // rho: (block, 64-AO output tile); cost ~ K = nbp
-                for (int nt = 0; nt < ctx->h_meta[b].nbp / 64; ++nt) it.push_back({ctx->h_meta[b].nbp, make_int2(b, (b - ctx->h_meta[b].lead) << 16 | nt)});
+                for (int nt = 0; nt < ctx->h_meta[b].nbp / 64; ++nt)
+                    it.push_back({ctx->h_meta[b].nbp, make_int2(b, (b - ctx->h_meta[b].lead) << 16 | nt)});
             std::stable_sort(it.begin(), it.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
             ctx->items_off_rho.push_back((int)items.size());
             ctx->items_n_rho.push_back((int)it.size());
@@ -936,7 +938,8 @@ void build_grid(pdfxc_ctx* ctx, int64_t npts, const double* xyzw, const int* ato
                 const BlockMeta& m = ctx->h_meta[b];
                 if (m.lead != b) continue;
                 for (int mt = 0; mt < (m.nbp + 127) / 128; ++mt)
-                    for (int nt = 0; nt < m.nbp / 64; ++nt) it.push_back({m.gn, make_int2(b, (int)((unsigned)(m.gn - 1) << 28 | mt << 16 | nt))});
+                    for (int nt = 0; nt < m.nbp / 64; ++nt)
+                        it.push_back({m.gn, make_int2(b, (int)((unsigned)(m.gn - 1) << 28 | mt << 16 | nt))});
             }
             std::stable_sort(it.begin(), it.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
             ctx->items_off_vxc.push_back((int)items.size());
@@ -1545,8 +1548,8 @@ void collect_profile(pdfxc_ctx* ctx) {
 
 // The open-shell build's launches on ctx->stream (FP64 path): per chunk phi (and the radial sums), the
 // X contractions of both spins, rho of both in one pass (an LDA: in the contractions), the open-shell
-// functional, the Z planes of both spins in one pass (GGA), and the two Vxc contractions. P_A, P_B in ctx->d_P, d_P_b; Vacc, Vacc_b zeroed.
-// Returns the launch count.
+// functional, the Z planes of both spins in one pass (GGA), and the two Vxc contractions. P_A, P_B in
+// ctx->d_P, d_P_b; Vacc, Vacc_b zeroed. Returns the launch count.
 int64_t enqueue_uks_fp64(pdfxc_ctx* ctx, int functional, bool incremental) {
     const bool gga = pdfxc::functional_is_gga(functional);
     const int nao = ctx->nao;

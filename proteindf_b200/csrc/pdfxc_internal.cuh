@@ -334,7 +334,8 @@ __host__ __device__ inline size_t block_ws_doubles(int nbp, bool gga) {
     return (size_t)nbp * BLOCK_PTS * (gga ? 5 : 2);
 }
 
-// The closed-shell FP64 build: phi and X (then Z) planes, then the shells' radial sums S0, S1 (the GGA form; an LDA uses the planes only).
+// The closed-shell FP64 build: phi and X (then Z) planes, then the shells' radial sums S0, S1 (the GGA
+// form; an LDA uses the planes only).
 __host__ __device__ inline size_t block_ws_doubles_rad(int nbp, int nsh) {
     return (size_t)BLOCK_PTS * (2 * (size_t)nbp + 2 * (size_t)nsh);
 }
