@@ -99,10 +99,11 @@ def test_contexts_of_different_sizes_in_several_threads():
     assert not bad, bad[:3]
 
 
-@pytest.mark.parametrize("n", [480, 481, 500, 1600, 1601])
+@pytest.mark.parametrize("n", [4, 16, 17, 480, 481, 500, 1600, 1601])
 def test_forms_at_their_ends_equal_oracle_bit_for_bit(n):
-    """The last atom count of the near form, the first ones and the last of the warp form, the first of the
-    form with a thread per point; 300 points, of which one is far outside."""
+    """Molecules below, at and above the 16 atoms of a near list, the last atom count of the near form, the
+    first ones and the last of the warp form, the first of the form with a thread per point; 300 points, of
+    which one is far outside."""
     from oracle import oracle
     sh, brad = chain(n, seed=3)
     pts, owner = near_points(sh, 300, seed=n)
