@@ -267,6 +267,11 @@ def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
         return
+    from oracle import refio
+    if not refio.ref_available():  # the CPU restatement is not the reference: no figure in its name
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not here to build its "
+                          "engine from (oracle/_ref/pdfxc_ref is absent)"}), flush=True)
+        return
     from proteindf_b200 import grids
     from oracle import oracle
     syms, xyz, sh, P, W, A, PA, brad = workload(args, args.seed)
